@@ -68,6 +68,32 @@ def test_backward_matches_oracle(cls, n, w, h, mode, max_width, bgp, seed):
         assert ref["tile_count"].max() == 1024
 
 
+@pytest.mark.parametrize("n,w,h,spread,width", [(1, 16, 16, 1.0, (0.01, 0.04)), (23, 17, 15, 0.3, (0.001, 0.003)),
+                                                (24, 33, 31, 0.3, (0.2, 0.6)), (25, 16, 48, 8.0, (0.01, 0.04)),
+                                                (49, 40, 24, 40.0, (0.05, 0.3)), (1100, 24, 16, 0.2, (0.002, 0.02))])
+def test_raster_strip_segments(cls, n, w, h, spread, width):
+    """The warp strips' segment lists at their edges: chunks of 24 curves with 1, 23, 24, 25, 49 and the 1024 cap,
+    ragged images, hairlines and strokes wider than the image, curves reaching far beyond it, and curves whose
+    control points coincide (zero-length segments).  Every sum bit-exact, as the walk over all segments gives it."""
+    b = bezier_scene(n, 40 + n, width=width)
+    b[:, [0, 1, 4, 5, 8, 9, 12, 13]] *= spread
+    b[::7, 4:7] = b[::7, 8:11] = b[::7, 12:15] = b[::7, 0:3]
+    vp, vpi = camera(w, h, dist=1.4)
+    tgt, depth, bg, bgd, nrm = bezier_textures(w, h, n)
+    m = cls(n, init=b)
+    m.write_vp(vp, vpi)
+    m.write_mode(1.0)
+    m.write_max_width(0.012)
+    m.set_backward_target(tgt, depth, bg, bgd, nrm, w, h)
+    img = torch.zeros((1, h, w, 4), device="cuda")
+    m.backward(out_rgbd=img)
+    st = m.read_state()
+    ref = orc.bezier_backward(b, vp, uni6(1.0, 0.012, 0, 0, 0.0), tgt, depth, bg, bgd, nrm,
+                              loss_accum=np.zeros(n, np.float32))
+    np.testing.assert_array_equal(img.cpu().numpy()[0], ref["image"])
+    np.testing.assert_array_equal(st["grads"], ref["grads_q"])
+
+
 def test_step_bit_exact(cls):
     n = 500
     rng = np.random.default_rng(9)
