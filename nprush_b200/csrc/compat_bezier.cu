@@ -7,8 +7,8 @@
 //                 point screen Jacobians of backproject_gradient (:74-88)
 //   scan, emit, stable radix sort, ranges (as for splats; 1024 cap at :166)
 //   k_bz_raster   one CTA per (tile, view): the closest-point walk over the
-//                 segments (of 16) within reach of a warp's pixels, pressure, analytic coverage, composite over the background
-//                 (:196-269), luma / contrast / depth / edge loss (:271-320),
+//                 segments (of 16) within reach of a warp's pixels, pressure,
+//                 analytic coverage, composite over the background (:196-269), luma / contrast / depth / edge loss (:271-320),
 //                 reverse backward through the closest segment with the width,
 //                 softness and direction-regulariser terms (:325-563),
 //                 transmittance replayed exactly from per-24-curve
@@ -47,12 +47,13 @@ __device__ __forceinline__ float smoothstepf(float lo, float hi, float x) {
   const float t = clampf((x - lo) / (hi - lo), 0.0f, 1.0f);
   return t * t * (3.0f - 2.0f * t);
 }
+// WGSL i32(f32): the conversion instruction truncates, clamps below at
+// INT32_MIN and maps NaN to 0 by itself; WGSL's upper bound is the largest
+// float below 2^31, and the minimum that keeps NaN applies it
 __device__ __forceinline__ int32_t to_i32(float a) {
-  // the conversion instruction truncates and clamps below at INT32_MIN by
-  // itself (float-to-integer conversions saturate); WGSL's upper bound is the
-  // largest float below 2^31
-  if (a != a) return 0;
-  return a >= 2147483520.0f ? 2147483520 : (int32_t)a;
+  float m;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(2147483520.0f));
+  return __float2int_rz(m);
 }
 __device__ __forceinline__ float4 mulv(const float* m, float x, float y, float z, float w) {
   float4 o;

@@ -73,6 +73,33 @@ def test_backward_matches_oracle(mgr_cls, n, w, h, seed, shape):
     assert m.stats()["pairs"] > 0
 
 
+@pytest.mark.parametrize("n,w,h,shape", [(31, 16, 16, (0.1, 0.3)), (32, 17, 33, (2.0, 0.5)), (33, 40, 24, (8.0, 4.0)),
+                                         (97, 64, 16, (1.0, 0.01))])
+def test_strip_masks(mgr_cls, n, w, h, shape):
+    """The warp strips' masks at their edges: splats much smaller and much larger than a strip, five to one
+    elongated, shapes from a near-constant to a near-box falloff, opacities around the 0.001 cut, chunks of 32 splats
+    one short, full and one over, ragged images.
+
+    Tolerances: the pixel's form is evaluated fused on the device and unfused by the oracle, a relative error of at
+    most 4 * 2^-24 * 25 = 6e-6 (25: the square of the elongation), which the exponent's derivative (a x e^-x / 2 <= 2)
+    and the sums over the pairs of a pixel turn into at most 1e-4 of the composite and 1e-3 of the gradients."""
+    rng = np.random.default_rng(n)
+    s = splat_scene(n, 60 + n, spread=0.5)
+    base = np.exp(rng.uniform(np.log(0.002), np.log(0.5), n))
+    for k in (3, 12, 15):
+        s[:, k] = base * np.exp(rng.uniform(-0.8, 0.8, n))
+    s[:, 13], s[:, 14] = shape
+    s[:, 7] = np.exp(rng.uniform(np.log(0.006), np.log(0.99), n))
+    vp, vpi = camera(w, h)
+    tgt, depth = targets(w, h, 70 + n)
+    ref = orc.splat_backward(s, vp, vpi, tgt, depth)
+    g, img, _ = run_backward(mgr_cls, s, [vp], [vpi], [tgt], [depth])
+    np.testing.assert_allclose(img[0], ref["image"], atol=1e-4, rtol=0)
+    diff = np.abs(g.astype(np.int64) - ref["grads_q"].astype(np.int64))
+    assert (diff <= 2 * ref["terms"].astype(np.float64)[:, None] + 1e-3 * np.abs(ref["grads_q"]) + 1).all()
+    assert np.linalg.norm(diff) <= 1e-3 * np.linalg.norm(ref["grads_q"].astype(np.float64))
+
+
 def test_multi_view_sums_views(mgr_cls):
     n, w, h = 500, 48, 48
     s = splat_scene(n, 21)
