@@ -42,6 +42,7 @@ constexpr int kFwd = 16;        // floats per forward record
 constexpr int kBwd = 36;        // floats per backward record (144 B)
 constexpr uint32_t kCap = 1024; // SPLAT_MAX_TILE_SPLATS, constants.ts:35
 constexpr int kChunk = 32;
+constexpr int kSlots = 16;      // pairs of a chunk differentiated per replay (k_raster)
 constexpr int kThreads = 256;
 constexpr int kRasterThreads = 128;  // k_raster: two pixels of a 16 x 16 tile each
 constexpr float kFpPos = 10000.0f, kFpCol = 100000.0f;  // constants.ts:36-37
@@ -428,11 +429,11 @@ struct RasterArgs {
 constexpr uint32_t kNumChunks = kCap / kChunk;
 constexpr uint32_t kFwdBytes = sizeof(float) * kFwd, kBwdBytes = sizeof(float) * kBwd;
 
-// Shared memory of one k_raster CTA (dynamic, ~50 KB: four CTAs per SM).
+// Shared memory of one k_raster CTA (dynamic, ~34 KB: six CTAs per SM).
 struct __align__(16) RasterSmem {
   float fwd[2][kChunk][kFwd];          // staged forward records (double-buffered)
   float bwd[2][kChunk][kBwd];          // staged backward records
-  float2 tprev[kChunk][kRasterThreads];  // T before each pair of the chunk being differentiated
+  float2 tprev[kSlots][kRasterThreads];  // T before each of the pairs being differentiated
   int32_t gacc[2][kChunk][16];         // per-chunk CTA sums of the i32 gradient terms
   uint32_t ids[3][kChunk];             // splat index of each staged record
   uint64_t bar[2];                     // one mbarrier per record buffer
@@ -562,14 +563,19 @@ __device__ __forceinline__ uint2 strip_masks(const float (*fwd)[kFwd], uint32_t 
 // instructions and their integer terms are added before the warp sums them, so a
 // pair's record loads, 16 warp sums and loop cost serve 64 pixels (38% fewer
 // instructions than one pixel per thread: 200k splats, 800 x 800, 8 views,
-// dispatch 22.9 -> 19.0 ms; 512 splats, 512 x 512: 1.07 -> 0.88 ms).
+// dispatch 22.9 -> 19.0 ms; 512 splats, 512 x 512: 1.07 -> 0.88 ms).  The
+// backward keeps T for at most 16 pairs of a chunk at a time (a fifth of the
+// pairs have a term; a chunk with more is replayed twice) and replays only up
+// to the last of them: 34 KB and 80 registers, six CTAs per SM instead of four
+// (19.0 -> 16.9 ms and 0.88 -> 0.85 ms; seven and eight CTAs with 12 and 8
+// slots gain 2% more there and lose 8% at 512 large splats).
 // Records are staged 32 at a time by warp 0 with bulk copies completing on
 // an mbarrier, double-buffered (the next chunk lands while this one is
 // composited); the forward stores T at every chunk start, and the backward
 // walks the chunks in reverse, replaying each from its checkpoint.  The
 // checkpoints (32 KB per CTA) live in global memory, where they stay in L2
 // between the forward's write and the backward's read: kept in shared memory
-// they held residency at two CTAs per SM, here four fit.
+// they held residency at two CTAs per SM.
 //
 // Exact skips (results identical to evaluating every pair):
 //  * a pair whose alpha is exactly 0 at every pixel of the warp (beyond shape_b
@@ -587,7 +593,7 @@ __device__ __forceinline__ uint2 strip_masks(const float (*fwd)[kFwd], uint32_t 
 //    only its shape regularisers: with T_prev == 0 every other term is a
 //    product with a zero factor, which is 0 or NaN, and i32() maps both to 0;
 //    so only dL/dT, d_shape_a and d_shape_b are evaluated and summed.
-__global__ void __launch_bounds__(kRasterThreads, 4) k_raster(RasterArgs a) {
+__global__ void __launch_bounds__(kRasterThreads, 6) k_raster(RasterArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RasterSmem& S = *reinterpret_cast<RasterSmem*>(smem_raw);
   constexpr unsigned kFull = 0xffffffffu;
@@ -743,18 +749,27 @@ __global__ void __launch_bounds__(kRasterThreads, 4) k_raster(RasterArgs a) {
     const float2 T0 = ckpt[cc * kRasterThreads + tid];
     const bool zero_chunk = __all_sync(kFull, T0.x == 0.0f && T0.y == 0.0f);
     const uint2 near = strip_masks(S.fwd[b], cnt, lane, sx0, sx1, sy0, sy1);
-    if (!zero_chunk) {
-      float2 Tc = T0;
-      for (uint32_t m = near.x; m != 0u; m &= m - 1u) {
-        const int k = __ffs((int)m) - 1;
-        S.tprev[k][tid] = Tc;
-        Tc = Tc * (1.0f - eval_px(S.fwd[b][k], ppx, ppy).al);
-      }
-    }
     int32_t* gacc = &S.gacc[b][0][0];
-    for (uint32_t m = near.y & near.x; m != 0u;) {
-      const int k = 31 - __clz((int)m);
-      m &= ~(1u << k);
+    uint32_t now = 0;  // the pairs whose T is in tprev, in index order
+    for (uint32_t todo = near.y & near.x; todo != 0u;) {
+      if (now == 0u) {
+        now = todo;
+        for (int drop = __popc(todo) - kSlots; drop > 0; --drop) now &= now - 1u;  // the last kSlots of them
+        if (!zero_chunk) {
+          float2 Tc = T0;
+          const uint32_t top = 0x80000000u >> __clz((int)now);
+          uint32_t slot = 0;
+          for (uint32_t m = near.x; m != 0u; m &= m - 1u) {
+            const uint32_t bit = m & (0u - m);
+            if (now & bit) S.tprev[slot++][tid] = Tc;
+            if (bit == top) break;
+            Tc = Tc * (1.0f - eval_px(S.fwd[b][__ffs((int)m) - 1], ppx, ppy).al);
+          }
+        }
+      }
+      const int k = 31 - __clz((int)now);
+      now &= ~(1u << k);
+      todo &= ~(1u << k);
       const float* f = S.fwd[b][k];
       const PixEval e = eval_px(f, ppx, ppy);
       const bool v0 = in0 && !(e.al.x < 0.001f), v1 = in1 && !(e.al.y < 0.001f);
@@ -763,7 +778,7 @@ __global__ void __launch_bounds__(kRasterThreads, 4) k_raster(RasterArgs a) {
       const float2 al = make_float2(v0 ? e.al.x : 0.0f, v1 ? e.al.y : 0.0f);
       float2 T_prev = both(0.0f);
       if (!zero_chunk) {
-        const float2 t = S.tprev[k][tid];
+        const float2 t = S.tprev[__popc(now)][tid];  // now holds the pairs before this one
         T_prev = make_float2(v0 ? t.x : 0.0f, v1 ? t.y : 0.0f);
       }
       const bool live = __any_sync(kFull, T_prev.x != 0.0f || T_prev.y != 0.0f);
