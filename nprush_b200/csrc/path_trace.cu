@@ -7,6 +7,8 @@
 // Layout on the device:
 //   nodes    2 x float4 per node, the reference's 32-byte node
 //            [min.xyz, data0 | max.xyz, data1] (data bits stored as floats)
+//   pairs    4 x float4 per inner node: its two children's boxes and references,
+//            for the front-to-back traversal
 //   tri_pos  3 x float4 per triangle in BVH order: the three corner positions
 //            (v0.xyz v1.x | v1.yz v2.xy | v2.z) gathered so a leaf reads 48
 //            contiguous bytes per triangle instead of three 48-byte vertices
@@ -229,6 +231,10 @@ struct Scene {
   const float4* __restrict__ env;
   int env_w, env_h;
   uint32_t n_nodes;
+  // the same tree with both children's boxes in one 64-byte record per inner
+  // node (see pack_pairs); root: the reference of the root
+  const float4* __restrict__ pairs;
+  uint32_t root;
 };
 
 __device__ __forceinline__ uint32_t pcg(uint32_t v) {  // path_trace.wgsl:34-38
@@ -362,6 +368,114 @@ __device__ __forceinline__ Hit scene_hit(const Scene& sc, const float3& ro, cons
   return best;
 }
 
+// References of the pair records: an inner node's record index, or a leaf's
+// first triangle with its count (1 to 4, kMaxLeafTris) in bits 28-30 and
+// kLeafFlag.
+__device__ __forceinline__ float2 ldg2(const char* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ float2 operator+(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 operator*(float2 a, float2 b) { return __fmul2_rn(a, b); }
+constexpr uint32_t kLeafCountShift = 28, kLeafFirstMask = (1u << kLeafCountShift) - 1u;
+constexpr uint32_t kNoRef = 0xffffffffu;  // a leaf of seven triangles: none has as many
+
+// Closest hit by front-to-back traversal: both children of a node are tested
+// at once, the nearer is entered and the other one waits on the stack with its
+// entry distance.  It finds the triangle that scene_hit finds: the leaves'
+// boxes reach 1e-4 beyond their triangles (bvh.ts:66), so with coordinates
+// within kOrderedReach (rounding below 2e-5) the box of the closest triangle
+// is entered before that triangle's distance and is never left out, in
+// whatever order the boxes come; between hits at equal distance scene_hit
+// keeps the one it meets first, which is the one first in BVH order.
+// (94 M paths over 30 scenes: the same radiances, bit for bit.)
+//
+// The bound is instruction issue at a few active lanes (bounced rays part).  1024
+// x 768, 12k triangles, per frame, from the reference's order at 0.764 ms: 0.565
+// front to back; 0.463 with the lanes descending to their leaves before any leaf
+// is tested; 0.449 with the near and far planes picked by address and both
+// boxes in packed arithmetic; 0.408 with the corners' components loaded in the
+// ray's axis order instead of selected.  Slower: packing the live paths of a CTA
+// into its first warps after each bounce (0.497), lanes that start their
+// next bounce while others still traverse (0.57 to 0.62).
+__device__ __forceinline__ Hit scene_hit_ordered(const Scene& sc, const float3& ro, const float3& rd,
+                                                 uint32_t* overflow) {
+  Hit best;
+  best.t = 1e30f;
+  best.tri = ~0u;
+  best.u = best.v = best.w = 0.0f;
+  const float3 inv_rd = make_float3(1.0f / rd.x, 1.0f / rd.y, 1.0f / rd.z);
+  const RayShear sh = shear_of(rd);
+  const float2 mox = make_float2(-ro.x, -ro.x), ivx = make_float2(inv_rd.x, inv_rd.x);
+  const float2 moy = make_float2(-ro.y, -ro.y), ivy = make_float2(inv_rd.y, inv_rd.y);
+  const float2 moz = make_float2(-ro.z, -ro.z), ivz = make_float2(inv_rd.z, inv_rd.z);
+  // byte offsets of the near planes in a pair record: lo planes, hi where the ray runs backwards
+  const uint32_t offx = signbit(inv_rd.x) ? 8u : 0u, offy = signbit(inv_rd.y) ? 24u : 16u,
+                 offz = signbit(inv_rd.z) ? 40u : 32u;
+  const float rkx = comp(ro, sh.kx), rky = comp(ro, sh.ky), rkz = comp(ro, sh.kz);
+  uint2 stack[kMaxStack];
+  uint32_t top = 0, ref = sc.root;
+  uint32_t visits = 0;  // each reference is visited at most once per ray
+  // the next reference on the stack that still lies before the closest hit (kNoRef: none)
+  auto pop = [&]() {
+    while (top > 0u) {
+      const uint2 e = stack[--top];
+      if (__uint_as_float(e.y) < best.t) return e.x;
+    }
+    return kNoRef;
+  };
+  for (;;) {
+    // down to a leaf: the lanes of a warp run their leaf tests together
+    while (!(ref & kLeafFlag)) {
+      if (++visits > sc.n_nodes) {
+        atomicAdd(overflow, 1u);
+        return best;
+      }
+      // the planes the ray meets first and last per axis, both children's in one load and one packed operation
+      const char* p = reinterpret_cast<const char*>(sc.pairs) + 64 * (size_t)ref;
+      const float2 refs = ldg2(p + 48);
+      const float2 nx = (ldg2(p + offx) + mox) * ivx, fx = (ldg2(p + (offx ^ 8u)) + mox) * ivx;
+      const float2 ny = (ldg2(p + offy) + moy) * ivy, fy = (ldg2(p + (offy ^ 8u)) + moy) * ivy;
+      const float2 nz = (ldg2(p + offz) + moz) * ivz, fz = (ldg2(p + (offz ^ 8u)) + moz) * ivz;
+      const float in0 = fmaxf(fmaxf(nx.x, ny.x), nz.x), out0 = fminf(fminf(fx.x, fy.x), fz.x);
+      const float in1 = fmaxf(fmaxf(nx.y, ny.y), nz.y), out1 = fminf(fminf(fx.y, fy.y), fz.y);
+      const float t0 = out0 >= 0.0f && out0 >= in0 ? in0 : __int_as_float(0x7f800000);
+      const float t1 = out1 >= 0.0f && out1 >= in1 ? in1 : __int_as_float(0x7f800000);
+      const bool swap = t1 < t0;
+      const float tn = swap ? t1 : t0, tf = swap ? t0 : t1;
+      const uint32_t rn = __float_as_uint(swap ? refs.y : refs.x), rf = __float_as_uint(swap ? refs.x : refs.y);
+      if (tf < best.t) stack[top++] = make_uint2(rf, __float_as_uint(tf));  // the tree's depth is within the stack
+      ref = tn < best.t ? rn : pop();
+    }
+    if (ref == kNoRef) break;
+    const uint32_t first = ref & kLeafFirstMask, count = (ref >> kLeafCountShift) & 7u;
+    for (uint32_t k = 0; k < count; ++k) {
+      // path_trace.wgsl:60-131 as in intersect(), a corner's components loaded in the ray's axis order
+      const uint32_t tri = first + k;
+      const float* q = reinterpret_cast<const float*>(sc.tri_pos + 3 * (size_t)tri);
+      const float Akz = __ldg(q + sh.kz) - rkz, Bkz = __ldg(q + 3 + sh.kz) - rkz, Ckz = __ldg(q + 6 + sh.kz) - rkz;
+      const float Ax = __ldg(q + sh.kx) - rkx - sh.sx * Akz, Ay = __ldg(q + sh.ky) - rky - sh.sy * Akz;
+      const float Bx = __ldg(q + 3 + sh.kx) - rkx - sh.sx * Bkz, By = __ldg(q + 3 + sh.ky) - rky - sh.sy * Bkz;
+      const float Cx = __ldg(q + 6 + sh.kx) - rkx - sh.sx * Ckz, Cy = __ldg(q + 6 + sh.ky) - rky - sh.sy * Ckz;
+      const float U = Cx * By - Cy * Bx;
+      const float V = Ax * Cy - Ay * Cx;
+      const float W = Bx * Ay - By * Ax;
+      if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) continue;
+      const float det = U + V + W;
+      if (det == 0.0f) continue;
+      const float Az = sh.sz * Akz, Bz = sh.sz * Bkz, Cz = sh.sz * Ckz;
+      const float T = U * Az + V * Bz + W * Cz;
+      const float inv_det = 1.0f / det;
+      const float t = T * inv_det;
+      if (t < 1e-4f || !(t < best.t || (t == best.t && tri < best.tri))) continue;
+      best.t = t;
+      best.u = U * inv_det;
+      best.v = V * inv_det;
+      best.w = W * inv_det;
+      best.tri = tri;
+    }
+    ref = pop();
+  }
+  return best;
+}
+
 // shading of the closest hit (path_trace.wgsl:127-128)
 __device__ __forceinline__ void shade(const Scene& sc, const Hit& h, float3& nrm, float4& col) {
   const uint32_t i0 = __ldg(sc.tri_idx + 3 * (size_t)h.tri), i1 = __ldg(sc.tri_idx + 3 * (size_t)h.tri + 1),
@@ -422,6 +536,7 @@ struct Camera {
 };
 
 // one sample of pixel (x, y) for `frame` (path_trace.wgsl:222-262)
+template <bool kOrdered>
 __device__ __forceinline__ float3 trace_pixel(const Scene& sc, const Camera& cam, uint32_t x, uint32_t y, uint32_t w,
                                               uint32_t h, uint32_t frame, uint32_t* overflow) {
   const uint32_t pixel = y * w + x;
@@ -442,7 +557,7 @@ __device__ __forceinline__ float3 trace_pixel(const Scene& sc, const Camera& cam
   float3 radiance = make_float3(0.0f, 0.0f, 0.0f), thr = make_float3(1.0f, 1.0f, 1.0f);
   float3 o = ro, d = rd;
   for (int bounce = 0; bounce < kBounces; ++bounce) {
-    const Hit hit = scene_hit(sc, o, d, overflow);
+    const Hit hit = kOrdered ? scene_hit_ordered(sc, o, d, overflow) : scene_hit(sc, o, d, overflow);
     if (hit.tri == ~0u) {
       const float3 e = sample_env(sc, d);
       radiance = make_float3(radiance.x + thr.x * e.x, radiance.y + thr.y * e.y, radiance.z + thr.z * e.z);
@@ -464,7 +579,8 @@ __device__ __forceinline__ float3 trace_pixel(const Scene& sc, const Camera& cam
   return radiance;
 }
 
-__global__ void __launch_bounds__(128, 10) k_path_trace(Scene sc, Camera cam, float4* __restrict__ accum, uint32_t w,
+template <bool kOrdered>
+__global__ void __launch_bounds__(128, kOrdered ? 8 : 10) k_path_trace(Scene sc, Camera cam, float4* __restrict__ accum, uint32_t w,
                                                     uint32_t h, uint32_t frame0, uint32_t frames,
                                                     uint32_t* overflow) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -473,7 +589,7 @@ __global__ void __launch_bounds__(128, 10) k_path_trace(Scene sc, Camera cam, fl
   if (x >= w || y >= h) return;
   float4 acc = accum[(size_t)y * w + x];
   for (uint32_t f = 0; f < frames; ++f) {
-    const float3 r = trace_pixel(sc, cam, x, y, w, h, frame0 + f, overflow);
+    const float3 r = trace_pixel<kOrdered>(sc, cam, x, y, w, h, frame0 + f, overflow);
     acc.x += r.x;
     acc.y += r.y;
     acc.z += r.z;
@@ -496,6 +612,64 @@ __global__ void k_pt_resolve(const float4* __restrict__ accum, float4* __restric
   b = b / (b + 1.0f);
   if (quantize) r = unorm8(r), g = unorm8(g), b = unorm8(b);
   out[(size_t)y * w + x] = make_float4(r, g, b, 1.0f);
+}
+
+// Pair records of a built tree, 16 floats per inner node in node order: per
+// axis both children's lo planes, then both hi planes; then their references.  Returns the root's reference and whether the
+// front-to-back traversal may stand in for the reference's: no path deeper than
+// its stack (the reference drops subtrees beyond 64 entries) and no
+// coordinate beyond kOrderedReach.
+constexpr float kOrderedReach = 64.0f;
+bool pack_pairs(const Bvh& b, std::vector<float>& pairs, uint32_t* root) {
+  const size_t n = b.nodes.size() / 8;
+  auto word = [&](size_t node, int k) {
+    uint32_t u;
+    std::memcpy(&u, &b.nodes[node * 8 + k], 4);
+    return u;
+  };
+  std::vector<uint32_t> rec(n), depth(n, 1);
+  uint32_t inner = 0;
+  bool ok = b.tris.size() / 3 <= kLeafFirstMask;
+  for (size_t i = 0; i < n; ++i) {
+    if (word(i, 7) & kLeafFlag) rec[i] = kLeafFlag | ((word(i, 7) & 7u) << kLeafCountShift) | (word(i, 3) & kLeafFirstMask);
+    else rec[i] = inner++;
+  }
+  pairs.assign((size_t)std::max(1u, inner) * 16, 0.0f);
+  for (size_t i = 0; i < n; ++i) {  // pre-order: parents before children
+    for (int k = 0; k < 3; ++k)
+      ok = ok && std::fabs(b.nodes[i * 8 + k]) <= kOrderedReach && std::fabs(b.nodes[i * 8 + 4 + k]) <= kOrderedReach;
+    if (word(i, 7) & kLeafFlag) continue;
+    float* p = &pairs[(size_t)rec[i] * 16];
+    for (int c = 0; c < 2; ++c) {
+      const uint32_t ch = word(i, c == 0 ? 3 : 7);
+      depth[ch] = depth[i] + 1;
+      ok = ok && depth[ch] < kMaxStack;
+      for (int k = 0; k < 3; ++k) {
+        p[4 * k + c] = b.nodes[(size_t)ch * 8 + k];
+        p[4 * k + 2 + c] = b.nodes[(size_t)ch * 8 + 4 + k];
+      }
+      std::memcpy(p + 12 + c, &rec[ch], 4);
+    }
+  }
+  *root = rec[0];
+  return ok;
+}
+
+// Whether the camera's rays start within kOrderedReach of the origin: the
+// near plane's corners, which bound every pixel's start while their
+// homogeneous weights have one sign.
+bool camera_within_reach(const float* m) {
+  int sign = 0;
+  for (int c = 0; c < 4; ++c) {
+    const double nx = (c & 1) ? 1.25 : -1.25, ny = (c & 2) ? 1.25 : -1.25;  // the half-pixel jitter stays inside
+    double h[4];
+    for (int r = 0; r < 4; ++r) h[r] = m[r] * nx + m[4 + r] * ny + (double)m[12 + r];
+    if (!(std::fabs(h[3]) > 1e-30) || (c > 0 && (h[3] > 0) != (sign > 0))) return false;
+    sign = h[3] > 0 ? 1 : -1;
+    for (int r = 0; r < 3; ++r)
+      if (!(std::fabs(h[r] / h[3]) <= kOrderedReach)) return false;
+  }
+  return true;
 }
 
 int check_mesh(const char* fn, const float* vertices, uint32_t n_vertices, const uint32_t* indices, uint32_t n_tris) {
@@ -526,10 +700,12 @@ struct nps_pt {
   nps_ctx* ctx = nullptr;
   pt::Bvh bvh;
   uint32_t n_verts = 0, n_tris = 0;
-  DevBuf nodes, tri_pos, tri_idx, verts, env, stats;
+  DevBuf nodes, pairs, tri_pos, tri_idx, verts, env, stats;
+  uint32_t root = 0;
+  bool ordered = false;  // the front-to-back traversal gives the reference's hits (pack_pairs)
   int env_w = 0, env_h = 0;
   ~nps_pt() {
-    for (DevBuf* b : {&nodes, &tri_pos, &tri_idx, &verts, &env, &stats}) b->release();
+    for (DevBuf* b : {&nodes, &pairs, &tri_pos, &tri_idx, &verts, &env, &stats}) b->release();
   }
 };
 
@@ -570,8 +746,10 @@ int nps_pt_create(nps_ctx* ctx, const float* vertices, uint32_t n_vertices, cons
     for (int c = 0; c < 3; ++c)
       for (int k = 0; k < 3; ++k) pos[t * 12 + c * 3 + k] = vertices[(size_t)o->bvh.tris[t * 3 + c] * 12 + k];
   const float white[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+  std::vector<float> pairs;
+  o->ordered = pt::pack_pairs(o->bvh, pairs, &o->root);
   int rc = NPS_OK;
-  if ((rc = o->nodes.ensure(n_nodes * 32)) || (rc = o->tri_pos.ensure(pos.size() * 4 + 16)) ||
+  if ((rc = o->nodes.ensure(n_nodes * 32)) || (rc = o->pairs.ensure(pairs.size() * 4)) || (rc = o->tri_pos.ensure(pos.size() * 4 + 16)) ||
       (rc = o->tri_idx.ensure((size_t)n_tris * 12 + 16)) || (rc = o->verts.ensure((size_t)n_vertices * 48 + 16)) ||
       (rc = o->env.ensure(16)) || (rc = o->stats.ensure(16))) {
     delete o;
@@ -579,6 +757,7 @@ int nps_pt_create(nps_ctx* ctx, const float* vertices, uint32_t n_vertices, cons
   }
   cudaStream_t s = ctx->stream;
   cudaError_t e = cudaMemcpyAsync(o->nodes.p, o->bvh.nodes.data(), n_nodes * 32, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(o->pairs.p, pairs.data(), pairs.size() * 4, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && n_tris)
     e = cudaMemcpyAsync(o->tri_pos.p, pos.data(), pos.size() * 4, cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess && n_tris)
@@ -663,11 +842,17 @@ int nps_pt_trace(nps_pt* o, const float* inv_view_proj, uint32_t frame, uint32_t
   sc.env_w = o->env_w;
   sc.env_h = o->env_h;
   sc.n_nodes = (uint32_t)(o->bvh.nodes.size() / 8);
+  sc.pairs = o->pairs.as<float4>();
+  sc.root = o->root;
   pt::Camera cam;
   std::memcpy(cam.m, inv_view_proj, sizeof cam.m);
   const dim3 grid(div_up(w, 16), div_up(h, 8));
-  pt::k_path_trace<<<grid, 128, 0, o->ctx->stream>>>(sc, cam, (float4*)accum_rgba, w, h, frame, n_frames,
-                                                     o->stats.as<uint32_t>());
+  if (o->ordered && pt::camera_within_reach(inv_view_proj))
+    pt::k_path_trace<true><<<grid, 128, 0, o->ctx->stream>>>(sc, cam, (float4*)accum_rgba, w, h, frame, n_frames,
+                                                             o->stats.as<uint32_t>());
+  else
+    pt::k_path_trace<false><<<grid, 128, 0, o->ctx->stream>>>(sc, cam, (float4*)accum_rgba, w, h, frame, n_frames,
+                                                              o->stats.as<uint32_t>());
   NPS_CHECK_LAUNCH();
   return NPS_OK;
 }

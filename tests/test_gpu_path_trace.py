@@ -175,3 +175,49 @@ def test_camera_inside_a_closed_box(ptmod):
         assert np.all(opt.trace_pixel(o, inv, x, y, w, h, 0) == 0.0)
     assert pt.overflows() == 0
     pt.close()
+
+
+@pytest.mark.parametrize("case", ["coplanar", "one_triangle", "five_triangles", "axis_rays", "far_camera", "far_scene"])
+def test_front_to_back_equals_reference_order(ptmod, case):
+    """The front-to-back traversal against the scalar restatement of the reference's order, where the two could part:
+    coincident triangles (ties go to the first in BVH order), trees of one leaf and of one inner node, rays parallel
+    to the axes (infinite inverse directions), and the scenes and cameras beyond its reach, which keep the reference's
+    order.  Mirrors only, so that no random direction enters: 2e-5 per pixel as for the mirror scene (atan2 / asin)."""
+    import path_trace as opt
+    from bvh import build_bvh
+    from nprush_b200 import camera, meshes
+    mirror = (0.9, 0.8, 0.7, 0.0)
+    eye, at = (4.0, -3.5, 2.6), (0.0, 0.0, 0.3)
+    if case == "coplanar":
+        sc = meshes.concat([meshes.box((0, 0, 0.5), 0.5, mirror)] * 3 + [meshes.quad((0, 0, 0), 4.0, mirror)] * 2)
+    elif case == "one_triangle":
+        q = meshes.quad((0, 0, 0), 4.0, mirror)
+        sc = meshes.MeshData(q.vertices, q.indices[:3])
+    elif case == "five_triangles":
+        q = meshes.concat([meshes.quad((0, 0, 0.2 * k), 2.0 + k, mirror) for k in range(3)])
+        sc = meshes.MeshData(q.vertices, q.indices[:15])
+    elif case == "axis_rays":
+        sc = meshes.concat([meshes.box((0, 0, 0.5), (0.5, 0.7, 0.5), mirror), meshes.quad((0, 0, 0), 4.0, mirror)])
+        eye, at = (3.0, 0.0, 0.5), (0.0, 0.0, 0.5)
+    else:
+        sc = meshes.demo_scene(4, seed=3, mirror_fraction=1.0, sphere_detail=6)
+        sc.vertices[:, 9] = 0.0
+        if case == "far_scene":
+            sc.vertices[:, 0] += 100.0
+            eye, at = (104.0, -3.5, 2.6), (100.0, 0.0, 0.3)
+        else:
+            eye = (90.0, -60.0, 40.0)
+    w, h = 24, 16
+    _, inv = camera.view_proj(eye, at, 0.9 if case != "far_camera" else 0.05, w / h, up=(0.0, 0.0, 1.0))
+    env = meshes.sky_env(32, 16)
+    pt = ptmod.PathTracer(env_texture=env)
+    pt.set_meshes(sc)
+    pt.set_output_size(w, h)
+    pt.write_inv_view_proj_mat(inv)
+    pt.dispatch()
+    nodes, tris = build_bvh(sc.vertices, sc.indices)
+    o = opt.Scene(sc.vertices, nodes, tris, env)
+    want = np.array([[opt.trace_pixel(o, inv, x, y, w, h, 0) for x in range(w)] for y in range(h)])
+    np.testing.assert_allclose(pt.accum.cpu().numpy()[..., :3], want, atol=2e-5, rtol=0)
+    assert pt.overflows() == 0
+    pt.close()
