@@ -96,3 +96,26 @@ def test_blur_manager_classes(tg):
     out = torch.zeros_like(src)
     tg.GpuDepthAwareBlurPipelineManager().blur(src, z, out, w, h, 3)
     check_q(out.cpu().numpy(), d[f"depth_blur{k}"])
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 15), (32, 16), (129, 33)])
+@pytest.mark.parametrize("radius", [0, 1, 5, 25, 26, 80])
+def test_tiled_blurs(tg, w, h, radius):
+    """The tiled kernels at the edges of their tiles (32 x 32, 128 x 8 and 32 x 16 pixels) and of the radii they take
+    (25 for the bilateral blur, 79 down the columns), against the numpy restatement.  Tolerance: its sums and the
+    device's round once per tap, 6e-8 of the largest tap each, on top of the stored floats' 2e-6."""
+    import preprocess as pp
+    rng = np.random.default_rng(w + radius)
+    color = rng.random((h, w, 4), dtype=np.float32)
+    depth = rng.random((h, w, 4), dtype=np.float32)
+    c, z = torch.from_numpy(color).cuda(), torch.from_numpy(depth).cuda()
+    out = torch.zeros_like(c)
+    sigma = max(0.5, radius / 2)
+    for direction in ((1, 0), (0, 1)):
+        tg.blur(c, out, direction, radius, sigma, tg.SRGB_IN)
+        want = pp.blur(color, direction, radius, tg.SRGB_IN, sigma)
+        np.testing.assert_allclose(out.cpu().numpy(), want, atol=2e-6 + 6e-8 * (2 * radius + 1), rtol=0)
+    if radius <= 26:
+        tg.depth_aware_blur(c, z, out, radius)
+        want = pp.depth_aware_blur(color, depth, radius)
+        np.testing.assert_allclose(out.cpu().numpy(), want, atol=2e-6 + 6e-8 * (2 * radius + 1) ** 2, rtol=0)
