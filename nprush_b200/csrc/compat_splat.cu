@@ -445,12 +445,12 @@ struct __align__(16) RasterSmem {
 // and log's by a few ULP: the reference's shaders are not bit-defined here.
 __device__ __forceinline__ float lg2_approx(float x) {
   float y;
-  asm("lg2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
-  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 constexpr float kLog2e = 1.4426950408889634f;

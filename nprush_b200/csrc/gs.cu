@@ -192,6 +192,15 @@ __device__ __forceinline__ uint32_t warp_sum9_index(uint32_t lane) {
   return (uint32_t)(0xfff8f765ff43f210ull >> (4u * ((lane >> 1) & 15u))) & 15u;
 }
 
+// exp(x) for x in the range the rasters evaluate, [-6, 0]: __expf without the
+// scaling that it adds for results near the smallest floats (the same bits
+// here; three instructions fewer per pixel and pair)
+__device__ __forceinline__ float exp_raster(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  return y;
+}
+
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // ------------------------------------------------------------ preprocess
@@ -512,7 +521,7 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1280 / (256 / PPT) : 1) 
         float cu, cw;
         const float power = gs_power(a, b.x, dx, dy, cu, cw);
         if (power > 0.0f || power < pmin) continue;  // pmin: alpha < 1/255 below it (see pix_bwd_pair)
-        const float alpha = fminf(kAlphaMax, b.y * __expf(power));
+        const float alpha = fminf(kAlphaMax, b.y * exp_raster(power));
         if (alpha < kAlphaMin) continue;
         const float test_T = T[k] * (1.0f - alpha);
         if (test_T < kTMin) {
@@ -950,7 +959,7 @@ __global__ void __launch_bounds__(kThreads) k_bwd(const Rec* __restrict__ recs, 
     float u, w;
     const float power = gs_power(a, b.x, dx, dy, u, w);
     if (power > 0.0f) return false;
-    const float G = __expf(power);
+    const float G = exp_raster(power);
     const float araw = b.y * G;
     const float alpha = fminf(kAlphaMax, araw);
     if (alpha < kAlphaMin) return false;
@@ -1112,7 +1121,7 @@ __device__ __forceinline__ bool pix_bwd_pair(PixBwd& s, const float4& a, const f
   // implies alpha < 1/255, so skipping those pixels before the exponential
   // leaves every decision of the alpha test below unchanged
   if (power > 0.0f || power < -0.5f * c4.y) return false;
-  const float G = __expf(power);
+  const float G = exp_raster(power);
   const float araw = b.y * G;
   const float alpha = fminf(kAlphaMax, araw);
   if (alpha < kAlphaMin) return false;

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(TS * TS / PPT + 32) k_fwd_ws(
             float cu, cw;
             const float power = gs_power(a, b.x, dx, dy, cu, cw);
             if (power > 0.0f || power < pmin) continue;  // alpha < 1/255 below pmin
-            const float alpha = fminf(kAlphaMax, b.y * __expf(power));
+            const float alpha = fminf(kAlphaMax, b.y * exp_raster(power));
             if (alpha < kAlphaMin) continue;
             const float test_T = T[k] * (1.0f - alpha);
             if (test_T < kTMin) {
