@@ -453,6 +453,11 @@ __device__ __forceinline__ float ex2_approx(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kHalfLn2 = 0.34657359027997264f;
 
@@ -542,7 +547,7 @@ __device__ __forceinline__ uint2 strip_masks(const float (*fwd)[kFwd], uint32_t 
     const float lx = x0 - f0.x, hx = x1 - f0.x, ly = y0 - f0.y, hy = y1 - f0.y;
     float q = 0.0f;
     if (!(lx <= 0.0f && hx >= 0.0f && ly <= 0.0f && hy >= 0.0f) && A > 0.0f && C > 0.0f) {
-      const float ba = -B * __fdividef(1.0f, A), bc = -B * __fdividef(1.0f, C);
+      const float ba = -B * rcp_approx(A), bc = -B * rcp_approx(C);
       const float yl = clampf(bc * lx, ly, hy), yh = clampf(bc * hx, ly, hy);
       const float xl = clampf(ba * ly, lx, hx), xh = clampf(ba * hy, lx, hx);
       const float B2 = 2.0f * B;
@@ -801,7 +806,7 @@ __global__ void __launch_bounds__(kRasterThreads, 6) k_raster(RasterArgs a) {
         collect(sum2(p.da * e.a_un * kFpCol), 7);
         const float2 d_depth = p.dD_T * al;
         // r^(a - 2) = r^a / r^2
-        const float2 rp = make_float2(__fdividef(e.rpa.x, e.r2c.x), __fdividef(e.rpa.y, e.r2c.y));
+        const float2 rp = e.rpa * make_float2(rcp_approx(e.r2c.x), rcp_approx(e.r2c.y));
         const float2 kk = p.d_power * (rp * (-f[6] * f[5]));
         // minus dL/d(screen offset); minus signs are exact wherever they stand
         const float2 nx = kk * e.spx * -1.0f, ny = kk * e.spy * -1.0f;

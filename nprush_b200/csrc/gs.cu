@@ -58,6 +58,14 @@ constexpr float kSsimC1 = 0.01f * 0.01f, kSsimC2 = 0.03f * 0.03f;
 
 __constant__ float c_ssim_w[kSsimWin];
 
+// 1 / x on the special-function unit for x well inside the normal range
+// (__fdividef(1, x)'s bits without its scaling for extreme x)
+__device__ __forceinline__ float rcp_normal(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 struct Rec {  // projected record, 3 x float4 = 48 B
   float4 a;   // u, v, conic a, conic b
   float4 b;   // conic c, opacity, r, g
@@ -76,7 +84,7 @@ __device__ __forceinline__ bool rec_misses_box(const float4& a, float cc, const 
   if (lx <= 0.0f && hx >= 0.0f && ly <= 0.0f && hy >= 0.0f) return false;  // centre inside
   const float ca = a.z, cb = a.w;
   // the form's minimum on each edge (the other coordinate clamped to the edge)
-  const float icc = cc > 0.0f ? 1.0f / cc : 0.0f, ica = ca > 0.0f ? 1.0f / ca : 0.0f;
+  const float icc = cc > 0.0f ? rcp_normal(cc) : 0.0f, ica = ca > 0.0f ? rcp_normal(ca) : 0.0f;
   const float y_l = fminf(fmaxf(-cb * lx * icc, ly), hy), y_h = fminf(fmaxf(-cb * hx * icc, ly), hy);
   const float x_l = fminf(fmaxf(-cb * ly * ica, lx), hx), x_h = fminf(fmaxf(-cb * hy * ica, lx), hx);
   const float q1 = ca * lx * lx + 2.0f * cb * lx * y_l + cc * y_l * y_l;
@@ -677,7 +685,7 @@ __global__ void __launch_bounds__(256) k_ssim_fwd2(const float4* __restrict__ im
       const float A1 = 2.0f * mx * my + kSsimC1, A2 = 2.0f * sxy + kSsimC2;
       const float B1 = mx * mx + my * my + kSsimC1, B2 = sxx + syy + kSsimC2;
       // two fast reciprocals instead of five divisions (B1, B2 >= C1, C2 > 0)
-      const float iB1 = __fdividef(1.0f, B1), iB2 = __fdividef(1.0f, B2), iB = iB1 * iB2;
+      const float iB1 = rcp_normal(B1), iB2 = rcp_normal(B2), iB = iB1 * iB2;
       const float sv = (A1 * A2) * iB;
       ss += sv;
       const float dLds = -lambda * inv_norm;
@@ -1126,7 +1134,7 @@ __device__ __forceinline__ bool pix_bwd_pair(PixBwd& s, const float4& a, const f
   const float alpha = fminf(kAlphaMax, araw);
   if (alpha < kAlphaMin) return false;
   // one reciprocal serves both divisions (approximate, ~2 ulp; alpha <= 0.99)
-  const float inv1ma = __fdividef(1.0f, 1.0f - alpha);
+  const float inv1ma = rcp_normal(1.0f - alpha);
   s.T = s.T * inv1ma;
   const float wgt = alpha * s.T;
   // colour behind this pair, dotted with dL/dpixel: last_alpha * last + (1 - last_alpha) * acc
