@@ -212,19 +212,49 @@ __device__ __forceinline__ float exp_raster(float x) {
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // ------------------------------------------------------------ preprocess
+// What binning needs of a projected record: its tile rectangle (x0 | x1 << 16,
+// y0 | y1 << 16), the mask of the rectangle's tiles that get a pair (rectangles
+// of at most 32 tiles) and the number of pairs.  One 16-byte word, because the
+// binning reads it in depth order, that is at random.
+__device__ __forceinline__ uint32_t rect_tiles(uint32_t x, uint32_t y) {
+  return ((x >> 16) - (x & 0xffffu)) * ((y >> 16) - (y & 0xffffu));
+}
+
+// A block projects group Gaussians for up to eight views at a time (thread t:
+// Gaussian t % group, view t / group).  Records of 256 and 48 bytes read and
+// written one per lane touch a cache line per lane and instruction, and the L1's
+// tag lookups bound the kernel; so the parameter records come through shared
+// memory, once for all views, and the projected ones leave through it, in whole
+// lines.  The shared strides (17 and 3 float4) keep 16-byte accesses free of
+// bank conflicts.  200k Gaussians, SH3, 8 views: 110 -> 78 us; 1M: 500 -> 336 us
+// (bytes that it cannot do without: 36 and 181 us).
+constexpr uint32_t kPreStride = 17;  // float4 per staged parameter record (16 and a pad)
+constexpr size_t pre_smem(uint32_t group, uint32_t threads) {
+  return (size_t)group * kPreStride * 16 + (size_t)threads * sizeof(Rec);
+}
 template <int DEG>
 __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ params, uint32_t n,
                                                     const float* __restrict__ views, uint32_t nv, uint32_t W,
                                                     uint32_t H, uint32_t tiles_x, uint32_t tiles_y, float inv_tile,
-                                                    Rec* __restrict__ recs, uint32_t* __restrict__ counts,
-                                                    uint2* __restrict__ rects, uint32_t* __restrict__ dkeys,
-                                                    uint32_t* __restrict__ dvals, uint32_t* __restrict__ ecounts,
-                                                    uint32_t* __restrict__ tmasks) {
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= nv * n) return;
-  const uint32_t v = g / n, i = g - v * n;
+                                                    uint32_t group, Rec* __restrict__ recs,
+                                                    uint32_t* __restrict__ counts, uint4* __restrict__ bins,
+                                                    uint32_t* __restrict__ dkeys, uint32_t* __restrict__ dvals) {
+  extern __shared__ float4 sm_pre[];
+  const uint32_t tv = threadIdx.x / group, gi = threadIdx.x - tv * group, lane = threadIdx.x & 31u;
+  const uint32_t i0 = blockIdx.x * group, i = i0 + gi, v = blockIdx.y * (blockDim.x / group) + tv;
+  constexpr uint32_t kUsed4 = 3 + (3 * (DEG + 1) * (DEG + 1) + 3) / 4;  // float4 of a record that are read
+  {
+    const float4* src = reinterpret_cast<const float4*>(params) + (size_t)i0 * (kP / 4);
+    const uint32_t have = min(group, n - i0) * (kP / 4);
+    for (uint32_t e = threadIdx.x; e < have; e += blockDim.x)
+      if ((e & 15u) < kUsed4) sm_pre[(e >> 4) * kPreStride + (e & 15u)] = __ldg(src + e);
+  }
+  __syncthreads();
+  if (v >= nv || i0 + (gi & ~31u) >= n) return;  // whole warps
+  const bool live = i < n;
+  const uint32_t g = v * n + (live ? i : n - 1);
   // the record in 16-byte loads (floats 0..11, then the SH coefficients if visible)
-  const float4* p4 = reinterpret_cast<const float4*>(params + (size_t)i * kP);
+  const float4* p4 = sm_pre + (live ? gi : n - 1 - i0) * kPreStride;
   const float4 q0 = p4[0], q1 = p4[1], q2 = p4[2];
   const float* view = views + (size_t)v * kViewRec;
   float mean[3] = {q0.x, q0.y, q0.z};
@@ -310,47 +340,73 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
       }
     }
   }
-  recs[g] = r;
+  // the warp's 32 records are consecutive: 96 float4
+  float4* out = sm_pre + group * kPreStride + (threadIdx.x & ~31u) * 3;
+  out[3 * lane] = r.a;
+  out[3 * lane + 1] = r.b;
+  out[3 * lane + 2] = r.c;
+  __syncwarp();
+  {
+    const uint32_t first = i - lane, have = 3u * min(32u, n - first);
+    float4* dst = reinterpret_cast<float4*>(recs + (size_t)v * n + first);
+#pragma unroll
+    for (uint32_t e = 0; e < 3; ++e)
+      if (e * 32 + lane < have) dst[e * 32 + lane] = out[e * 32 + lane];
+  }
+  if (!live) return;
   counts[g] = cnt;
-  ecounts[g] = ecnt;
-  tmasks[g] = tmask;
-  rects[g] = rect;
+  bins[g] = make_uint4(rect.x, rect.y, tmask, ecnt);
   dkeys[g] = key;
   dvals[g] = g;
 }
 
-__global__ void k_gather_counts(const uint32_t* __restrict__ sorted_g, const uint32_t* __restrict__ counts,
-                                uint32_t m, uint32_t* __restrict__ out) {
+__global__ void k_gather_counts(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins, uint32_t m,
+                                uint32_t* __restrict__ out) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < m) out[j] = counts[sorted_g[j]];
+  if (j < m) out[j] = bins[sorted_g[j]].w;
+}
+
+// Index of the k-th set bit of m (k below its population count), by halving.
+__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
+  uint32_t at = 0;
+#pragma unroll
+  for (uint32_t step = 16; step > 0; step >>= 1) {
+    const uint32_t c = __popc(m & ((1u << step) - 1u));
+    if (k >= c) {
+      k -= c;
+      at += step;
+      m >>= step;
+    }
+  }
+  return at;
 }
 
 // One warp per 32 consecutive depth-sorted (view, Gaussian) entries: their
 // pairs are one contiguous output range, written 32 consecutive slots at a
 // time (coalesced); each lane finds the entry owning its slot by a binary
 // search over the warp's offsets (shuffles).  Output identical to writing
-// each entry's tile rectangle row by row.
-__global__ void __launch_bounds__(256) k_emit(const uint32_t* __restrict__ sorted_g,
-                                              const uint32_t* __restrict__ ecounts,
-                                              const uint32_t* __restrict__ offsets, const uint2* __restrict__ rects,
-                                              const uint32_t* __restrict__ tmasks, uint32_t m, uint32_t n,
+// each entry's tile rectangle row by row.  An entry's fields are one 16-byte word
+// and its slots need no integer division: 84 -> 52 us at 11.5 M pairs, 310 -> 187
+// us at 38 M.
+__global__ void __launch_bounds__(256) k_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
+                                              const uint32_t* __restrict__ offsets, uint32_t m, uint32_t n,
                                               uint32_t tiles_x, uint32_t num_tiles, uint32_t cap,
                                               uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   if (__all_sync(0xffffffffu, j >= m)) return;
-  uint32_t g = 0, c = 0, off = 0xffffffffu, x0 = 0, w = 1, y0 = 0, tm = 0;
+  // per entry: its record, first slot, tile mask (all ones: every tile), key of its first tile and row width
+  uint32_t g = 0, c = 0, off = 0xffffffffu, tm = 0, key0 = 0, w = 1;
   if (j < m) {
     g = sorted_g[j];
-    c = ecounts[g];
     off = offsets[j];
-    const uint2 r = rects[g];
-    x0 = r.x & 0xffffu;
-    w = max((r.x >> 16) - x0, 1u);
-    y0 = r.y & 0xffffu;
-    // boxes of at most 32 tiles emit only the tiles of their mask
-    if (((r.y >> 16) - y0) * ((r.x >> 16) - x0) <= 32u) tm = tmasks[g];
-    else tm = 0xffffffffu;
+    const uint4 b = bins[g];
+    c = b.w;
+    const uint32_t x0 = b.x & 0xffffu;
+    w = max((b.x >> 16) - x0, 1u);
+    tm = rect_tiles(b.x, b.y) <= 32u ? b.z : 0xffffffffu;
+    key0 = (g / n) * num_tiles + (b.y & 0xffffu) * tiles_x + x0;
   }
+  const float iw = 1.0f / (float)w;
   const uint32_t start = __shfl_sync(0xffffffffu, off, 0);
   const uint32_t end = __reduce_max_sync(0xffffffffu, j < m ? off + c : 0u);
   for (uint32_t base = start; base < end; base += 32) {
@@ -363,18 +419,18 @@ __global__ void __launch_bounds__(256) k_emit(const uint32_t* __restrict__ sorte
       if (o2 <= sl) L += step;
     }
     const uint32_t gL = __shfl_sync(0xffffffffu, g, L), oL = __shfl_sync(0xffffffffu, off, L);
-    const uint32_t x0L = __shfl_sync(0xffffffffu, x0, L), wL = __shfl_sync(0xffffffffu, w, L);
-    const uint32_t y0L = __shfl_sync(0xffffffffu, y0, L), tmL = __shfl_sync(0xffffffffu, tm, L);
+    const uint32_t kL = __shfl_sync(0xffffffffu, key0, L), wL = __shfl_sync(0xffffffffu, w, L);
+    const uint32_t tmL = __shfl_sync(0xffffffffu, tm, L);
+    const float iwL = __shfl_sync(0xffffffffu, iw, L);
     if (sl < end && sl < cap) {
-      uint32_t local = sl - oL;
-      if (tmL != 0xffffffffu) {
-        // the local-th set bit of the mask is the tile's index in the box
-        uint32_t mk = tmL;
-        for (uint32_t t = 0; t < local; ++t) mk &= mk - 1u;
-        local = (uint32_t)(__ffs(mk) - 1);
-      }
-      const uint32_t ry = local / wL;
-      keys[sl] = (gL / n) * num_tiles + (y0L + ry) * tiles_x + x0L + (local - ry * wL);
+      const uint32_t k = sl - oL;
+      // the tile's index in the box: the k-th of the mask, or the k-th
+      const uint32_t local = tmL != 0xffffffffu ? nth_set_bit(tmL, k) : k;
+      // its row: exact, one correction on the float quotient
+      uint32_t ry = (uint32_t)((float)local * iwL);
+      if (ry * wL > local) --ry;
+      else if ((ry + 1) * wL <= local) ++ry;
+      keys[sl] = kL + ry * tiles_x + (local - ry * wL);
       vals[sl] = gL;
     }
   }
@@ -1394,10 +1450,12 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 1) k_project_bwd(const float* _
   bool one_has = false;
   for (uint32_t v = sub; live && v < nv; v += 8) {
     const size_t gi = (size_t)v * n + i;
+    // the gradient record (48 B, 16-byte aligned) is fetched with the count, not after it
+    const float4* gr = reinterpret_cast<const float4*>(g2 + gi * kG2);
+    const float4 r0 = __ldg(gr), r1 = __ldg(gr + 1), r2 = __ldg(gr + 2);
     if (counts[gi] == 0) continue;
-    const float* gr = g2 + gi * kG2;
-    const float du = gr[0], dv = gr[1], dca = gr[2], dcb = gr[3], dcc = gr[4], dop = gr[5];
-    const float dcol[3] = {gr[6], gr[7], gr[8]};
+    const float du = r0.x, dv = r0.y, dca = r0.z, dcb = r0.w, dcc = r1.x, dop = r1.y;
+    const float dcol[3] = {r1.z, r1.w, r2.x};
     const float* view = views + (size_t)v * kViewRec;
     Proj<float> P;
     project<float>(view, mean, ls, q, (float)W, (float)H, kLowpass, P);
@@ -1871,7 +1929,7 @@ struct nps_gs {
   uint32_t nv = 0;
   DevBuf views, tids;
   // forward state
-  DevBuf recs, counts, ecounts, tmasks, rects, dkeys, dvals, cnt_sorted, offsets, total, mcount, keys, vals, ranges;
+  DevBuf recs, counts, bins, dkeys, dvals, cnt_sorted, offsets, total, mcount, keys, vals, ranges;
   DevBuf img, ncontrib;
   DevBuf maps, partial, loss, dimg, g2;
   SortWork sw_depth, sw_tile;
@@ -2063,7 +2121,7 @@ int nps_gs_destroy(nps_gs* o) {
     b->release();
   for (DevBuf* b : {&o->tile_last, &o->ws_order_f, &o->ws_order_b, &o->ws_q}) b->release();
   for (DevBuf* b : {&o->params, &o->grads, &o->am, &o->av, &o->adc_grad, &o->adc_denom, &o->tgt_own, &o->views,
-                    &o->tids, &o->recs, &o->counts, &o->ecounts, &o->tmasks, &o->rects, &o->dkeys, &o->dvals,
+                    &o->tids, &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals,
                     &o->cnt_sorted, &o->offsets, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->img,
                     &o->ncontrib, &o->maps,
                     &o->partial, &o->loss, &o->dimg, &o->g2, &o->sw_depth.hist, &o->sw_depth.partial,
@@ -2526,9 +2584,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
   }
   NPS_TRY(o->recs.ensure(sizeof(gs::Rec) * (M + 1)));
   NPS_TRY(o->counts.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->ecounts.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->tmasks.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->rects.ensure(sizeof(uint2) * (M + 1)));
+  NPS_TRY(o->bins.ensure(sizeof(uint4) * (M + 1)));
   NPS_TRY(o->dkeys.ensure(sizeof(uint32_t) * (M + 1)));
   NPS_TRY(o->dvals.ensure(sizeof(uint32_t) * (M + 1)));
   NPS_TRY(o->cnt_sorted.ensure(sizeof(uint32_t) * (M + 1)));
@@ -2543,13 +2599,14 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
   const uint32_t* vs = o->counts.as<uint32_t>();
   if (M > 0) {
     { StageTimer t_pre(o, ST_PRE);
-#define NPS_PRE(D)                                                                                          \
-  gs::k_preprocess<D><<<div_up(M, 256), 256, 0, s>>>(o->params.as<float>(), n, o->views.as<float>(), nv, W, H, \
-                                                      tiles_x, tiles_y, 1.0f / (float)o->tile,                  \
-                                                      o->recs.as<gs::Rec>(),                                    \
-                                                      o->counts.as<uint32_t>(), o->rects.as<uint2>(),           \
-                                                      o->dkeys.as<uint32_t>(), o->dvals.as<uint32_t>(),         \
-                                                      o->ecounts.as<uint32_t>(), o->tmasks.as<uint32_t>())
+    // whole warps of one view; at most 256 threads
+    const uint32_t vb = std::min(nv, 8u), group = vb <= 4 ? 64u : 32u;
+    const dim3 pgrid(div_up(n, group), div_up(nv, vb));
+#define NPS_PRE(D)                                                                                              \
+  gs::k_preprocess<D><<<pgrid, group * vb, gs::pre_smem(group, group * vb), s>>>(                               \
+      o->params.as<float>(), n, o->views.as<float>(), nv, W, H, tiles_x, tiles_y, 1.0f / (float)o->tile, group, \
+      o->recs.as<gs::Rec>(), o->counts.as<uint32_t>(), o->bins.as<uint4>(), o->dkeys.as<uint32_t>(),            \
+      o->dvals.as<uint32_t>())
     switch (o->sh_deg) {
       case 0: NPS_PRE(0); break;
       case 1: NPS_PRE(1); break;
@@ -2564,7 +2621,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
     NPS_TRY(radix_sort_u32(o->dkeys.as<uint32_t>(), o->dvals.as<uint32_t>(), o->mcount.as<uint32_t>(), (uint32_t)M, 32,
                            o->sw_depth, s, &dk, &dv)); }
     o->sorted_vals = dv;
-    gs::k_gather_counts<<<div_up(M, 256), 256, 0, s>>>(dv, o->ecounts.as<uint32_t>(), (uint32_t)M,
+    gs::k_gather_counts<<<div_up(M, 256), 256, 0, s>>>(dv, o->bins.as<uint4>(), (uint32_t)M,
                                                         o->cnt_sorted.as<uint32_t>());
     NPS_CHECK_LAUNCH();
     uint32_t* total = o->total.as<uint32_t>();
@@ -2592,10 +2649,9 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
     }
     if (K > 0 || capture) {
       { StageTimer t(o, ST_EMIT);
-      gs::k_emit<<<div_up(M, 256), 256, 0, s>>>(dv, o->ecounts.as<uint32_t>(), o->offsets.as<uint32_t>(),
-                                                 o->rects.as<uint2>(), o->tmasks.as<uint32_t>(), (uint32_t)M, n,
-                                                 tiles_x, num_tiles, o->pair_cap,
-                                                 o->keys.as<uint32_t>(), o->vals.as<uint32_t>());
+      gs::k_emit<<<div_up(M, 256), 256, 0, s>>>(dv, o->bins.as<uint4>(), o->offsets.as<uint32_t>(), (uint32_t)M, n,
+                                                 tiles_x, num_tiles, o->pair_cap, o->keys.as<uint32_t>(),
+                                                 o->vals.as<uint32_t>());
       NPS_CHECK_LAUNCH(); }
       int bits = 1;
       while ((1ull << bits) < (uint64_t)num_tiles * nv) ++bits;

@@ -83,6 +83,31 @@ def test_forward_loss_backward_match_oracle(trainer_cls, n, w, h, deg, eyes, lsm
     assert t.stats()["pairs"] > 0
 
 
+@pytest.mark.parametrize("n,nv,deg", [(1, 1, 3), (31, 1, 0), (65, 2, 1), (33, 3, 2), (32, 4, 3), (63, 5, 0), (95, 8, 3),
+                                      (129, 9, 1), (64, 17, 2)])
+def test_counts_and_views_at_block_edges(trainer_cls, n, nv, deg):
+    """Projection, binning and projection backward at the edges of their blocks: Gaussian counts around the 32 and 64
+    of a block, view counts around the 1, 2, 4 and 8 lanes per Gaussian, every SH degree.  Tolerances as above; the
+    gradient as relative L2."""
+    w, h = 40, 36
+    p = gs_scene(n, 70 + n, deg=deg, log_scale_mean=-2.5)
+    ang = np.linspace(0.0, 2 * np.pi, nv, endpoint=False)
+    vp, vpi, views = gs_views(w, h, [(4 * np.sin(a), 0.7, 4 * np.cos(a)) for a in ang])
+    tg = gs_targets(nv, w, h, 6)
+    tids = np.arange(nv, dtype=np.uint32)
+    t, img, l3, st = run_gpu(trainer_cls, p, deg, vp, vpi, tg, tids)
+    rimg, rnc = orc.gs_forward(p, deg, views, w, h)
+    np.testing.assert_allclose(img, rimg, atol=1e-5, rtol=0)
+    _, rdimg = orc.gs_loss(rimg, tg, tids)
+    rg, radc = orc.gs_backward(p, deg, views, w, h, rimg, rnc, rdimg, with_adc=True)
+    np.testing.assert_array_equal(st["adc_denom"], radc[:, 1])
+    used = np.r_[0:11, 12:12 + 3 * (deg + 1) ** 2]
+    a, b = st["grads"][:, used].astype(np.float64), rg[:, used].astype(np.float64)
+    assert np.linalg.norm(a - b) < 1e-4 * np.linalg.norm(b)
+    rest = np.setdiff1d(np.arange(64), used)
+    assert (st["grads"][:, rest] == 0.0).all()
+
+
 def test_per_view_accumulation_matches_batched(trainer_cls):
     """The plain per-view trainer's accumulated gradient (one launch per view)
     equals the batched multi-view gradient; so do the loss and ADC statistic."""
