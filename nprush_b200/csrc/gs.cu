@@ -26,7 +26,7 @@
 //                  CTA in shared memory, then one global atomic per (tile,
 //                  Gaussian, value); k_bwd<true> + k_det_segsum: the
 //                  deterministic two-pass variant
-//   k_project_bwd  eight lanes per Gaussian over the views: screen-space
+//   k_project_bwd  up to eight lanes per Gaussian over the views: screen-space
 //                  gradients -> parameter gradients, ADC statistics
 //   k_adam         fused Adam over the 59 parameters of every Gaussian
 #include <cuda_runtime.h>
@@ -1409,17 +1409,20 @@ __global__ void k_det_segsum(const uint32_t* __restrict__ keys, const uint32_t* 
 }
 
 // ------------------------------------------------------------ projection backward
-// Eight lanes per Gaussian, each taking the views v = lane, lane + 8, ...: a
-// lane accumulates its views' parameter gradients in record layout (64
-// registers), then the eight partial records are summed by a reduce-scatter
-// over the group (xor 4, 2, 1: 56 shuffles) and lane s writes floats
-// 8s .. 8s + 7 of the Gaussian's gradient record.  The ADC statistic rides in
-// the padding floats 60 and 61 through the reduction.
-// ONE: at most eight views, so each lane has at most one view.  Its SH
+// LANES lanes per Gaussian, each taking the views v = lane, lane + LANES, ...:
+// a lane accumulates its views' parameter gradients in record layout (64
+// registers), then the partial records are summed by a reduce-scatter over the
+// group (56 shuffles for eight lanes) and lane s writes the s-th part of the
+// Gaussian's gradient record.  The ADC statistic rides in the padding floats 60
+// and 61 through the reduction.  As many lanes as views, in powers of two up to
+// eight: with fewer views the rest of eight would only carry zeros through the
+// reduction (one view: 16k Gaussians, SH1, 14.8 -> 10.8 us; three views: 57k, SH2,
+// 38 -> 27 us).
+// ONE: at most LANES views, so each lane has at most one view.  Its SH
 // gradient is then basis[k] * dc[c] exactly (a sum of one term), which is
 // formed just before the reduction instead of being accumulated through the
 // view's projection arithmetic: 48 fewer live registers there.
-template <int DEG, bool ONE>
+template <int DEG, int LANES, bool ONE>
 __global__ void __launch_bounds__(128, ONE ? 4 : 1) k_project_bwd(const float* __restrict__ params, uint32_t n,
                                                      const float* __restrict__ views, uint32_t nv, uint32_t W,
                                                      uint32_t H, const uint32_t* __restrict__ counts,
@@ -1428,8 +1431,8 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 1) k_project_bwd(const float* _
                                                      int accumulate, float adc_scale) {
   constexpr int nb = (DEG + 1) * (DEG + 1);
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t i = t >> 3, sub = t & 7;
-  const bool live = i < n;  // whole groups are live or not (n * 8 threads, groups aligned)
+  const uint32_t i = t / LANES, sub = t % LANES;
+  const bool live = i < n;  // whole groups are live or not (n * LANES threads, groups aligned)
   if (__all_sync(0xffffffffu, !live)) return;
   const float4* p4 = reinterpret_cast<const float4*>(params + (size_t)(live ? i : 0) * kP);
   const float4 q0 = p4[0], q1 = p4[1], q2 = p4[2];
@@ -1448,7 +1451,7 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 1) k_project_bwd(const float* _
   for (int k = 0; k < kP; ++k) g[k] = 0.0f;
   float one_basis[ONE ? nb : 1], one_dc[3] = {0.0f, 0.0f, 0.0f};
   bool one_has = false;
-  for (uint32_t v = sub; live && v < nv; v += 8) {
+  for (uint32_t v = sub; live && v < nv; v += LANES) {
     const size_t gi = (size_t)v * n + i;
     // the gradient record (48 B, 16-byte aligned) is fetched with the count, not after it
     const float4* gr = reinterpret_cast<const float4*>(g2 + gi * kG2);
@@ -1583,44 +1586,41 @@ __global__ void __launch_bounds__(128, ONE ? 4 : 1) k_project_bwd(const float* _
         for (int c = 0; c < 3; ++c) g[kSH + 3 * k + c] = one_basis[k] * one_dc[c];
     }
   }
-  // reduce-scatter over the group's eight lanes
-  const bool b2 = sub & 4, b1 = sub & 2, b0 = sub & 1;
+  // reduce-scatter over the group's lanes: kPart floats of the record stay in each
+  constexpr int kPart = kP / LANES;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
-    const float send = b2 ? g[j] : g[j + 32], keep = b2 ? g[j + 32] : g[j];
-    g[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
+  for (int half = LANES / 2, cnt = kP / 2; half > 0; half /= 2, cnt /= 2) {
+    const bool up = (sub & half) != 0;
 #pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    const float send = b1 ? g[j] : g[j + 16], keep = b1 ? g[j + 16] : g[j];
-    g[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float send = b0 ? g[j] : g[j + 8], keep = b0 ? g[j + 8] : g[j];
-    g[j] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+    for (int j = 0; j < kP / 2; ++j) {
+      if (j >= cnt) break;
+      const float send = up ? g[j] : g[j + cnt], keep = up ? g[j + cnt] : g[j];
+      g[j] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+    }
   }
   if (!live) return;
-  // this lane holds record floats 8 * sub .. 8 * sub + 7 in g[0..7]
-  if (sub == 1) {
+  // this lane holds record floats kPart * sub .. kPart * sub + kPart - 1 in g[0 ..]
+  constexpr int kOpPart = kOpacity / kPart, kOpAt = kOpacity % kPart;
+  if (sub == kOpPart) {
     const float op = sigmoidf(op_logit);
-    g[kOpacity - 8] *= op * (1.0f - op);
-    g[11 - 8] = 0.0f;
+    g[kOpAt] *= op * (1.0f - op);
+    g[kOpAt + 1] = 0.0f;
   }
-  if (sub == 7) {
-    adc_grad[i] += g[60 - 56];
-    adc_denom[i] += g[61 - 56];
-    g[4] = g[5] = g[6] = g[7] = 0.0f;
+  if (sub == LANES - 1) {
+    adc_grad[i] += g[kPart - 4];
+    adc_denom[i] += g[kPart - 3];
+    g[kPart - 4] = g[kPart - 3] = g[kPart - 2] = g[kPart - 1] = 0.0f;
   }
-  float4* out4 = reinterpret_cast<float4*>(grads + (size_t)i * kP + 8 * sub);
-  float4 w0 = make_float4(g[0], g[1], g[2], g[3]), w1 = make_float4(g[4], g[5], g[6], g[7]);
-  if (accumulate) {
-    const float4 a0 = out4[0], a1 = out4[1];
-    w0.x += a0.x; w0.y += a0.y; w0.z += a0.z; w0.w += a0.w;
-    w1.x += a1.x; w1.y += a1.y; w1.z += a1.z; w1.w += a1.w;
+  float4* out4 = reinterpret_cast<float4*>(grads + (size_t)i * kP + kPart * sub);
+#pragma unroll
+  for (int q = 0; q < kPart / 4; ++q) {
+    float4 w = make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
+    if (accumulate) {
+      const float4 old = out4[q];
+      w.x += old.x; w.y += old.y; w.z += old.z; w.w += old.w;
+    }
+    out4[q] = w;
   }
-  out4[0] = w0;
-  out4[1] = w1;
 }
 
 // ------------------------------------------------------------ Adam
@@ -1657,14 +1657,17 @@ __device__ __forceinline__ float lr_of(const AdamArgs& a, int k) {
   return k < 3 ? a.lr[0] : k < 6 ? a.lr[1] : k < 10 ? a.lr[2] : k < 12 ? a.lr[3] : k < 15 ? a.lr[4] : a.lr[5];
 }
 
-// one thread per float4 of the parameter record (16 per Gaussian)
+// one thread per float4 of the parameter record (16 per Gaussian).  Was bound by
+// its four full divisions per value as much as by memory; the two bias corrections
+// are now products with their reciprocals: 1M Gaussians 420 -> 289 us, 200k 91 ->
+// 66 us (floors at the copy rate: 250 and 50).
 __global__ void __launch_bounds__(256) k_adam(float4* __restrict__ p, const float4* __restrict__ g,
                                               float4* __restrict__ m, float4* __restrict__ v, uint32_t n4,
                                               AdamArgs a, const uint32_t* __restrict__ st) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n4 || st[1] != 0u) return;
   if ((t & 15u) * 4u >= (uint32_t)kUsed) return;  // floats 60-63: nothing to update, nothing to move
-  const float bc1 = __uint_as_float(st[2]), bc2 = __uint_as_float(st[3]);
+  const float ibc1 = 1.0f / __uint_as_float(st[2]), ibc2 = 1.0f / __uint_as_float(st[3]);
   const int k0 = (int)(t & 15u) * 4;
   float4 pp = p[t], gg = g[t], mm = m[t], vv = v[t];
   float* pf = &pp.x;
@@ -1678,7 +1681,7 @@ __global__ void __launch_bounds__(256) k_adam(float4* __restrict__ p, const floa
     const float gr = gf[c];
     mf[c] = a.b1 * mf[c] + (1.0f - a.b1) * gr;
     vf[c] = a.b2 * vf[c] + (1.0f - a.b2) * gr * gr;
-    const float mh = mf[c] / bc1, vh = vf[c] / bc2;
+    const float mh = mf[c] * ibc1, vh = vf[c] * ibc2;
     pf[c] -= lr_of(a, k) * mh / (sqrtf(vh) + a.eps);
   }
   p[t] = pp;
@@ -2788,18 +2791,22 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
   }
   if (n > 0) {
     StageTimer t(o, ST_PBWD);
-    const uint32_t blocks = div_up((size_t)n * 8, 128);
     const float adc_scale = (float)(o->loss_views ? o->loss_views : nv);
-#define NPS_PBWD1(D, ONE)                                                                                        \
-  gs::k_project_bwd<D, ONE><<<blocks, 128, 0, s>>>(o->params.as<float>(), n, o->views.as<float>(), nv, W, H,     \
-                                                    o->counts.as<uint32_t>(), o->g2.as<float>(),                  \
-                                                    o->grads.as<float>(), o->adc_grad.as<float>(),                \
-                                                    o->adc_denom.as<float>(), o->accumulate ? 1 : 0, adc_scale)
+#define NPS_PBWD1(D, L, ONE)                                                                                     \
+  gs::k_project_bwd<D, L, ONE><<<div_up((size_t)n * L, 128), 128, 0, s>>>(                                       \
+      o->params.as<float>(), n, o->views.as<float>(), nv, W, H, o->counts.as<uint32_t>(), o->g2.as<float>(),     \
+      o->grads.as<float>(), o->adc_grad.as<float>(), o->adc_denom.as<float>(), o->accumulate ? 1 : 0, adc_scale)
 #define NPS_PBWD(D)            \
-  if (nv <= 8) {               \
-    NPS_PBWD1(D, true);        \
+  if (nv == 1) {               \
+    NPS_PBWD1(D, 1, true);     \
+  } else if (nv == 2) {        \
+    NPS_PBWD1(D, 2, true);     \
+  } else if (nv <= 4) {        \
+    NPS_PBWD1(D, 4, true);     \
+  } else if (nv <= 8) {        \
+    NPS_PBWD1(D, 8, true);     \
   } else {                     \
-    NPS_PBWD1(D, false);       \
+    NPS_PBWD1(D, 8, false);    \
   }
     switch (o->sh_deg) {
       case 0: NPS_PBWD(0); break;
