@@ -64,9 +64,8 @@ inline unsigned div_up(size_t a, size_t b) { return (unsigned)((a + b - 1) / b);
 // Work buffers for the device-wide scan and the radix sort.  Sizes depend only
 // on the grid, never on the number of keys, so no host sync is needed.
 struct SortWork {
-  DevBuf hist;      // per-pass digit histograms, tile counters, own timeout counter
   DevBuf partial;   // scan partial sums
-  DevBuf lookback;  // per pass and tile: the published per-digit counts
+  DevBuf lookback;  // digit histograms, tile counters, own timeout counter, published per-digit counts
   DevBuf keys_alt, vals_alt;
   // bounded look-back: polls of an unpublished tile status before giving up
   // (counted in *err, or in the work's own counter when err is null); tests
@@ -83,9 +82,10 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
 // key bits (at most 32, at most 2^30 - 1 pairs).
 // The number of pairs is read from device memory (*count_dev, clamped to cap).
 // keys/vals hold the input; on return *keys_out / *vals_out point at the sorted
-// arrays (either the inputs or the work buffers).
+// arrays (either the inputs or the work buffers).  iota: the values are 0, 1,
+// 2, ... and vals is only room for cap of them.
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out);
+                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota = false);
 
 
 }  // namespace nps

@@ -1177,8 +1177,7 @@ struct RenderWork {
   SortWork sw;
   uint32_t pair_cap = 0;
   void release() {
-    for (DevBuf* b : {&rec, &counts, &offsets, &rects, &total, &cam, &keys, &vals, &ranges, &tabs, &sw.hist,
-                      &sw.partial, &sw.lookback, &sw.keys_alt, &sw.vals_alt})
+    for (DevBuf* b : {&rec, &counts, &offsets, &rects, &total, &cam, &keys, &vals, &ranges, &tabs, &sw.partial, &sw.lookback, &sw.keys_alt, &sw.vals_alt})
       b->release();
   }
 };
@@ -1279,8 +1278,7 @@ int nps_splat_opt_destroy(nps_splat_opt* o) {
   for (DevBuf* b : {&o->params, &o->grads, &o->am, &o->av, &o->gacc, &o->views, &o->tgt_rgba_own,
                     &o->tgt_depth_own, &o->fwd, &o->bwd, &o->counts, &o->kept, &o->offsets, &o->rects, &o->total,
                     &o->grid, &o->cutoff, &o->tile_len, &o->ckbuf,
-                    &o->keys, &o->vals, &o->ranges, &o->tabs, &o->dead, &o->stat, &o->tstat, &o->sw.hist,
-                    &o->sw.partial, &o->sw.lookback, &o->sw.keys_alt, &o->sw.vals_alt})
+                    &o->keys, &o->vals, &o->ranges, &o->tabs, &o->dead, &o->stat, &o->tstat, &o->sw.partial, &o->sw.lookback, &o->sw.keys_alt, &o->sw.vals_alt})
     b->release();
   if (o->rw) {
     o->rw->release();

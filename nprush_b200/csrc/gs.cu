@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
                                                     uint32_t H, uint32_t tiles_x, uint32_t tiles_y, float inv_tile,
                                                     uint32_t group, Rec* __restrict__ recs,
                                                     uint32_t* __restrict__ counts, uint4* __restrict__ bins,
-                                                    uint32_t* __restrict__ dkeys, uint32_t* __restrict__ dvals) {
+                                                    uint32_t* __restrict__ dkeys) {
   extern __shared__ float4 sm_pre[];
   const uint32_t tv = threadIdx.x / group, gi = threadIdx.x - tv * group, lane = threadIdx.x & 31u;
   const uint32_t i0 = blockIdx.x * group, i = i0 + gi, v = blockIdx.y * (blockDim.x / group) + tv;
@@ -264,7 +264,9 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
   project<float>(view, mean, ls, q, (float)W, (float)H, kLowpass, P);
   uint32_t cnt = 0, ecnt = 0, tmask = 0;
   uint2 rect = make_uint2(0, 0);
-  uint32_t key = 0xffffffffu;
+  // a record without pairs may stand anywhere in the depth order; at 2.0 it shares
+  // the top byte of every depth in [2, 8), and that digit's sort pass is free
+  uint32_t key = __float_as_uint(2.0f);
   Rec r;
   r.a = make_float4(0, 0, 0, 0);
   r.b = make_float4(0, 0, 0, 0);
@@ -357,7 +359,6 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
   counts[g] = cnt;
   bins[g] = make_uint4(rect.x, rect.y, tmask, ecnt);
   dkeys[g] = key;
-  dvals[g] = g;
 }
 
 __global__ void k_gather_counts(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins, uint32_t m,
@@ -2119,7 +2120,7 @@ int nps_gs_destroy(nps_gs* o) {
   for (cudaEvent_t e : o->ev_pool) cudaEventDestroy(e);
   for (DevBuf* b : {&o->p_alt, &o->m_alt, &o->v_alt, &o->aflags, &o->akeep, &o->acand, &o->akeep_off, &o->acand_off,
                     &o->acnt, &o->aoff, &o->atot, &o->psnr_acc, &o->stepst, &o->afeat, &o->alogits,
-                    &o->det_part, &o->det_keys, &o->det_pos, &o->sw_det.hist, &o->sw_det.partial,
+                    &o->det_part, &o->det_keys, &o->det_pos, &o->sw_det.partial,
                     &o->sw_det.lookback, &o->sw_det.keys_alt, &o->sw_det.vals_alt})
     b->release();
   for (DevBuf* b : {&o->tile_last, &o->ws_order_f, &o->ws_order_b, &o->ws_q}) b->release();
@@ -2127,9 +2128,8 @@ int nps_gs_destroy(nps_gs* o) {
                     &o->tids, &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals,
                     &o->cnt_sorted, &o->offsets, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->img,
                     &o->ncontrib, &o->maps,
-                    &o->partial, &o->loss, &o->dimg, &o->g2, &o->sw_depth.hist, &o->sw_depth.partial,
-                    &o->sw_depth.lookback, &o->sw_depth.keys_alt, &o->sw_depth.vals_alt, &o->sw_tile.hist,
-                    &o->sw_tile.partial, &o->sw_tile.lookback, &o->sw_tile.keys_alt, &o->sw_tile.vals_alt})
+                    &o->partial, &o->loss, &o->dimg, &o->g2, &o->sw_depth.partial,
+                    &o->sw_depth.lookback, &o->sw_depth.keys_alt, &o->sw_depth.vals_alt, &o->sw_tile.partial, &o->sw_tile.lookback, &o->sw_tile.keys_alt, &o->sw_tile.vals_alt})
     b->release();
   delete o;
   return NPS_OK;
@@ -2608,8 +2608,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
 #define NPS_PRE(D)                                                                                              \
   gs::k_preprocess<D><<<pgrid, group * vb, gs::pre_smem(group, group * vb), s>>>(                               \
       o->params.as<float>(), n, o->views.as<float>(), nv, W, H, tiles_x, tiles_y, 1.0f / (float)o->tile, group, \
-      o->recs.as<gs::Rec>(), o->counts.as<uint32_t>(), o->bins.as<uint4>(), o->dkeys.as<uint32_t>(),            \
-      o->dvals.as<uint32_t>())
+      o->recs.as<gs::Rec>(), o->counts.as<uint32_t>(), o->bins.as<uint4>(), o->dkeys.as<uint32_t>())
     switch (o->sh_deg) {
       case 0: NPS_PRE(0); break;
       case 1: NPS_PRE(1); break;
@@ -2622,7 +2621,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
     uint32_t *dk = nullptr, *dv = nullptr;
     { StageTimer t(o, ST_DSORT);
     NPS_TRY(radix_sort_u32(o->dkeys.as<uint32_t>(), o->dvals.as<uint32_t>(), o->mcount.as<uint32_t>(), (uint32_t)M, 32,
-                           o->sw_depth, s, &dk, &dv)); }
+                           o->sw_depth, s, &dk, &dv, true)); }
     o->sorted_vals = dv;
     gs::k_gather_counts<<<div_up(M, 256), 256, 0, s>>>(dv, o->bins.as<uint4>(), (uint32_t)M,
                                                         o->cnt_sorted.as<uint32_t>());

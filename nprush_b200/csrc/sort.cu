@@ -1,13 +1,17 @@
 // sort.cu — device-wide exclusive scan and stable LSD radix sort.
 //
-// Used for the (view, tile[, depth]) keys of the binning stage.  The sort is
-// a onesweep radix sort: one histogram kernel for all 8-bit digits, then one
+// Used for the (view, tile[, depth]) keys of the binning stage.  Up to 8192
+// pairs are sorted by one block in shared memory; beyond, the sort is a
+// onesweep radix sort: one histogram kernel for all 8-bit digits, then one
 // kernel per digit that ranks each tile of keys stably (warp-level ranking in
 // original order from per-bit ballots), finds the tile's global offsets by a
 // bounded decoupled look-back over the earlier tiles, and scatters.  The grid
 // never depends on the key count (read from device memory), so the whole sort
 // can be captured in a CUDA graph.  The exclusive scan is reduce-then-scan.
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <utility>
 
 #include "common.cuh"
 #include "context.h"
@@ -20,8 +24,12 @@ namespace {
 #endif
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kItems = 12;
-constexpr int kTile = kSortThreads * kItems;  // 3072 keys
+// keys per thread of a onesweep tile: 12 (3072 keys a tile), or 4 where even
+// those tiles leave most SMs without one and a tile's own latency is the pass's
+// (four-pass sort of 16384 keys 56 -> 38 us, of 171k keys 62 -> 52 us; at 500k keys
+// the shorter look-back wins, two passes 49 against 54 us)
+constexpr int kItemsLong = 12, kItemsShort = 4;
+constexpr uint32_t kShortMax = 1u << 18;
 constexpr int kSortGrid = 4 * kNumSMs;  // four resident blocks per SM (64 registers)
 
 constexpr int kScanThreads = 1024;
@@ -124,19 +132,9 @@ __global__ void k_scan_down(const uint32_t* __restrict__ in, uint32_t n, const u
   }
 }
 
-__device__ __forceinline__ void block_range(const uint32_t* count_dev, uint32_t cap, uint32_t* n, uint32_t* t0,
-                                            uint32_t* t1) {
-  uint32_t nn = min(*count_dev, cap);
-  uint32_t tiles = (nn + kTile - 1) / kTile;
-  uint32_t per = (tiles + gridDim.x - 1) / gridDim.x;
-  *n = nn;
-  *t0 = min(blockIdx.x * per, tiles);
-  *t1 = min(*t0 + per, tiles);
-}
-
 // ---------------------------------------------------------------- onesweep
 // One launch per 8-bit digit (Adinets and Merrill's onesweep): a CTA claims
-// the next tile of kTile keys from a counter (tiles are claimed in order, so
+// the next tile of keys from a counter (tiles are claimed in order, so
 // every tile a CTA waits for belongs to a CTA that is already running), ranks
 // its keys locally and stably, publishes its per-digit counts, and finds the
 // number of keys of each digit in all earlier tiles by looking back through
@@ -164,26 +162,51 @@ __device__ __forceinline__ void st_status(uint32_t* p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// Digit histograms of every pass in one read: ghist[pass * 256 + digit].
-template <class K>
+// Digit histograms of every pass in one read: ghist[pass * 256 + digit].  Keys
+// in 16-byte loads, two at a time per thread (one 4-byte load in flight left
+// the kernel waiting on memory: 11.5 M pairs' tile sort 250 -> 242 us, 38 M 886 ->
+// 838 us), from the first aligned one on; block 0 adds what lies before and
+// after.
+template <class K, int PASSES>
 __global__ void __launch_bounds__(kSortThreads) k_hist_all(const K* __restrict__ keys, const uint32_t* count_dev,
-                                                            uint32_t cap, int passes, uint32_t* __restrict__ ghist) {
-  __shared__ uint32_t h[4][256];
-  for (int i = threadIdx.x; i < 4 * 256; i += kSortThreads) (&h[0][0])[i] = 0;
+                                                            uint32_t cap, uint32_t* __restrict__ ghist) {
+  static_assert(sizeof(K) == 4, "four keys per 16-byte load");
+  __shared__ uint32_t h[PASSES][256];
+  for (int i = threadIdx.x; i < PASSES * 256; i += kSortThreads) (&h[0][0])[i] = 0;
   __syncthreads();
   const uint32_t n = min(*count_dev, cap);
-  for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += gridDim.x * kSortThreads) {
-    const K k = keys[i];
-    for (int p = 0; p < passes; ++p) atomicAdd(&h[p][(uint32_t)(k >> (8 * p)) & 255u], 1u);
+  auto add = [&](K k) {
+#pragma unroll
+    for (int p = 0; p < PASSES; ++p) atomicAdd(&h[p][(uint32_t)(k >> (8 * p)) & 255u], 1u);
+  };
+  const uint32_t head = min(n, (uint32_t)((16u - ((uintptr_t)keys & 15u)) & 15u) / 4u);
+  const uint32_t n4 = (n - head) / 4;
+  const uint4* k4 = reinterpret_cast<const uint4*>(keys + head);
+  const uint32_t stride = gridDim.x * kSortThreads;
+  uint32_t i = blockIdx.x * kSortThreads + threadIdx.x;
+  for (; i + stride < n4; i += 2 * stride) {
+    const uint4 a = __ldg(k4 + i), b = __ldg(k4 + i + stride);
+    add(a.x); add(a.y); add(a.z); add(a.w);
+    add(b.x); add(b.y); add(b.z); add(b.w);
+  }
+  if (i < n4) {
+    const uint4 a = __ldg(k4 + i);
+    add(a.x); add(a.y); add(a.z); add(a.w);
+  }
+  if (blockIdx.x == 0) {
+    if (threadIdx.x < head) add(keys[threadIdx.x]);
+    const uint32_t tail = head + 4 * n4 + threadIdx.x;
+    if (tail < n) add(keys[tail]);
   }
   __syncthreads();
-  for (int p = 0; p < passes; ++p) {
+#pragma unroll
+  for (int p = 0; p < PASSES; ++p) {
     const uint32_t c = h[p][threadIdx.x];
     if (c) atomicAdd(ghist + p * 256 + threadIdx.x, c);
   }
 }
 
-template <class K>
+template <class K, int kItems>
 __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const K* __restrict__ kin,
                                                                const uint32_t* __restrict__ vin, K* __restrict__ kout,
                                                                uint32_t* __restrict__ vout, const uint32_t* count_dev,
@@ -193,6 +216,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const K* __restric
                                                                uint32_t* __restrict__ tile_counter,
                                                                uint32_t* __restrict__ err, uint32_t spin_limit,
                                                                uint32_t stall_tile) {
+  constexpr int kTile = kSortThreads * kItems;
   __shared__ uint32_t pass_off[256];
   __shared__ uint32_t run[256];
   __shared__ uint32_t toff[256];
@@ -204,6 +228,15 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const K* __restric
   const uint32_t d_own = threadIdx.x;  // the digit this thread publishes and looks back for
   const uint32_t n = min(*count_dev, cap);
   const uint32_t tiles = (n + kTile - 1) / kTile;
+  // all keys have this digit in common (the top byte of depths within a factor
+  // of four, say): the pass moves nothing
+  if (__syncthreads_or(ghist[d_own] == n)) {
+    for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += gridDim.x * kSortThreads) {
+      kout[i] = kin[i];
+      vout[i] = vin ? vin[i] : i;
+    }
+    return;
+  }
   // this pass's digit offsets: exclusive scan of its histogram
   pass_off[d_own] = block_exclusive_scan<kSortThreads>(ghist[d_own], &scan_total);
   const uint32_t lt = lanemask_lt();
@@ -221,7 +254,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const K* __restric
       const uint32_t idx = base + j * 32 + lane;
       const bool ok = idx < n;
       k[j] = ok ? kin[idx] : (K)0;
-      v[j] = ok ? vin[idx] : 0u;
+      v[j] = !ok ? 0u : vin ? vin[idx] : idx;
       dg[j] = ok ? ((uint32_t)(k[j] >> shift) & 255u) : 256u;
     }
     // stable local rank: per warp in (item, lane) order, warps in order
@@ -311,39 +344,188 @@ __global__ void __launch_bounds__(kSortThreads, 4) k_onesweep(const K* __restric
   }
 }
 
+// ------------------------------------------------------------- one block
+// Up to 1024 * ITEMS pairs in one block: keys and values in registers, each
+// pass ranked as the onesweep ranks a tile, scattered into shared memory and
+// read back.  A onesweep of so few keys is five or more launches of a few
+// blocks each (1024 pairs: 45 us with their gaps, here 18).  Sixteen items per
+// thread would take 68 us at 16384 pairs against the onesweep's 38, so it ends at
+// eight.  In place; a digit common to all keys costs no pass.
+constexpr uint32_t kSmallThreads = 1024, kSmallMax = 8 * kSmallThreads;
+constexpr size_t small_smem(int items) {
+  return sizeof(uint32_t) * (2 * kSmallThreads * (size_t)items + 32 * 256 + 4 * 256 + 256);
+}
+template <int ITEMS>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
+                                                              const uint32_t* count_dev, uint32_t cap, int passes,
+                                                              int iota) {
+  extern __shared__ uint32_t sm_small[];
+  uint32_t* sk = sm_small;
+  uint32_t* sv = sk + kSmallThreads * ITEMS;
+  uint32_t* wh = sv + kSmallThreads * ITEMS;  // [32][256]: per warp, counts then offsets within the digit
+  uint32_t* part = wh + 32 * 256;             // [4][256]: the same for eight warps together
+  uint32_t* doff = part + 4 * 256;            // [256]: first position of each digit
+  __shared__ uint32_t scan_total;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, lt = lanemask_lt();
+  const uint32_t n = min(*count_dev, cap), base = wid * (32 * ITEMS) + lane;
+  uint32_t k[ITEMS], v[ITEMS], rk[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t idx = base + j * 32;
+    k[j] = idx < n ? keys[idx] : 0u;
+    v[j] = idx >= n ? 0u : iota ? idx : vals[idx];
+  }
+  for (int p = 0; p < passes; ++p) {
+    const int shift = 8 * p;
+    for (uint32_t i = tid; i < 32 * 256; i += kSmallThreads) wh[i] = 0;
+    __syncthreads();
+    uint32_t* mine = wh + wid * 256;
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t d = base + j * 32 < n ? (k[j] >> shift) & 255u : 256u;
+      uint32_t peers = 0xffffffffu;
+#pragma unroll
+      for (int b = 0; b < 9; ++b) {
+        const bool bit = (d >> b) & 1u;
+        const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? bal : ~bal;
+      }
+      const int leader = __ffs((int)peers) - 1;
+      uint32_t old = 0;
+      if ((int)lane == leader && d < 256u) {
+        old = mine[d];
+        mine[d] = old + __popc(peers);
+      }
+      rk[j] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lt);
+      __syncwarp();
+    }
+    __syncthreads();
+    {  // thread (q, d): the counts of digit d in warps 8 q .. 8 q + 7 become offsets
+      const uint32_t d = tid & 255u, q = tid >> 8;
+      uint32_t acc = 0;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        uint32_t* c = wh + (q * 8 + w) * 256 + d;
+        const uint32_t x = *c;
+        *c = acc;
+        acc += x;
+      }
+      part[q * 256 + d] = acc;
+    }
+    __syncthreads();
+    uint32_t tot = 0;
+    if (tid < 256) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t x = part[q * 256 + tid];
+        part[q * 256 + tid] = tot;
+        tot += x;
+      }
+    }
+    const bool common = __syncthreads_or(tid < 256 && tot == n);
+    if (common) continue;  // every key has this digit
+    const uint32_t off = block_exclusive_scan<(int)kSmallThreads>(tot, &scan_total);
+    if (tid < 256) doff[tid] = off;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (base + j * 32 < n) {
+        const uint32_t d = (k[j] >> shift) & 255u;
+        const uint32_t pos = doff[d] + part[(wid >> 3) * 256 + d] + mine[d] + rk[j];
+        sk[pos] = k[j];
+        sv[pos] = v[j];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const uint32_t idx = base + j * 32;
+      if (idx < n) {
+        k[j] = sk[idx];
+        v[j] = sv[idx];
+      }
+    }
+    // the next pass's first barrier stands before anything here is overwritten
+  }
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const uint32_t idx = base + j * 32;
+    if (idx < n) {
+      keys[idx] = k[j];
+      vals[idx] = v[j];
+    }
+  }
+}
+
+template <int ITEMS>
+int launch_small(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int passes, bool iota,
+                 cudaStream_t s) {
+  static bool set[64] = {};  // per device; a second thread setting it again does no harm
+  int dev = 0;
+  NPS_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64 || !set[dev]) {
+    NPS_CUDA(cudaFuncSetAttribute(k_sort_small<ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)small_smem(ITEMS)));
+    if (dev >= 0 && dev < 64) set[dev] = true;
+  }
+  k_sort_small<ITEMS><<<1, kSmallThreads, small_smem(ITEMS), s>>>(keys, vals, count_dev, cap, passes, iota ? 1 : 0);
+  NPS_CHECK_LAUNCH();
+  return NPS_OK;
+}
+
 template <class K>
 int radix_sort_impl(K* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                    cudaStream_t s, K** keys_out, uint32_t** vals_out) {
+                    cudaStream_t s, K** keys_out, uint32_t** vals_out, bool iota) {
   if (cap >= (1u << 30)) {
     set_error("radix sort: capacity %u beyond the look-back's 30-bit counts", cap);
     return NPS_ERR_INVALID;
   }
   const int passes = (bits + 7) / 8;
-  const uint32_t max_tiles = (cap + kTile - 1) / kTile;
-  // hist: the per-pass histograms, the per-pass tile counters and the
-  // timeout counter of callers without their own; lookback: per pass and tile
-  NPS_TRY(w.hist.ensure(sizeof(uint32_t) * (4 * 256 + 4 + 1)));
-  NPS_TRY(w.lookback.ensure(sizeof(uint32_t) * 256 * (size_t)max_tiles * 4 + 256));
+  // one block's worth (a stalled tile, for tests, stalls the onesweep's look-back)
+  if (cap <= kSmallMax && w.stall_tile == 0xffffffffu) {
+    *keys_out = keys;
+    *vals_out = vals;
+    return cap <= 4 * kSmallThreads ? launch_small<4>(keys, vals, count_dev, cap, passes, iota, s)
+                                    : launch_small<8>(keys, vals, count_dev, cap, passes, iota, s);
+  }
+  const bool is_short = cap <= kShortMax;
+  const uint32_t tile = kSortThreads * (is_short ? kItemsShort : kItemsLong);
+  const uint32_t max_tiles = (cap + tile - 1) / tile;
+  // one buffer, cleared at once: the per-pass histograms, the per-pass tile
+  // counters, the timeout counter of callers without their own, then the
+  // published counts per pass and tile
+  constexpr size_t kHead = 4 * 256 + 64;
+  NPS_TRY(w.lookback.ensure(sizeof(uint32_t) * (kHead + 256 * (size_t)max_tiles * 4)));
   NPS_TRY(w.keys_alt.ensure(sizeof(K) * (size_t)cap));
   NPS_TRY(w.vals_alt.ensure(sizeof(uint32_t) * (size_t)cap));
-  uint32_t* ghist = w.hist.as<uint32_t>();
+  uint32_t* ghist = w.lookback.as<uint32_t>();
   uint32_t* counters = ghist + 4 * 256;
   uint32_t* err = w.err ? w.err : counters + 4;
-  NPS_CUDA(cudaMemsetAsync(ghist, 0, sizeof(uint32_t) * (4 * 256 + 4), s));
-  NPS_CUDA(cudaMemsetAsync(w.lookback.p, 0, sizeof(uint32_t) * 256 * (size_t)max_tiles * passes, s));
-  k_hist_all<K><<<kSortGrid, kSortThreads, 0, s>>>(keys, count_dev, cap, passes, ghist);
+  uint32_t* status = ghist + kHead;
+  NPS_CUDA(cudaMemsetAsync(ghist, 0, sizeof(uint32_t) * (kHead + 256 * (size_t)max_tiles * passes), s));
+  const uint32_t grid = std::min<uint32_t>(kSortGrid, max_tiles);
+  switch (passes) {
+    case 1: k_hist_all<K, 1><<<grid, kSortThreads, 0, s>>>(keys, count_dev, cap, ghist); break;
+    case 2: k_hist_all<K, 2><<<grid, kSortThreads, 0, s>>>(keys, count_dev, cap, ghist); break;
+    case 3: k_hist_all<K, 3><<<grid, kSortThreads, 0, s>>>(keys, count_dev, cap, ghist); break;
+    default: k_hist_all<K, 4><<<grid, kSortThreads, 0, s>>>(keys, count_dev, cap, ghist); break;
+  }
   NPS_CHECK_LAUNCH();
   K* ka = keys;
   uint32_t* va = vals;
   K* kb = w.keys_alt.as<K>();
   uint32_t* vb = w.vals_alt.as<uint32_t>();
   for (int p = 0; p < passes; ++p) {
-    k_onesweep<K><<<kSortGrid, kSortThreads, 0, s>>>(ka, va, kb, vb, count_dev, cap, 8 * p, ghist + 256 * p,
-                                                     w.lookback.as<uint32_t>() + (size_t)256 * max_tiles * p,
-                                                     counters + p, err, w.spin_limit, w.stall_tile);
+    const uint32_t* vin = p == 0 && iota ? nullptr : va;
+    uint32_t* st = status + (size_t)256 * max_tiles * p;
+    if (is_short)
+      k_onesweep<K, kItemsShort><<<grid, kSortThreads, 0, s>>>(ka, vin, kb, vb, count_dev, cap, 8 * p, ghist + 256 * p,
+                                                               st, counters + p, err, w.spin_limit, w.stall_tile);
+    else
+      k_onesweep<K, kItemsLong><<<grid, kSortThreads, 0, s>>>(ka, vin, kb, vb, count_dev, cap, 8 * p, ghist + 256 * p,
+                                                              st, counters + p, err, w.spin_limit, w.stall_tile);
     NPS_CHECK_LAUNCH();
-    K* tk = ka; ka = kb; kb = tk;
-    uint32_t* tv = va; va = vb; vb = tv;
+    std::swap(ka, kb);
+    std::swap(va, vb);
   }
   *keys_out = ka;
   *vals_out = va;
@@ -368,8 +550,8 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
 }
 
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out) {
-  return radix_sort_impl<uint32_t>(keys, vals, count_dev, cap, bits, w, s, keys_out, vals_out);
+                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota) {
+  return radix_sort_impl<uint32_t>(keys, vals, count_dev, cap, bits, w, s, keys_out, vals_out, iota);
 }
 
 
@@ -416,7 +598,7 @@ extern "C" int nps_sort_pairs(nps_ctx* ctx, uint32_t* keys, uint32_t* vals, uint
     rc = NPS_ERR_CUDA;
   if (rc == NPS_ERR_CUDA) set_error("sort_pairs: %s", cudaGetErrorString(cudaGetLastError()));
   cudaStreamSynchronize(s);
-  for (DevBuf* b : {&w.hist, &w.partial, &w.lookback, &w.keys_alt, &w.vals_alt, &count}) b->release();
+  for (DevBuf* b : {&w.partial, &w.lookback, &w.keys_alt, &w.vals_alt, &count}) b->release();
   if (rc == NPS_OK && timeouts) {
     set_error("sort_pairs: %u look-back waits gave up (the output is not sorted)", timeouts);
     return NPS_ERR_TIMEOUT;

@@ -62,6 +62,26 @@ def test_sort_matches_numpy_stable(lib, what, n, bits):
     np.testing.assert_array_equal(k, keys[order])
 
 
+@pytest.mark.parametrize("n", [2, 31, 1023, 4096, 4097, 8192, 8193, 262144, 262145, 592 * 3072, 592 * 3072 + 1])
+@pytest.mark.parametrize("bits,common", [(8, 0), (32, 0), (32, 0xFF000000), (24, 0x00FF00)])
+def test_sort_at_the_limits_of_its_paths(lib, n, bits, common):
+    """One block (4 and 8 items per thread) and the first count beyond; the last count of short tiles and the first of
+    long ones; one wave of tiles and one tile more; digits that all keys share (top, middle); keys aligned to 4 bytes
+    only."""
+    rng = np.random.default_rng(n + bits)
+    keys = rng.integers(0, 2 ** bits, n + 1, dtype=np.uint64).astype(np.uint32)
+    keys = (keys & ~np.uint32(common)) | np.uint32(0x40302010 & common)
+    vals = rng.integers(0, 2 ** 32, n + 1, dtype=np.uint64).astype(np.uint32)
+    k, v = (torch.from_numpy(a.view(np.int32)).cuda() for a in (keys, vals))
+    torch.cuda.synchronize()
+    rc = lib.load().nps_sort_pairs(lib.context(0), ctypes.c_void_p(k.data_ptr() + 4), ctypes.c_void_p(v.data_ptr() + 4),
+                                   n, bits, 0, 0xFFFFFFFF)
+    assert rc == 0, lib.load().nps_last_error()
+    order = np.argsort(keys[1:], kind="stable")
+    np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32)[1:], keys[1:][order])
+    np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32)[1:], vals[1:][order])
+
+
 def test_lookback_gives_up_on_a_stalled_tile(lib):
     """Tile 2's status is treated as never published and the look-back may
     poll it 1000 times: the sort reports NPS_ERR_TIMEOUT, writes nothing
