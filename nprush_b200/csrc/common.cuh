@@ -84,8 +84,14 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
 // keys/vals hold the input; on return *keys_out / *vals_out point at the sorted
 // arrays (either the inputs or the work buffers).  iota: the values are 0, 1,
 // 2, ... and vals is only room for cap of them.
+// cleared: the caller has zeroed the region that radix_sort_prepare names (in
+// a kernel that clears other things too), else the sort does it.
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota = false);
+                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota = false, bool cleared = false);
+
+// Sizes the sort's buffers and gives the region (16-byte aligned and sized,
+// possibly empty) that has to be zero before each sort of these sizes.
+int radix_sort_prepare(uint32_t cap, int bits, SortWork& w, void** region, size_t* bytes);
 
 
 }  // namespace nps

@@ -7,8 +7,7 @@
 //                  tile rectangle of the alpha >= 1/255 ellipse, SH colour,
 //                  depth key
 //   radix sort     32-bit depth keys of all (view, Gaussian) records
-//   k_gather_counts + scan + k_emit: (view * tiles + tile, record) pairs
-//                  written in depth order
+//   k_bin_emit     (view * tiles + tile, record) pairs written in depth order
 //   radix sort     stable by tile key -> every tile list is depth ordered
 //   k_ranges       tile list bounds
 //   k_fwd          one CTA per (tile, view): records staged in shared memory
@@ -361,12 +360,6 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
   dkeys[g] = key;
 }
 
-__global__ void k_gather_counts(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins, uint32_t m,
-                                uint32_t* __restrict__ out) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < m) out[j] = bins[sorted_g[j]].w;
-}
-
 // Index of the k-th set bit of m (k below its population count), by halving.
 __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
   uint32_t at = 0;
@@ -382,59 +375,171 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
   return at;
 }
 
-// One warp per 32 consecutive depth-sorted (view, Gaussian) entries: their
-// pairs are one contiguous output range, written 32 consecutive slots at a
-// time (coalesced); each lane finds the entry owning its slot by a binary
-// search over the warp's offsets (shuffles).  Output identical to writing
-// each entry's tile rectangle row by row.  An entry's fields are one 16-byte word
-// and its slots need no integer division: 84 -> 52 us at 11.5 M pairs, 310 -> 187
-// us at 38 M.
-__global__ void __launch_bounds__(256) k_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
-                                              const uint32_t* __restrict__ offsets, uint32_t m, uint32_t n,
-                                              uint32_t tiles_x, uint32_t num_tiles, uint32_t cap,
-                                              uint32_t* __restrict__ keys, uint32_t* __restrict__ vals) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
-  if (__all_sync(0xffffffffu, j >= m)) return;
-  // per entry: its record, first slot, tile mask (all ones: every tile), key of its first tile and row width
-  uint32_t g = 0, c = 0, off = 0xffffffffu, tm = 0, key0 = 0, w = 1;
-  if (j < m) {
-    g = sorted_g[j];
-    off = offsets[j];
-    const uint4 b = bins[g];
-    c = b.w;
-    const uint32_t x0 = b.x & 0xffffu;
-    w = max((b.x >> 16) - x0, 1u);
-    tm = rect_tiles(b.x, b.y) <= 32u ? b.z : 0xffffffffu;
-    key0 = (g / n) * num_tiles + (b.y & 0xffffu) * tiles_x + x0;
-  }
-  const float iw = 1.0f / (float)w;
-  const uint32_t start = __shfl_sync(0xffffffffu, off, 0);
-  const uint32_t end = __reduce_max_sync(0xffffffffu, j < m ? off + c : 0u);
-  for (uint32_t base = start; base < end; base += 32) {
-    const uint32_t sl = base + lane;
-    // largest lane whose offset <= sl (lanes past m carry offset ~0u)
-    uint32_t L = 0;
+// Writes the pairs of the depth-sorted (view, Gaussian) entries in their order,
+// positions beyond cap dropped, and their number to *total: one kernel
+// gathers the entries' records, scans their counts and emits (instead of a
+// gather, three scan kernels, a host round trip for the total and an emit that
+// gathers again; with the clears in one launch, the status written by Adam's
+// preparation and the count read back behind the raster, a step of 1k Gaussians
+// goes 217 -> 190 us, two views of 16k 809 -> 717 us one at a time).
+//
+// A block claims a tile of kBinTile entries from a counter, publishes the tile's
+// pair count, finds the pairs of all earlier tiles by a decoupled look-back 32
+// tiles at a time (earlier tiles were claimed by blocks that run), and emits: a
+// warp takes 32 entries at a time, whose pairs are one contiguous output range
+// written 32 consecutive slots at a time (coalesced); each lane finds the
+// entry owning its slot by a binary search over the warp's offsets (shuffles).
+// Output identical to writing each entry's tile rectangle row by row.  An
+// entry's fields are one 16-byte word and its slots need no integer division
+// (84 -> 52 us at 11.5 M pairs).
+//
+// Status words as in the sort (flag and 32-bit count), cleared beforehand.  The
+// look-back is bounded: after spin_limit polls of an unpublished tile the
+// block counts a timeout in *err and carries on; positions stay below cap.
+// host (page-locked, may be null) gets the total and *err for the host.
+constexpr uint32_t kBinTile = 1024;
+__global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
+                                                  uint32_t m, uint32_t n, uint32_t tiles_x, uint32_t num_tiles,
+                                                  uint32_t cap, uint32_t* __restrict__ keys,
+                                                  uint32_t* __restrict__ vals, uint32_t* __restrict__ total,
+                                                  unsigned long long* __restrict__ status,
+                                                  uint32_t* __restrict__ counter, uint32_t* __restrict__ err,
+                                                  uint32_t spin_limit, volatile uint32_t* host) {
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32;
+  __shared__ uint32_t s_tile, s_excl, s_warp[8];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t tiles = (m + kBinTile - 1) / kBinTile;
+  auto load_status = [&](uint32_t t) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(status + t) : "memory");
+    return w;
+  };
+  auto store_status = [&](uint32_t t, unsigned long long w) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(status + t), "l"(w) : "memory");
+  };
+  for (;;) {
+    __syncthreads();  // the tile before is done with the shared words
+    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile >= tiles) return;
+    const uint32_t first = tile * kBinTile + warp * 128u + lane;
+    uint32_t g[4], off[4];
+    uint4 b[4];
 #pragma unroll
-    for (uint32_t step = 16; step > 0; step >>= 1) {
-      const uint32_t o2 = __shfl_sync(0xffffffffu, off, L + step);
-      if (o2 <= sl) L += step;
+    for (int q = 0; q < 4; ++q) g[q] = first + 32 * q < m ? sorted_g[first + 32 * q] : 0u;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = first + 32 * q < m ? bins[g[q]] : make_uint4(0u, 0u, 0u, 0u);
+    uint32_t run = 0;  // pairs of the warp's entries so far
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t inc = b[q].w;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kFull, inc, o);
+        if ((int)lane >= o) inc += y;
+      }
+      off[q] = run + inc - b[q].w;
+      run += __shfl_sync(kFull, inc, 31);
     }
-    const uint32_t gL = __shfl_sync(0xffffffffu, g, L), oL = __shfl_sync(0xffffffffu, off, L);
-    const uint32_t kL = __shfl_sync(0xffffffffu, key0, L), wL = __shfl_sync(0xffffffffu, w, L);
-    const uint32_t tmL = __shfl_sync(0xffffffffu, tm, L);
-    const float iwL = __shfl_sync(0xffffffffu, iw, L);
-    if (sl < end && sl < cap) {
-      const uint32_t k = sl - oL;
-      // the tile's index in the box: the k-th of the mask, or the k-th
-      const uint32_t local = tmL != 0xffffffffu ? nth_set_bit(tmL, k) : k;
-      // its row: exact, one correction on the float quotient
-      uint32_t ry = (uint32_t)((float)local * iwL);
-      if (ry * wL > local) --ry;
-      else if ((ry + 1) * wL <= local) ++ry;
-      keys[sl] = kL + ry * tiles_x + (local - ry * wL);
-      vals[sl] = gL;
+    if (lane == 0) s_warp[warp] = run;
+    __syncthreads();
+    uint32_t before = 0, sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < 8; ++k) {
+      before += k < warp ? s_warp[k] : 0u;
+      sum += s_warp[k];
+    }
+    if (warp == 0) {
+      uint32_t excl = 0;
+      if (tile == 0) {
+        if (lane == 0) store_status(0, kInc | sum);
+      } else {
+        if (lane == 0) store_status(tile, kAgg | sum);
+        uint32_t j = tile, polls = 0;  // tiles below j are still to be added
+        while (j > 0) {
+          const unsigned long long w = lane < j ? load_status(j - 1 - lane) : kInc;
+          const uint32_t inc = __ballot_sync(kFull, (w & kInc) != 0ull), none = __ballot_sync(kFull, (w >> 32) == 0ull);
+          const uint32_t take = inc ? inc ^ (inc - 1u) : kFull;  // up to the nearest inclusive prefix
+          if (none & take) {
+            if (++polls > spin_limit) {
+              if (lane == 0) atomicAdd(err, 1u);
+              break;
+            }
+            continue;
+          }
+          excl += __reduce_add_sync(kFull, (take >> lane) & 1u ? (uint32_t)w : 0u);
+          if (inc) break;
+          j -= 32;
+        }
+        if (lane == 0) store_status(tile, kInc | (uint32_t)(excl + sum));
+      }
+      if (lane == 0) {
+        s_excl = excl;
+        if (tile == tiles - 1) {
+          *total = excl + sum;
+          if (host) {
+            host[0] = excl + sum;
+            host[1] = *(volatile uint32_t*)err;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    const uint32_t warp0 = s_excl + before;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint32_t start = warp0 + __shfl_sync(kFull, off[q], 0);
+      const uint32_t end = warp0 + __shfl_sync(kFull, off[q] + b[q].w, 31);
+      if (start == end) continue;
+      // per entry: first slot, tile mask (all ones: every tile), key of its first tile and row width
+      const uint32_t o = warp0 + off[q], x0 = b[q].x & 0xffffu, w = max((b[q].x >> 16) - x0, 1u);
+      const uint32_t tm = rect_tiles(b[q].x, b[q].y) <= 32u ? b[q].z : 0xffffffffu;
+      const uint32_t key0 = (g[q] / n) * num_tiles + (b[q].y & 0xffffu) * tiles_x + x0;
+      const float iw = 1.0f / (float)w;
+      for (uint32_t base = start; base < end; base += 32) {
+        const uint32_t sl = base + lane;
+        uint32_t L = 0;  // largest lane whose first slot <= sl
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+          const uint32_t o2 = __shfl_sync(kFull, o, L + step);
+          if (o2 <= sl) L += step;
+        }
+        const uint32_t gL = __shfl_sync(kFull, g[q], L), oL = __shfl_sync(kFull, o, L);
+        const uint32_t kL = __shfl_sync(kFull, key0, L), wL = __shfl_sync(kFull, w, L);
+        const uint32_t tmL = __shfl_sync(kFull, tm, L);
+        const float iwL = __shfl_sync(kFull, iw, L);
+        if (sl < end && sl < cap) {
+          const uint32_t k = sl - oL;
+          // the tile's index in the box: the k-th of the mask, or the k-th
+          const uint32_t local = tmL != 0xffffffffu ? nth_set_bit(tmL, k) : k;
+          // its row: exact, one correction on the float quotient
+          uint32_t ry = (uint32_t)((float)local * iwL);
+          if (ry * wL > local) --ry;
+          else if ((ry + 1) * wL <= local) ++ry;
+          keys[sl] = kL + ry * tiles_x + (local - ry * wL);
+          vals[sl] = gL;
+        }
+      }
     }
   }
+}
+
+// Everything a forward (and a train step's backward) needs zeroed, and one
+// word set, in one launch: a memset node costs a small step as much as a kernel.
+struct ClearList {
+  uint4* p[6];
+  uint32_t n16[6];
+  uint32_t* word;
+  uint32_t value;
+};
+__global__ void __launch_bounds__(256) k_clear(ClearList c) {
+  const uint32_t t = blockIdx.x * 256 + threadIdx.x, stride = gridDim.x * 256;
+  if (t == 0 && c.word) *c.word = c.value;
+#pragma unroll
+  for (int r = 0; r < 6; ++r)
+    for (uint32_t i = t; i < c.n16[r]; i += stride) c.p[r][i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // Four consecutive sorted keys per thread from one 16-byte load (the key
@@ -1638,16 +1743,20 @@ struct AdamArgs {
 // pair buffers hold (only possible in a captured graph, whose capacity is
 // fixed: parameters stay unchanged and the host grows the capacity), or when
 // a bounded wait gave up since the last step (its results are incomplete).
-__global__ void k_adam_prep(uint32_t* st, const uint32_t* total, uint32_t cap) {
+// host (page-locked, may be null): the pair count, [4] and [6] for the host,
+// written here because a graph's copy nodes cost a small step 6 us each.
+__global__ void k_adam_prep(uint32_t* st, const uint32_t* total, uint32_t cap, volatile uint32_t* host) {
   const bool overflow = *total > cap;
   const bool timed_out = st[6] != st[7];
   st[7] = st[6];
   st[1] = (overflow || timed_out) ? 1u : 0u;
-  if (overflow) {
-    st[4] += 1u;  // skipped steps so far (read by the host after graph replays)
-    return;
+  if (overflow) st[4] += 1u;  // skipped steps so far (read by the host after graph replays)
+  if (host) {
+    host[0] = *total;
+    host[1] = st[4];
+    host[2] = st[6];
   }
-  if (timed_out) return;
+  if (overflow || timed_out) return;
   const uint32_t step = st[0] + 1;
   st[0] = step;
   st[2] = __float_as_uint((float)(1.0 - pow(0.9, (double)step)));
@@ -1931,9 +2040,11 @@ struct nps_gs {
   const float4* tgt = nullptr;
   // views of the current step
   uint32_t nv = 0;
-  DevBuf views, tids;
+  DevBuf views;  // nv view records, then nv target ids (one upload)
+  const uint32_t* tids() const { return reinterpret_cast<const uint32_t*>(views.as<float>() + (size_t)gsm::kViewRec * nv); }
   // forward state
-  DevBuf recs, counts, bins, dkeys, dvals, cnt_sorted, offsets, total, mcount, keys, vals, ranges;
+  DevBuf recs, counts, bins, dkeys, dvals, total, mcount, keys, vals, ranges;
+  DevBuf bin_status;             // k_bin_emit: tile counter, then one status word per tile
   DevBuf img, ncontrib;
   DevBuf maps, partial, loss, dimg, g2;
   SortWork sw_depth, sw_tile;
@@ -1961,7 +2072,10 @@ struct nps_gs {
     cudaEvent_t done = nullptr;
   } vstage[4];
   uint32_t vstage_next = 0;
-  uint32_t* h_status = nullptr;  // pinned: pair count of the last graph replay
+  uint32_t* h_status = nullptr;  // pinned: pair count, skips and timeouts of the last graph replay
+  uint32_t* h_fwd = nullptr;     // pinned: pair count and timeouts of the last eager forward
+  cudaEvent_t fwd_counted = nullptr;
+  bool g2_cleared = false;       // the forward cleared the backward's accumulators too
   uint64_t gkey = 0;
   uint32_t gcap = 0, skipped = 0;
   uint32_t graph_kernels = 0;  // kernel nodes of the captured step (launches per replay)
@@ -2115,6 +2229,8 @@ int nps_gs_destroy(nps_gs* o) {
     if (st.host) cudaFreeHost(st.host);
   }
   if (o->h_status) cudaFreeHost(o->h_status);
+  if (o->h_fwd) cudaFreeHost(o->h_fwd);
+  if (o->fwd_counted) cudaEventDestroy(o->fwd_counted);
   for (auto& u : o->ev_used) { cudaEventDestroy(u.second.first); cudaEventDestroy(u.second.second); }
   for (auto& u : o->gtimers) { cudaEventDestroy(u.second.first); cudaEventDestroy(u.second.second); }
   for (cudaEvent_t e : o->ev_pool) cudaEventDestroy(e);
@@ -2125,8 +2241,7 @@ int nps_gs_destroy(nps_gs* o) {
     b->release();
   for (DevBuf* b : {&o->tile_last, &o->ws_order_f, &o->ws_order_b, &o->ws_q}) b->release();
   for (DevBuf* b : {&o->params, &o->grads, &o->am, &o->av, &o->adc_grad, &o->adc_denom, &o->tgt_own, &o->views,
-                    &o->tids, &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals,
-                    &o->cnt_sorted, &o->offsets, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->img,
+                    &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals, &o->bin_status, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->img,
                     &o->ncontrib, &o->maps,
                     &o->partial, &o->loss, &o->dimg, &o->g2, &o->sw_depth.partial,
                     &o->sw_depth.lookback, &o->sw_depth.keys_alt, &o->sw_depth.vals_alt, &o->sw_tile.partial, &o->sw_tile.lookback, &o->sw_tile.keys_alt, &o->sw_tile.vals_alt})
@@ -2324,11 +2439,10 @@ int nps_gs_set_views(nps_gs* o, const float* vp, const float* vp_inv, const uint
       return NPS_ERR_INVALID;
     }
   }
-  NPS_TRY(o->views.ensure(sizeof(float) * host.size()));
-  NPS_TRY(o->tids.ensure(sizeof(uint32_t) * nv));
+  NPS_TRY(o->views.ensure(sizeof(float) * host.size() + sizeof(uint32_t) * nv));
   cudaStream_t s = o->ctx->stream;
-  // stage through a pinned slot so that the copies queue behind in-flight
-  // work instead of waiting for it; a slot is reused once its copies are done
+  // stage through a pinned slot so that the copy queues behind in-flight
+  // work instead of waiting for it; a slot is reused once its copy is done
   nps_gs::Stage& sl = o->vstage[o->vstage_next];
   o->vstage_next = (o->vstage_next + 1) % 4;
   const size_t vb = sizeof(float) * host.size(), ib = sizeof(uint32_t) * nv;
@@ -2343,8 +2457,7 @@ int nps_gs_set_views(nps_gs* o, const float* vp, const float* vp_inv, const uint
   }
   std::memcpy(sl.host, host.data(), vb);
   std::memcpy(static_cast<char*>(sl.host) + vb, ids.data(), ib);
-  NPS_CUDA(cudaMemcpyAsync(o->views.p, sl.host, vb, cudaMemcpyHostToDevice, s));
-  NPS_CUDA(cudaMemcpyAsync(o->tids.p, static_cast<char*>(sl.host) + vb, ib, cudaMemcpyHostToDevice, s));
+  NPS_CUDA(cudaMemcpyAsync(o->views.p, sl.host, vb + ib, cudaMemcpyHostToDevice, s));
   NPS_CUDA(cudaEventRecord(sl.done, s));
   o->nv = nv;
   o->fwd_valid = false;
@@ -2353,11 +2466,6 @@ int nps_gs_set_views(nps_gs* o, const float* vp, const float* vp_inv, const uint
 
 }  // extern "C"
 
-// Forward over all views.  Eager (capture == false): reads the pair count back
-// and grows the pair buffers to fit.  Captured (capture == true): no host
-// synchronisation; the pair buffers keep their capacity and the emit kernel
-// drops pairs beyond it (Adam then skips the step, see k_adam_prep).
-// Raster launches of the current forward state, by variant (pixels per thread).
 // Raster variants: (form, pixels per thread, records staged per batch), for
 // a tile edge T.  Form 0: one CTA per (tile, view), records double-buffered
 // (k_fwd, k_bwd2), T = 16 only; form 1: persistent warp-specialised kernels
@@ -2411,7 +2519,7 @@ static int ensure_ws_buffers(nps_gs* o, uint32_t nitems) {
 // Raster launches of the current forward state, by variant.  Both forms
 // write every tile's last contributor (tile_last), which orders and bounds
 // the persistent backward whatever form the forward took.
-static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage) {
+static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool cleared = false) {
   cudaStream_t s = o->ctx->stream;
   const uint32_t W = o->w, H = o->h, nv = o->nv;
   const uint32_t tiles_x = div_up(W, o->tile), tiles_y = div_up(H, o->tile), num_tiles = tiles_x * tiles_y;
@@ -2420,7 +2528,7 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage) {
   const uint32_t* rend = rstart + (size_t)num_tiles * nv;
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
   NPS_TRY(ensure_ws_buffers(o, nitems));
-  NPS_CUDA(cudaMemsetAsync(o->tile_last.p, 0, sizeof(uint32_t) * (size_t)nitems, s));
+  if (!cleared) NPS_CUDA(cudaMemsetAsync(o->tile_last.p, 0, sizeof(uint32_t) * (size_t)nitems, s));
   uint32_t* err = o->stepst.as<uint32_t>() + 6;
   if (form == 1) {
     uint32_t* q = o->ws_q.as<uint32_t>();
@@ -2571,7 +2679,12 @@ static int launch_bwd_raster(nps_gs* o, int form, int ppt, int stage, const floa
   return NPS_OK;
 }
 
-static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
+// Forward over all views.  capture: no host synchronisation; the pair buffers
+// keep their capacity and pairs beyond it are dropped (Adam then skips the step,
+// see k_adam_prep).  Else the pair count comes back while the raster runs, and
+// a forward whose pairs outgrew the buffers is repeated from the emission on
+// with larger ones.  train: a backward follows; its accumulators are cleared here.
+static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train = false) {
   if (o->nv == 0 || o->w == 0) {
     set_error("gs_forward: set_views and set_targets (or set_image_size) first");
     return NPS_ERR_STATE;
@@ -2579,27 +2692,64 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
   cudaStream_t s = o->ctx->stream;
   const uint32_t n = o->n, nv = o->nv, W = o->w, H = o->h;
   const uint32_t tiles_x = div_up(W, o->tile), tiles_y = div_up(H, o->tile), num_tiles = tiles_x * tiles_y;
-  const size_t M = (size_t)n * nv;
+  const size_t M = (size_t)n * nv, nitems = (size_t)num_tiles * nv;
   const size_t npix = (size_t)W * H * nv;
   if (M >= (1ull << 31) || (uint64_t)num_tiles * nv >= (1ull << 31)) {
     set_error("gs_forward: problem too large");
     return NPS_ERR_INVALID;
   }
+  const uint32_t bin_tiles = div_up(M, gs::kBinTile);
+  auto up16 = [](size_t b) { return (b + 15) / 16 * 16; };
   NPS_TRY(o->recs.ensure(sizeof(gs::Rec) * (M + 1)));
   NPS_TRY(o->counts.ensure(sizeof(uint32_t) * (M + 1)));
   NPS_TRY(o->bins.ensure(sizeof(uint4) * (M + 1)));
   NPS_TRY(o->dkeys.ensure(sizeof(uint32_t) * (M + 1)));
   NPS_TRY(o->dvals.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->cnt_sorted.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->offsets.ensure(sizeof(uint32_t) * (M + 1)));
-  NPS_TRY(o->ranges.ensure(sizeof(uint32_t) * 2 * (size_t)num_tiles * nv));
+  NPS_TRY(o->bin_status.ensure(up16(16 + 8 * (size_t)bin_tiles)));
+  NPS_TRY(o->ranges.ensure(up16(sizeof(uint32_t) * 2 * nitems)));
+  NPS_TRY(o->tile_last.ensure(up16(sizeof(uint32_t) * nitems)));
   NPS_TRY(o->img.ensure(sizeof(float4) * npix));
   NPS_TRY(o->ncontrib.ensure(sizeof(uint32_t) * npix));
+  if (train) NPS_TRY(o->g2.ensure(sizeof(float) * gs::kG2 * (M + 1)));
+  if (!capture && !o->h_fwd) {
+    NPS_CUDA(cudaMallocHost((void**)&o->h_fwd, 16));
+    NPS_CUDA(cudaEventCreateWithFlags(&o->fwd_counted, cudaEventDisableTiming));
+  }
   uint32_t* rstart = o->ranges.as<uint32_t>();
-  uint32_t* rend = rstart + (size_t)num_tiles * nv;
-  NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * (size_t)num_tiles * nv, s));
+  uint32_t* rend = rstart + nitems;
+  uint32_t* total = o->total.as<uint32_t>();
+  uint32_t* err = o->stepst.as<uint32_t>() + 6;
+  int bits = 1;
+  while ((1ull << bits) < (uint64_t)nitems) ++bits;
+  void *dclear = nullptr, *tclear = nullptr;
+  size_t dbytes = 0, tbytes = 0;
+  if (M > 0) {
+    NPS_TRY(radix_sort_prepare((uint32_t)M, 32, o->sw_depth, &dclear, &dbytes));
+    if (o->pair_cap) NPS_TRY(radix_sort_prepare(o->pair_cap, bits, o->sw_tile, &tclear, &tbytes));
+  }
+  gs::ClearList cl{};
+  size_t n16 = 0;
+  int nr = 0;
+  auto clear = [&](void* p, size_t bytes) {
+    if (bytes == 0) return;
+    cl.p[nr] = static_cast<uint4*>(p);
+    cl.n16[nr++] = (uint32_t)(up16(bytes) / 16);
+    n16 += up16(bytes) / 16;
+  };
+  clear(o->ranges.p, sizeof(uint32_t) * 2 * nitems);
+  clear(o->tile_last.p, sizeof(uint32_t) * nitems);
+  clear(dclear, dbytes);
+  clear(tclear, tbytes);
+  clear(o->bin_status.p, 16 + 8 * (size_t)bin_tiles);
+  if (train) clear(o->g2.p, sizeof(float) * gs::kG2 * M);
+  cl.word = o->mcount.as<uint32_t>();
+  cl.value = (uint32_t)M;
+  gs::k_clear<<<std::min(div_up(n16, 512), 8u * kNumSMs), 256, 0, s>>>(cl);
+  NPS_CHECK_LAUNCH();
+  o->g2_cleared = train;
   uint32_t K = 0;
   const uint32_t* vs = o->counts.as<uint32_t>();
+  uint32_t *dk = nullptr, *dv = nullptr;
   if (M > 0) {
     { StageTimer t_pre(o, ST_PRE);
     // whole warps of one view; at most 256 threads
@@ -2617,62 +2767,67 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture) {
     }
 #undef NPS_PRE
     NPS_CHECK_LAUNCH(); }
-    k_set_u32<<<1, 1, 0, s>>>(o->mcount.as<uint32_t>(), (uint32_t)M);
-    uint32_t *dk = nullptr, *dv = nullptr;
     { StageTimer t(o, ST_DSORT);
     NPS_TRY(radix_sort_u32(o->dkeys.as<uint32_t>(), o->dvals.as<uint32_t>(), o->mcount.as<uint32_t>(), (uint32_t)M, 32,
-                           o->sw_depth, s, &dk, &dv, true)); }
-    o->sorted_vals = dv;
-    gs::k_gather_counts<<<div_up(M, 256), 256, 0, s>>>(dv, o->bins.as<uint4>(), (uint32_t)M,
-                                                        o->cnt_sorted.as<uint32_t>());
-    NPS_CHECK_LAUNCH();
-    uint32_t* total = o->total.as<uint32_t>();
-    NPS_TRY(exclusive_scan_u32(o->cnt_sorted.as<uint32_t>(), o->offsets.as<uint32_t>(), (uint32_t)M, total, o->sw_tile,
-                               s));
-    if (!capture) {
-      uint32_t tmo = 0;
-      NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      NPS_CUDA(cudaMemcpyAsync(&tmo, o->stepst.as<uint32_t>() + 6, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-      NPS_CUDA(cudaStreamSynchronize(s));
-      if (tmo != o->timeouts_seen) {
-        // reported here: the next Adam step must not skip for it again
-        o->timeouts_seen = tmo;
-        k_set_u32<<<1, 1, 0, s>>>(o->stepst.as<uint32_t>() + 7, tmo);
-        set_error("gs_forward: a bounded device wait (sort look-back or raster staging) gave up in this or an "
-                  "earlier call; its results were incomplete and no update used them");
-        return NPS_ERR_TIMEOUT;
+                           o->sw_depth, s, &dk, &dv, true, true)); }
+  }
+  // The rest depends on the pair buffers' capacity: a second round only where
+  // the count came back larger (or there were no buffers yet).
+  for (int round = 0;; ++round) {
+    const bool cleared = round == 0;
+    const uint32_t cap = o->pair_cap;
+    if (M > 0) {
+      if (!cleared) {
+        NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * nitems, s));
+        NPS_CUDA(cudaMemsetAsync(o->bin_status.p, 0, 16 + 8 * (size_t)bin_tiles, s));
       }
-      if (K > o->pair_cap || o->pair_cap == 0) {
-        const uint32_t cap = K + K / 4 + 4096;
-        NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)cap));
-        NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)cap));
-        o->pair_cap = cap;
-      }
-    }
-    if (K > 0 || capture) {
       { StageTimer t(o, ST_EMIT);
-      gs::k_emit<<<div_up(M, 256), 256, 0, s>>>(dv, o->bins.as<uint4>(), o->offsets.as<uint32_t>(), (uint32_t)M, n,
-                                                 tiles_x, num_tiles, o->pair_cap, o->keys.as<uint32_t>(),
-                                                 o->vals.as<uint32_t>());
+      gs::k_bin_emit<<<std::min<uint32_t>(bin_tiles, 8u * kNumSMs), 256, 0, s>>>(
+          dv, o->bins.as<uint4>(), (uint32_t)M, n, tiles_x, num_tiles, cap, o->keys.as<uint32_t>(),
+          o->vals.as<uint32_t>(), total, reinterpret_cast<unsigned long long*>(o->bin_status.as<char>() + 16),
+          o->bin_status.as<uint32_t>(), err, o->sw_tile.spin_limit, capture ? nullptr : o->h_fwd);
       NPS_CHECK_LAUNCH(); }
-      int bits = 1;
-      while ((1ull << bits) < (uint64_t)num_tiles * nv) ++bits;
-      uint32_t *ks = nullptr, *vv = nullptr;
-      { StageTimer t(o, ST_TSORT);
-      NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total, o->pair_cap, bits, o->sw_tile, s,
-                             &ks, &vv)); }
-      { StageTimer t(o, ST_RANGES);
-      gs::k_ranges<<<16 * kNumSMs, 256, 0, s>>>(ks, total, o->pair_cap, rstart, rend);
-      NPS_CHECK_LAUNCH(); }
-      vs = vv;
+      if (!capture) NPS_CUDA(cudaEventRecord(o->fwd_counted, s));
+      if (cap > 0) {
+        uint32_t *ks = nullptr, *vv = nullptr;
+        { StageTimer t(o, ST_TSORT);
+        NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total, cap, bits, o->sw_tile, s, &ks,
+                               &vv, false, cleared && tbytes > 0)); }
+        { StageTimer t(o, ST_RANGES);
+        gs::k_ranges<<<std::min(16u * kNumSMs, div_up(cap, 1024)), 256, 0, s>>>(ks, total, cap, rstart, rend);
+        NPS_CHECK_LAUNCH(); }
+        vs = vv;
+      }
     }
+    o->sorted_vals = vs;
+    if (M == 0 || cap > 0) {
+      StageTimer t_fwd(o, ST_FWD);
+      NPS_TRY(launch_fwd_raster(o, o->fwd_form, o->fwd_ppt, o->fwd_stage, cleared));
+      NPS_CHECK_LAUNCH();
+    }
+    if (capture || M == 0) break;
+    NPS_CUDA(cudaEventSynchronize(o->fwd_counted));
+    K = o->h_fwd[0];
+    const uint32_t tmo = o->h_fwd[1];
+    if (tmo != o->timeouts_seen) {
+      // reported here: the next Adam step must not skip for it again
+      o->timeouts_seen = tmo;
+      k_set_u32<<<1, 1, 0, s>>>(o->stepst.as<uint32_t>() + 7, tmo);
+      o->fwd_valid = o->loss_valid = false;
+      set_error("gs_forward: a bounded device wait (sort look-back or raster staging) gave up in this or an "
+                "earlier call; its results were incomplete and no update used them");
+      return NPS_ERR_TIMEOUT;
+    }
+    if (cap > 0 && K <= cap) break;
+    const uint32_t want = K + K / 4 + 4096;
+    NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)want));
+    NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)want));
+    // slots that an emission which gave up waiting leaves unwritten hold valid keys and records
+    NPS_CUDA(cudaMemsetAsync(o->keys.p, 0, sizeof(uint32_t) * (size_t)want, s));
+    NPS_CUDA(cudaMemsetAsync(o->vals.p, 0, sizeof(uint32_t) * (size_t)want, s));
+    o->pair_cap = want;
   }
   o->K = K;
-  o->sorted_vals = vs;
-  const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
-  StageTimer t_fwd(o, ST_FWD);
-  NPS_TRY(launch_fwd_raster(o, o->fwd_form, o->fwd_ppt, o->fwd_stage));
-  NPS_CHECK_LAUNCH();
   if (out_rgba) NPS_CUDA(cudaMemcpyAsync(out_rgba, o->img.p, sizeof(float4) * npix, cudaMemcpyDeviceToDevice, s));
   o->fwd_valid = true;
   o->loss_valid = false;
@@ -2705,10 +2860,10 @@ int nps_gs_loss(nps_gs* o, float* loss3_host) {
     NPS_TRY(o->partial.ensure(sizeof(float) * 2 * nblocks));
     StageTimer t(o, ST_LOSS);
     if (o->loss_kind == gs::kLossL2)
-      gs::k_pix_loss<gs::kLossL2><<<grid, 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids.as<uint32_t>(), W * H,
+      gs::k_pix_loss<gs::kLossL2><<<grid, 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids(), W * H,
                                                        inv_norm, o->dimg.as<float4>(), o->partial.as<float>());
     else
-      gs::k_pix_loss<gs::kLossL1><<<grid, 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids.as<uint32_t>(), W * H,
+      gs::k_pix_loss<gs::kLossL1><<<grid, 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids(), W * H,
                                                        inv_norm, o->dimg.as<float4>(), o->partial.as<float>());
     gs::k_loss_reduce<<<1, gs::kThreads, 0, s>>>(o->partial.as<float>(), nblocks, o->loss_kind, 0.0f, inv_norm,
                                                  (float)nv / (float)lv, o->loss.as<float>());
@@ -2719,10 +2874,10 @@ int nps_gs_loss(nps_gs* o, float* loss3_host) {
     NPS_TRY(o->maps.ensure(sizeof(float) * 9 * npix));
     NPS_TRY(o->partial.ensure(sizeof(float) * 2 * nblocks));
     StageTimer t(o, ST_LOSS);
-    gs::k_ssim_fwd2<<<grid, 256, gs::kSsimFwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids.as<uint32_t>(), W, H,
+    gs::k_ssim_fwd2<<<grid, 256, gs::kSsimFwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids(), W, H,
                                                        o->lambda, inv_norm, o->maps.as<float>(),
                                                        o->partial.as<float>());
-    gs::k_ssim_bwd2<<<grid, 256, gs::kSsimBwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids.as<uint32_t>(),
+    gs::k_ssim_bwd2<<<grid, 256, gs::kSsimBwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids(),
                                                        o->maps.as<float>(), W, H, o->lambda, inv_norm,
                                                        o->dimg.as<float4>());
     gs::k_loss_reduce<<<1, gs::kThreads, 0, s>>>(o->partial.as<float>(), nblocks, o->loss_kind, o->lambda,
@@ -2752,7 +2907,8 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
   const uint32_t tiles_x = div_up(W, o->tile), tiles_y = div_up(H, o->tile), num_tiles = tiles_x * tiles_y;
   const size_t M = (size_t)n * nv;
   NPS_TRY(o->g2.ensure(sizeof(float) * gs::kG2 * (M + 1)));
-  NPS_CUDA(cudaMemsetAsync(o->g2.p, 0, sizeof(float) * gs::kG2 * M, s));
+  if (!o->g2_cleared) NPS_CUDA(cudaMemsetAsync(o->g2.p, 0, sizeof(float) * gs::kG2 * M, s));
+  o->g2_cleared = false;
   const uint32_t* rstart = o->ranges.as<uint32_t>();
   const uint32_t* rend = rstart + (size_t)num_tiles * nv;
   const float3 bg = make_float3(o->bg[0], o->bg[1], o->bg[2]);
@@ -2848,7 +3004,8 @@ int nps_gs_adam(nps_gs* o) {
   const uint32_t n4 = o->n * 16;
   StageTimer t_adam(o, ST_ADAM);
   gs::k_adam_prep<<<1, 1, 0, o->ctx->stream>>>(o->stepst.as<uint32_t>(), o->total.as<uint32_t>(),
-                                               o->pair_cap ? o->pair_cap : 0xffffffffu);
+                                               o->pair_cap ? o->pair_cap : 0xffffffffu,
+                                               o->capturing ? o->h_status : nullptr);
   gs::k_adam<<<div_up(n4, 256), 256, 0, o->ctx->stream>>>(o->params.as<float4>(), o->grads.as<float4>(),
                                                            o->am.as<float4>(), o->av.as<float4>(), n4, a,
                                                            o->stepst.as<uint32_t>());
@@ -2860,7 +3017,7 @@ int nps_gs_adam(nps_gs* o) {
 }  // extern "C"
 
 static int gs_step_eager(nps_gs* o) {
-  NPS_TRY(gs_forward_impl(o, nullptr, false));
+  NPS_TRY(gs_forward_impl(o, nullptr, false, true));
   NPS_TRY(nps_gs_loss(o, nullptr));
   NPS_TRY(nps_gs_backward(o, nullptr));
   NPS_TRY(nps_gs_adam(o));
@@ -2905,21 +3062,10 @@ static int gs_capture(nps_gs* o) {
   NPS_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   o->capturing = true;
   const uint32_t step_before = o->step;
-  int rc = gs_forward_impl(o, nullptr, true);
+  int rc = gs_forward_impl(o, nullptr, true, true);
   if (rc == NPS_OK) rc = nps_gs_loss(o, nullptr);
   if (rc == NPS_OK) rc = nps_gs_backward(o, nullptr);
   if (rc == NPS_OK) rc = nps_gs_adam(o);
-  if (rc == NPS_OK) {
-    cudaError_t e = cudaMemcpyAsync(o->h_status, o->total.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(o->h_status + 1, o->stepst.as<uint32_t>() + 4, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(o->h_status + 2, o->stepst.as<uint32_t>() + 6, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess) {
-      set_error("graph capture: %s", cudaGetErrorString(e));
-      rc = NPS_ERR_CUDA;
-    }
-  }
   o->capturing = false;
   o->step = step_before;  // captured, not executed
   cudaGraph_t graph = nullptr;
@@ -3208,7 +3354,7 @@ int nps_gs_psnr(nps_gs* o, float* psnr_host) {
   cudaStream_t s = o->ctx->stream;
   NPS_TRY(o->psnr_acc.ensure(sizeof(double) * o->nv));
   NPS_CUDA(cudaMemsetAsync(o->psnr_acc.p, 0, sizeof(double) * o->nv, s));
-  gs::k_sq_err<<<dim3(2 * kNumSMs, o->nv), 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids.as<uint32_t>(), o->w,
+  gs::k_sq_err<<<dim3(2 * kNumSMs, o->nv), 256, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids(), o->w,
                                                         o->h, o->psnr_acc.as<double>());
   NPS_CHECK_LAUNCH();
   std::vector<double> acc(o->nv);

@@ -472,36 +472,49 @@ int launch_small(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint
   return NPS_OK;
 }
 
+// How a sort of up to cap pairs is done, and its one cleared buffer: the
+// per-pass histograms, the per-pass tile counters, the timeout counter of callers
+// without their own, then the published counts per pass and tile.
+struct SortPlan {
+  bool one_block, is_short;
+  int passes;
+  uint32_t max_tiles;
+  size_t clear_bytes;
+};
+constexpr size_t kSortHead = 4 * 256 + 64;
+SortPlan sort_plan(uint32_t cap, int bits, const SortWork& w) {
+  SortPlan p;
+  p.passes = (bits + 7) / 8;
+  // a stalled tile (tests) stalls the onesweep's look-back
+  p.one_block = cap <= kSmallMax && w.stall_tile == 0xffffffffu;
+  p.is_short = cap <= kShortMax;
+  const uint32_t tile = kSortThreads * (p.is_short ? kItemsShort : kItemsLong);
+  p.max_tiles = (cap + tile - 1) / tile;
+  p.clear_bytes = p.one_block ? 0 : sizeof(uint32_t) * (kSortHead + 256 * (size_t)p.max_tiles * p.passes);
+  return p;
+}
+
 template <class K>
 int radix_sort_impl(K* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                    cudaStream_t s, K** keys_out, uint32_t** vals_out, bool iota) {
-  if (cap >= (1u << 30)) {
-    set_error("radix sort: capacity %u beyond the look-back's 30-bit counts", cap);
-    return NPS_ERR_INVALID;
-  }
-  const int passes = (bits + 7) / 8;
-  // one block's worth (a stalled tile, for tests, stalls the onesweep's look-back)
-  if (cap <= kSmallMax && w.stall_tile == 0xffffffffu) {
+                    cudaStream_t s, K** keys_out, uint32_t** vals_out, bool iota, bool cleared) {
+  void* region = nullptr;
+  size_t region_bytes = 0;
+  NPS_TRY(radix_sort_prepare(cap, bits, w, &region, &region_bytes));
+  const SortPlan plan = sort_plan(cap, bits, w);
+  const int passes = plan.passes;
+  if (plan.one_block) {
     *keys_out = keys;
     *vals_out = vals;
     return cap <= 4 * kSmallThreads ? launch_small<4>(keys, vals, count_dev, cap, passes, iota, s)
                                     : launch_small<8>(keys, vals, count_dev, cap, passes, iota, s);
   }
-  const bool is_short = cap <= kShortMax;
-  const uint32_t tile = kSortThreads * (is_short ? kItemsShort : kItemsLong);
-  const uint32_t max_tiles = (cap + tile - 1) / tile;
-  // one buffer, cleared at once: the per-pass histograms, the per-pass tile
-  // counters, the timeout counter of callers without their own, then the
-  // published counts per pass and tile
-  constexpr size_t kHead = 4 * 256 + 64;
-  NPS_TRY(w.lookback.ensure(sizeof(uint32_t) * (kHead + 256 * (size_t)max_tiles * 4)));
-  NPS_TRY(w.keys_alt.ensure(sizeof(K) * (size_t)cap));
-  NPS_TRY(w.vals_alt.ensure(sizeof(uint32_t) * (size_t)cap));
+  const bool is_short = plan.is_short;
+  const uint32_t max_tiles = plan.max_tiles;
   uint32_t* ghist = w.lookback.as<uint32_t>();
   uint32_t* counters = ghist + 4 * 256;
   uint32_t* err = w.err ? w.err : counters + 4;
-  uint32_t* status = ghist + kHead;
-  NPS_CUDA(cudaMemsetAsync(ghist, 0, sizeof(uint32_t) * (kHead + 256 * (size_t)max_tiles * passes), s));
+  uint32_t* status = ghist + kSortHead;
+  if (!cleared) NPS_CUDA(cudaMemsetAsync(region, 0, region_bytes, s));
   const uint32_t grid = std::min<uint32_t>(kSortGrid, max_tiles);
   switch (passes) {
     case 1: k_hist_all<K, 1><<<grid, kSortThreads, 0, s>>>(keys, count_dev, cap, ghist); break;
@@ -549,9 +562,25 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* 
   return NPS_OK;
 }
 
+int radix_sort_prepare(uint32_t cap, int bits, SortWork& w, void** region, size_t* bytes) {
+  if (cap >= (1u << 30)) {
+    set_error("radix sort: capacity %u beyond the look-back's 30-bit counts", cap);
+    return NPS_ERR_INVALID;
+  }
+  const SortPlan p = sort_plan(cap, bits, w);
+  *region = nullptr;
+  *bytes = p.clear_bytes;
+  if (p.one_block) return NPS_OK;
+  NPS_TRY(w.lookback.ensure(sizeof(uint32_t) * (kSortHead + 256 * (size_t)p.max_tiles * 4)));
+  NPS_TRY(w.keys_alt.ensure(sizeof(uint32_t) * (size_t)cap));
+  NPS_TRY(w.vals_alt.ensure(sizeof(uint32_t) * (size_t)cap));
+  *region = w.lookback.p;
+  return NPS_OK;
+}
+
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
-                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota) {
-  return radix_sort_impl<uint32_t>(keys, vals, count_dev, cap, bits, w, s, keys_out, vals_out, iota);
+                   cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota, bool cleared) {
+  return radix_sort_impl<uint32_t>(keys, vals, count_dev, cap, bits, w, s, keys_out, vals_out, iota, cleared);
 }
 
 
