@@ -340,6 +340,8 @@ int nps_gs_read_image(nps_gs* gs, float* rgba_host, float* dl_dimage_host);
  *     (view, tile) items longest first (the forward by list length, the
  *     backward by its last contributor), so the longest tiles start first
  *     and the grid's tail is short: T = 16, the (ppt, stage) of form 0.
+ * Until one is selected, form 0 runs on 16 x 16 tiles with 1 pixel per thread
+ * where the views have few tiles and 2 where they have many (per pass).
  * nps_gs_set_raster selects one per pass for the current tile (a stage of 0
  * means the form's default: 256 / ppt for form 0, 128 for form 1);
  * nps_gs_set_variant selects form 0; nps_gs_set_tile changes the tile (and

@@ -93,9 +93,6 @@ __device__ __forceinline__ bool rec_misses_box(const float4& a, float cc, const 
   return fminf(fminf(q1, q2), fminf(q3, q4)) > c.y;
 }
 
-#ifndef NPS_GS_SOLO
-#define NPS_GS_SOLO 0
-#endif
 #ifndef NPS_GS_STRIP_W
 #define NPS_GS_STRIP_W 8
 #endif
@@ -117,15 +114,15 @@ struct TileMap16 {
   __device__ static uint32_t y(uint32_t tid) { return wy(tid) + PPT * ((tid & 31) / kW); }
 };
 
-// Exponent of the Gaussian at offset d = (dx, dy) from its centre, -q(d) / 2
-// with q(d) = dx u + dy w and (u, w) the conic (a.z, a.w; a.w, cc) times d.
-// Every raster kernel evaluates it in this one order, so the forward and the
-// backward take the same alpha >= 1/255 decisions; u and w are reused by the
-// backward's mean gradient.
-__device__ __forceinline__ float gs_power(const float4& a, float cc, float dx, float dy, float& u, float& w) {
+// Quadratic form of the Gaussian at offset d = (dx, dy) from its centre (its
+// exponent is -q / 2): q = dx u + dy w with (u, w) the conic (a.z, a.w; a.w, cc)
+// times d.  Every raster kernel evaluates it in this one order, so the forward
+// and the backward take the same alpha >= 1/255 decisions; u and w are reused by
+// the backward's mean gradient.
+__device__ __forceinline__ float gs_quad(const float4& a, float cc, float dx, float dy, float& u, float& w) {
   u = fmaf(a.w, dy, a.z * dx);
   w = fmaf(cc, dy, a.w * dx);
-  return -0.5f * fmaf(dy, w, dx * u);
+  return fmaf(dy, w, dx * u);
 }
 
 // true if the Gaussian's alpha >= 1/255 box misses the warp's pixels
@@ -161,50 +158,85 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16], uint32_t lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// Sum of 9 values over the warp by uneven recursive halving: at each level a
-// lane keeps the first ceil(m/2) of its m partial values (lower half of the
-// lane pair) or the rest (upper half, padded with a zero), 5 + 3 + 2 + 1 + 1
-// = 12 shuffles.  On return, lanes 2q and 2q + 1 hold the warp total of value
-// warp_sum9_index(lane) when that is below 9 (every value has one q).
-__device__ __forceinline__ float warp_sum9(const float (&v)[9], uint32_t lane) {
-  const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
-  float w[5], x[3], y[2];
+// Sums of 9 values over the warp through shared memory (sm: one 9 x kRedStride
+// array per warp): each lane stores its values, then lanes 2k and 2k + 1 each add
+// half of row k in packed pairs and exchange their halves.  Returns value k's
+// total in lanes 2k, 2k + 1 (k < 9).  27 warp instructions; a reduce-scatter by
+// shuffles takes 12 shuffles and 40 selects and additions (50% more instructions
+// in a kernel bound by issue: backward 1020 -> 965 us at 200k Gaussians, 8 views of
+// 800 x 800).  A row of 36 words keeps the 16-byte loads of eight lanes, and the
+// stores, free of bank conflicts.
+constexpr int kRedStride = 36;
+__device__ __forceinline__ float warp_total9(const float (&v)[9], uint32_t lane, float* sm) {
+#pragma unroll
+  for (int k = 0; k < 9; ++k) sm[k * kRedStride + lane] = v[k];
+  __syncwarp();
+  const uint32_t l = min(lane, 17u);
+  const float4* c = reinterpret_cast<const float4*>(sm + (l >> 1) * kRedStride + (l & 1u) * 16u);
+  const float4 q0 = c[0], q1 = c[1], q2 = c[2], q3 = c[3];
+  const float2 s01 = __fadd2_rn(__fadd2_rn(make_float2(q0.x, q0.y), make_float2(q0.z, q0.w)),
+                                __fadd2_rn(make_float2(q1.x, q1.y), make_float2(q1.z, q1.w)));
+  const float2 s23 = __fadd2_rn(__fadd2_rn(make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)),
+                                __fadd2_rn(make_float2(q3.x, q3.y), make_float2(q3.z, q3.w)));
+  const float2 s = __fadd2_rn(s01, s23);
+  const float half = s.x + s.y;
+  const float t = half + __shfl_xor_sync(0xffffffffu, half, 1);
+  __syncwarp();  // sm may be written again
+  return t;
+}
+
+// Sums of two sets of 9 values over the warp by a reduce-scatter of shuffles (21
+// of them), the two sets sharing the levels after the first: the shorter chain
+// of the two reductions, for grids whose time is that chain.  warp_sum9x2_index
+// is the value whose total the lane returns (15: none); lanes with bit 3 set
+// return set B's.
+__device__ __forceinline__ void warp_half9(const float (&v)[9], uint32_t lane, float (&w)[5]) {
+  const bool b4 = lane & 16;
 #pragma unroll
   for (int j = 0; j < 5; ++j) {
     const float hi = j + 5 < 9 ? v[j + 5] : 0.0f;
     const float send = b4 ? v[j] : hi, keep = b4 ? hi : v[j];
     w[j] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
   }
+}
+__device__ __forceinline__ float warp_sum9x2(const float (&va)[9], const float (&vb)[9], uint32_t lane) {
+  const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2, b0 = lane & 1;
+  float wa[5], wb[5], x[5], y[3], z[2];
+  warp_half9(va, lane, wa);
+  warp_half9(vb, lane, wb);
 #pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const float hi = j + 3 < 5 ? w[j + 3] : 0.0f;
-    const float send = b3 ? w[j] : hi, keep = b3 ? hi : w[j];
+  for (int j = 0; j < 5; ++j) {
+    const float send = b3 ? wa[j] : wb[j], keep = b3 ? wb[j] : wa[j];
     x[j] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
   }
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const float hi = j + 2 < 3 ? x[j + 2] : 0.0f;
+  for (int j = 0; j < 3; ++j) {
+    const float hi = j + 3 < 5 ? x[j + 3] : 0.0f;
     const float send = b2 ? x[j] : hi, keep = b2 ? hi : x[j];
     y[j] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
   }
-  const float send = b1 ? y[0] : y[1], keep = b1 ? y[1] : y[0];
-  const float z = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  return z + __shfl_xor_sync(0xffffffffu, z, 1);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float hi = j + 2 < 3 ? y[j + 2] : 0.0f;
+    const float send = b1 ? y[j] : hi, keep = b1 ? hi : y[j];
+    z[j] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+  }
+  const float send = b0 ? z[0] : z[1], keep = b0 ? z[1] : z[0];
+  return keep + __shfl_xor_sync(0xffffffffu, send, 1);
+}
+__device__ __forceinline__ uint32_t warp_sum9x2_index(uint32_t lane) {
+  // of the five values of a half set, the one kept by lanes with low bits b2 b1 b0
+  const uint32_t x = (0xff43f210u >> (4u * (lane & 7u))) & 15u;
+  const uint32_t k = x + ((lane & 16u) ? 5u : 0u);
+  return x < 5u && k < 9u ? k : 15u;
 }
 
-// The value whose total warp_sum9 leaves in this lane; 15 for a padding slot.
-// Nibble q of the table is the index kept by lanes 2q, 2q + 1 (the
-// partition above traced through its four uneven levels).
-__device__ __forceinline__ uint32_t warp_sum9_index(uint32_t lane) {
-  return (uint32_t)(0xfff8f765ff43f210ull >> (4u * ((lane >> 1) & 15u))) & 15u;
-}
-
-// exp(x) for x in the range the rasters evaluate, [-6, 0]: __expf without the
-// scaling that it adds for results near the smallest floats (the same bits
-// here; three instructions fewer per pixel and pair)
-__device__ __forceinline__ float exp_raster(float x) {
+// exp(-q / 2): one multiplication and the special-function unit's 2^x.  Where
+// alpha can reach 1/255, -q / 2 is in [-6, 0] and the bits are __expf's; far
+// outside the footprint the result underflows to 0 and fails the alpha test.
+__device__ __forceinline__ float exp_half(float q) {
   float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(q * (-0.5f * 1.4426950408889634f)));
   return y;
 }
 
@@ -593,15 +625,75 @@ __device__ __forceinline__ void stage_batch(const Rec* __restrict__ recs, const 
   }
 }
 
+// Composites the staged pairs of mask m (bit i: record sr[i], whose sorted offset
+// in the tile is off + i) into PPT pixels of column fx, rows fy .. fy + PPT - 1,
+// front to back, until all of them are done (dn).  Each pixel evaluates the
+// exponential of every pair whether it contributes or not: skipping it saved
+// 7 instructions of 24 where a whole warp skipped, and cost a divergent
+// branch and its reconvergence on every pair (forward 574 -> 487 us at 200k
+// Gaussians, 8 views of 800 x 800).  One pixel per thread serves small grids, which
+// are bound by the latency of that chain: four pairs at a time are evaluated
+// before they are composited (36 -> 22 us at 16 tiles).
+template <int PPT>
+__device__ __forceinline__ void fwd_pairs(const Rec* __restrict__ sr, uint32_t m, uint32_t off, float fx, float fy,
+                                          float (&T)[PPT], float (&C0)[PPT], float (&C1)[PPT], float (&C2)[PPT],
+                                          uint32_t (&last)[PPT], bool (&dn)[PPT]) {
+  constexpr int U = PPT == 1 ? 4 : 1;
+  auto all_done = [&] {
+    bool d = true;
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) d = d && dn[k];
+    return d;
+  };
+  for (bool done = all_done(); m != 0u && !done; done = all_done()) {
+    uint32_t j[U];
+    float alpha[U][PPT];
+    bool ok[U][PPT];
+    float3 col[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool have = U == 1 || m != 0u;
+      j[u] = have ? __ffs(m) - 1 : 0;
+      m &= m - 1u;
+      const float4 a = sr[j[u]].a, b = sr[j[u]].b;
+      col[u] = make_float3(b.z, b.w, sr[j[u]].c.x);
+      const float dx = a.x - fx;
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) {
+        float cu, cw;
+        const float q = gs_quad(a, b.x, dx, a.y - (fy + (float)k), cu, cw);
+        alpha[u][k] = fminf(kAlphaMax, b.y * exp_half(q));
+        ok[u][k] = have && !(q < 0.0f || alpha[u][k] < kAlphaMin);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) {
+        const float test_T = T[k] * (1.0f - alpha[u][k]);
+        const float w = alpha[u][k] * T[k];
+        const bool act = ok[u][k] && !dn[k], stop = test_T < kTMin;
+        dn[k] = dn[k] || (act && stop);
+        if (act && !stop) {
+          C0[k] += col[u].x * w;
+          C1[k] += col[u].y * w;
+          C2[k] += col[u].z * w;
+          T[k] = test_T;
+          last[k] = off + j[u] + 1;
+        }
+      }
+  }
+}
+
 // Forward raster, PPT vertically adjacent pixels per thread: 256 / PPT
 // threads per 16 x 16 tile, a warp covers a 16 x 2·PPT strip, records staged
 // SB = SPS · 256 / PPT at a time.  (PPT, SB) is the autotuned variant.
 // kOrd: a 1D grid whose block b takes work item order[b] (longest tile
-// lists first), else the grid is (tiles x, tiles y, views).  With 1 or 2
-// pixels per thread at most 51 registers: ten 128-thread blocks per SM (the
-// shared-memory limit) instead of nine.
+// lists first), else the grid is (tiles x, tiles y, views).  Registers: 64 for
+// 1 pixel per thread, 56 for 2 (nine 128-thread blocks per SM; ten spill, eight
+// give 493 us where nine give 487).
 template <int PPT, int SPS, bool kOrd>
-__global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1280 / (256 / PPT) : 1) k_fwd(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 4 : PPT == 2 ? 9 : 1) k_fwd(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
                                                    const uint32_t* __restrict__ rstart,
                                                    const uint32_t* __restrict__ rend, uint32_t W, uint32_t H,
                                                    uint32_t tiles_x, uint32_t num_tiles, float3 bg,
@@ -672,41 +764,10 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1280 / (256 / PPT) : 1) 
       if (jj < nb) h = !rec_misses_box(sr[jj].a, sr[jj].b.x, sr[jj].c, wx0, wy0, ww, wh);
       hit[qq] = __ballot_sync(0xffffffffu, h);
     }
-    bool done;
-    NPS_ALL_DONE(done);
 #pragma unroll
     for (int qq = 0; qq < SB / 32; ++qq)
-    for (uint32_t m = hit[qq]; m != 0u && !done;) {
-      const int bit = __ffs(m) - 1;
-      m &= m - 1u;
-      const uint32_t j = qq * 32 + bit;
-      const float4 a = sr[j].a;
-      const float4 c4 = sr[j].c;
-      const float4 b = sr[j].b;
-      const float dx = a.x - fx, pmin = -0.5f * c4.y;
-#pragma unroll
-      for (int k = 0; k < PPT; ++k) {
-        if (dn[k]) continue;
-        const float dy = a.y - (float)(py + k);
-        float cu, cw;
-        const float power = gs_power(a, b.x, dx, dy, cu, cw);
-        if (power > 0.0f || power < pmin) continue;  // pmin: alpha < 1/255 below it (see pix_bwd_pair)
-        const float alpha = fminf(kAlphaMax, b.y * exp_raster(power));
-        if (alpha < kAlphaMin) continue;
-        const float test_T = T[k] * (1.0f - alpha);
-        if (test_T < kTMin) {
-          dn[k] = true;
-          continue;
-        }
-        const float w = alpha * T[k];
-        C0[k] += b.z * w;
-        C1[k] += b.w * w;
-        C2[k] += c4.x * w;
-        T[k] = test_T;
-        last[k] = base - start + j + 1;
-      }
-      NPS_ALL_DONE(done);
-    }
+      fwd_pairs<PPT>(sr + qq * 32, hit[qq], base - start + qq * 32, fx, (float)py, T, C0, C1, C2, last, dn);
+    bool done;
     // every pixel of the tile done: stop (after the prefetch in flight lands)
     NPS_ALL_DONE(done);
     if (__syncthreads_count(done) == NT || s_abort) {
@@ -1127,9 +1188,9 @@ __global__ void __launch_bounds__(kThreads) k_bwd(const Rec* __restrict__ recs, 
     const float col[3] = {b.z, b.w, c4.x};
     const float dx = a.x - fx, dy = a.y - fy;
     float u, w;
-    const float power = gs_power(a, b.x, dx, dy, u, w);
-    if (power > 0.0f) return false;
-    const float G = exp_raster(power);
+    const float q = gs_quad(a, b.x, dx, dy, u, w);
+    if (q < 0.0f) return false;
+    const float G = exp_half(q);
     const float araw = b.y * G;
     const float alpha = fminf(kAlphaMax, araw);
     if (alpha < kAlphaMin) return false;
@@ -1271,66 +1332,99 @@ __device__ __forceinline__ void pix_bwd_init(PixBwd& s, uint32_t px, uint32_t py
   s.last_alpha = s.acc_dot = s.last_dot = 0.0f;
 }
 
-// Scale of gradient term k that pix_bwd_pair leaves out of its per-pixel sums
+// Scale of gradient term k that pix_bwd_apply leaves out of its per-pixel sums
 // (applied once to the warp total): terms 0..4 are accumulated with their
 // common factor -1 and terms 2 and 4 with twice their value.
 __device__ __forceinline__ float bwd_term_scale(uint32_t k) {
   return k < 5u ? ((k == 2u || k == 4u) ? -0.5f : -1.0f) : 1.0f;
 }
 
-// adds this pixel's gradient w.r.t. the pair (a, b, c4) at sorted offset cur
-// to gv[0..8] (terms 0..4 without their bwd_term_scale); returns whether the
-// pair contributes here
-__device__ __forceinline__ bool pix_bwd_pair(PixBwd& s, const float4& a, const float4& b, const float4& c4,
-                                             uint32_t cur, float* gv) {
-  if (cur >= s.last) return false;
-  const float dx = a.x - s.fx, dy = a.y - s.fy;
-  float u, w;
-  const float power = gs_power(a, b.x, dx, dy, u, w);
-  // power < -c4.y / 2 (outside the alpha >= 1/255 ellipse with its margin)
-  // implies alpha < 1/255, so skipping those pixels before the exponential
-  // leaves every decision of the alpha test below unchanged
-  if (power > 0.0f || power < -0.5f * c4.y) return false;
-  const float G = exp_raster(power);
-  const float araw = b.y * G;
-  const float alpha = fminf(kAlphaMax, araw);
-  if (alpha < kAlphaMin) return false;
+// What a pair (a, b) at sorted offset cur is to a pixel, before its replay state
+// is advanced: the same instructions whether the pair contributes (ok) or not, so
+// that several pixels' or pairs' exponentials and reciprocals are in flight at
+// once.  Skipping the rest for pixels outside the ellipse instead put a branch and
+// its reconvergence between them (backward 1195 -> 1015 us at 200k Gaussians, 8 views
+// of 800 x 800).
+struct PairAt {
+  float dx, dy, u, w, G, araw, alpha, inv1ma;
+  bool ok;
+};
+__device__ __forceinline__ PairAt pix_bwd_prep(const PixBwd& s, const float4& a, const float4& b, uint32_t cur) {
+  PairAt r;
+  r.dx = a.x - s.fx;
+  r.dy = a.y - s.fy;
+  const float q = gs_quad(a, b.x, r.dx, r.dy, r.u, r.w);
+  r.G = exp_half(q);
+  r.araw = b.y * r.G;
+  r.alpha = fminf(kAlphaMax, r.araw);
   // one reciprocal serves both divisions (approximate, ~2 ulp; alpha <= 0.99)
-  const float inv1ma = rcp_normal(1.0f - alpha);
-  s.T = s.T * inv1ma;
-  const float wgt = alpha * s.T;
+  r.inv1ma = rcp_normal(1.0f - r.alpha);
+  r.ok = !(cur >= s.last || q < 0.0f || r.alpha < kAlphaMin);
+  return r;
+}
+
+// advances the replay state past a contributing pair of colour (b.z, b.w, cx) and
+// adds this pixel's gradient with respect to it to gv[0..8] (terms 0..4 without
+// their bwd_term_scale)
+__device__ __forceinline__ void pix_bwd_apply(PixBwd& s, const PairAt& r, const float4& b, float cx, float (&gv)[9]) {
+  if (!r.ok) return;
+  s.T = s.T * r.inv1ma;
+  const float wgt = r.alpha * s.T;
   // colour behind this pair, dotted with dL/dpixel: last_alpha * last + (1 - last_alpha) * acc
-  const float cdot = fmaf(c4.x, s.dC[2], fmaf(b.w, s.dC[1], b.z * s.dC[0]));
+  const float cdot = fmaf(cx, s.dC[2], fmaf(b.w, s.dC[1], b.z * s.dC[0]));
   s.acc_dot = fmaf(s.last_alpha, s.last_dot - s.acc_dot, s.acc_dot);
   s.last_dot = cdot;
-  s.last_alpha = alpha;
-  const float dL_dalpha = fmaf(s.nbg, inv1ma, (cdot - s.acc_dot) * s.T);
+  s.last_alpha = r.alpha;
+  const float dL_dalpha = fmaf(s.nbg, r.inv1ma, (cdot - s.acc_dot) * s.T);
 #pragma unroll
   for (int c = 0; c < 3; ++c) gv[6 + c] = fmaf(wgt, s.dC[c], gv[6 + c]);
-  if (araw <= kAlphaMax) {
+  if (r.araw <= kAlphaMax) {
     // dL/dG = opacity dL/dalpha; h = G dL/dG
-    const float h = araw * dL_dalpha, hx = h * dx, hy = h * dy;
-    gv[0] = fmaf(h, u, gv[0]);     // d/du:  -h u
-    gv[1] = fmaf(h, w, gv[1]);     // d/dv:  -h w
-    gv[2] = fmaf(hx, dx, gv[2]);   // d/d conic a: -h dx dx / 2
-    gv[3] = fmaf(hx, dy, gv[3]);   // d/d conic b: -h dx dy
-    gv[4] = fmaf(hy, dy, gv[4]);   // d/d conic c: -h dy dy / 2
-    gv[5] = fmaf(G, dL_dalpha, gv[5]);  // d/d opacity
+    const float h = r.araw * dL_dalpha, hx = h * r.dx, hy = h * r.dy;
+    gv[0] = fmaf(h, r.u, gv[0]);          // d/du:  -h u
+    gv[1] = fmaf(h, r.w, gv[1]);          // d/dv:  -h w
+    gv[2] = fmaf(hx, r.dx, gv[2]);        // d/d conic a: -h dx dx / 2
+    gv[3] = fmaf(hx, r.dy, gv[3]);        // d/d conic b: -h dx dy
+    gv[4] = fmaf(hy, r.dy, gv[4]);        // d/d conic c: -h dy dy / 2
+    gv[5] = fmaf(r.G, dL_dalpha, gv[5]);  // d/d opacity
   }
-  return true;
+}
+
+// gv: the gradient of PPT pixels with respect to the pair; returns whether it
+// contributes to any of them
+template <int PPT>
+__device__ __forceinline__ bool pixels_bwd(PixBwd (&p)[PPT], const Rec& rec, uint32_t cur, float (&gv)[9]) {
+  const float4 a = rec.a, b = rec.b;
+  const float cx = rec.c.x;
+  PairAt r[PPT];
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) r[k] = pix_bwd_prep(p[k], a, b, cur);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) gv[k] = 0.0f;
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    pix_bwd_apply(p[k], r[k], b, cx, gv);
+    any |= r[k].ok;
+  }
+  return any;
 }
 
 // Backward raster, PPT vertically adjacent pixels per thread (256 / PPT
-// threads per 16 x 16 tile, a warp covers a 16 x 2·PPT strip): one warp
-// reduction serves 32·PPT pixels.  The warp first ballots the staged pairs
-// that meet its strip and that some of its pixels reached, then walks them in
-// reverse order.  Per-pair sums go to shared memory and then to the (view,
-// Gaussian) records with global atomics.  PPT is the autotuned variant.
-// With 1 or 2 pixels per thread at most 64 registers (1024 / (256 / PPT) blocks of 256 / PPT threads,
-// 32 warps per SM): eight 128-thread blocks per SM instead of six cut the backward by 8% at the
-// benchmark workload.  4 pixels per thread would spill under that bound and keep their registers.
+// threads per 16 x 16 tile): one warp reduction serves 32·PPT pixels.  The warp
+// first ballots the staged pairs that meet its strip and that some of its pixels
+// reached, then walks them in reverse order and adds each pair's warp totals to
+// the (view, Gaussian) record with one coalesced instruction of global
+// additions: nothing waits for them, where sums kept per block cost a
+// compare-and-swap loop in shared memory per warp and pair and a scattered flush
+// per batch (1240 -> 1195 us at 200k Gaussians, 8 views of 800 x 800).  PPT is the
+// autotuned variant.  Issue-bound at 2 pixels per thread (77% of the issue slots):
+// 72 registers, seven 128-thread blocks per SM (eight give 1020 us where seven give
+// 965).  One pixel per thread serves small grids, which are bound by the latency of
+// the chain from pair to pair: two pairs are evaluated and reduced together
+// (65 -> 43 us at 16 tiles, with 80 registers).
 template <int PPT, int SPS, bool kOrd>
-__global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) k_bwd2(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_bwd2(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
                                                     const uint32_t* __restrict__ rstart,
                                                     const uint32_t* __restrict__ rend, uint32_t W, uint32_t H,
                                                     uint32_t tiles_x, uint32_t num_tiles, float3 bg,
@@ -1342,8 +1436,8 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) 
   constexpr int NT = 256 / PPT, SB = NT * SPS;
   static_assert(SB <= 256, "staging buffers beyond the static shared-memory budget");
   __shared__ __align__(16) Rec s_rec[2][SB];
-  __shared__ uint32_t s_g[3][SB];
-  __shared__ float s_acc[2][SB][9];
+  __shared__ uint32_t s_g[2][SB];
+  __shared__ __align__(16) float s_red[PPT == 1 ? 1 : NT / 32][9 * kRedStride];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ uint32_t s_max;
   uint32_t tx = blockIdx.x, ty = blockIdx.y, v = blockIdx.z;
@@ -1378,7 +1472,6 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) 
     mbar_init(&s_bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  for (uint32_t r = tid; r < (uint32_t)(2 * SB * 9); r += NT) (&s_acc[0][0][0])[r] = 0.0f;
   __syncthreads();
   atomicMax(&s_max, mylast);
   __syncthreads();
@@ -1396,25 +1489,19 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) 
     const uint32_t b0 = bstart_of(0);
     stage_batch(recs, vals, b0, start + maxlast - b0, s_rec[0], &s_bar[0], s_g[0]);
   }
-  // One CTA barrier per batch: batch bi accumulates into s_acc[bi & 1]; after
-  // the barrier each thread flushes and clears its rows of that buffer while
-  // others may already walk batch bi + 1 into the other one.  The barrier also
-  // orders the re-staging of s_rec[bi & 1] (issued at batch bi + 1, after the
-  // barrier of batch bi) after every read of it, and the record ids rotate
-  // through three buffers so that staging batch bi + 2 never overwrites the
-  // ids the flush of batch bi is still reading.
-  uint32_t gb = 0;  // bi % 3
+  // One CTA barrier per batch: it orders the re-staging of s_rec[bi & 1] (issued at
+  // batch bi + 1, after the barrier of batch bi) after every read of it.
   for (uint32_t bi = 0; bi < nbatch; ++bi) {
-    const uint32_t buf = bi & 1u, gnext = gb == 2u ? 0u : gb + 1u;
+    const uint32_t buf = bi & 1u;
     const uint32_t bend = start + maxlast - bi * SB, bstart = bstart_of(bi);
     const uint32_t nb = bend - bstart;
     if (bi + 1 < nbatch) {
       const uint32_t nbs = bstart_of(bi + 1);
-      stage_batch(recs, vals, nbs, bstart - nbs, s_rec[buf ^ 1u], &s_bar[buf ^ 1u], s_g[gnext]);
+      stage_batch(recs, vals, nbs, bstart - nbs, s_rec[buf ^ 1u], &s_bar[buf ^ 1u], s_g[buf ^ 1u]);
     }
     if (!mbar_wait(&s_bar[buf], (bi >> 1) & 1u)) s_abort = 1u;  // the batch is undefined: end the tile below
     const Rec* sr = s_rec[buf];
-    float(*acc)[9] = s_acc[buf];
+    const uint32_t* sg = s_g[buf];
     uint32_t hit[SB / 32];
 #pragma unroll
     for (int qq = 0; qq < SB / 32; ++qq) {
@@ -1426,36 +1513,37 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) 
     }
 #pragma unroll
     for (int qq = SB / 32 - 1; qq >= 0; --qq)
-    for (uint32_t m = hit[qq]; m != 0u;) {
-      const int bit = 31 - __clz(m);
-      m &= ~(1u << bit);
-      const int j = qq * 32 + bit;  // descending within the batch
-      const float4 a = sr[j].a;
-      const float4 c4 = sr[j].c;
-      const float4 b = sr[j].b;
-      const uint32_t cur = bstart + (uint32_t)j - start;
-      float gv[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) gv[k] = 0.0f;
-      bool any = false;
-#pragma unroll
-      for (int k = 0; k < PPT; ++k) any |= pix_bwd_pair(p[k], a, b, c4, cur, gv);
-      const uint32_t cm = __ballot_sync(0xffffffffu, any);
-#if NPS_GS_SOLO
-      if (cm != 0u && (cm & (cm - 1u)) == 0u) {
-        // one contributing lane: its values are the warp totals
-        if (any) {
-#pragma unroll
-          for (int k = 0; k < 9; ++k) atomicAdd(&acc[j][k], gv[k] * bwd_term_scale((uint32_t)k));
+      for (uint32_t m = hit[qq]; m != 0u;) {  // descending within the batch
+        const int bit = 31 - __clz(m), j = qq * 32 + bit;
+        m &= ~(1u << bit);
+        const uint32_t cur = bstart + (uint32_t)j - start;
+        if constexpr (PPT == 1) {
+          const bool two = m != 0u;
+          const int bit2 = two ? 31 - __clz(m) : bit, j2 = qq * 32 + bit2;
+          m &= ~(1u << bit2);
+          const float4 b1 = sr[j].b, b2 = sr[j2].b;
+          const PairAt r1 = pix_bwd_prep(p[0], sr[j].a, b1, cur);
+          const PairAt r2 = pix_bwd_prep(p[0], sr[j2].a, b2, two ? bstart + (uint32_t)j2 - start : 0xffffffffu);
+          float g1[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, g2v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+          pix_bwd_apply(p[0], r1, b1, sr[j].c.x, g1);
+          pix_bwd_apply(p[0], r2, b2, sr[j2].c.x, g2v);
+          if (__any_sync(0xffffffffu, r1.ok || r2.ok)) {
+            const float tot = warp_sum9x2(g1, g2v, lane);
+            const uint32_t k = warp_sum9x2_index(lane);
+            const bool second = lane & 8u;
+            if (k < 9 && (two || !second))
+              atomicAdd(g2 + (size_t)sg[second ? j2 : j] * kG2 + k, tot * bwd_term_scale(k));
+          }
+        } else {
+          float gv[9];
+          const bool any = pixels_bwd<PPT>(p, sr[j], cur, gv);
+          if (__any_sync(0xffffffffu, any)) {
+            const float tot = warp_total9(gv, lane, s_red[tid >> 5]);
+            const uint32_t k = lane >> 1;
+            if ((lane & 1) == 0 && k < 9) atomicAdd(g2 + (size_t)sg[j] * kG2 + k, tot * bwd_term_scale(k));
+          }
         }
-      } else
-#endif
-      if (cm != 0u) {
-        const float tot = warp_sum9(gv, lane);
-        const uint32_t k = warp_sum9_index(lane);
-        if ((lane & 1) == 0 && k < 9) atomicAdd(&acc[j][k], tot * bwd_term_scale(k));
       }
-    }
     __syncthreads();
     if (s_abort) {
       // a bounded wait gave up: no further sums leave the tile (the step reports NPS_ERR_TIMEOUT); the
@@ -1467,18 +1555,6 @@ __global__ void __launch_bounds__(256 / PPT, PPT <= 2 ? 1024 / (256 / PPT) : 1) 
       }
       return;
     }
-    for (uint32_t r = tid; r < nb; r += NT) {
-      float* dst = g2 + (size_t)s_g[gb][r] * kG2;
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const float x = acc[r][k];
-        if (x != 0.0f) {
-          atomicAdd(dst + k, x);
-          acc[r][k] = 0.0f;
-        }
-      }
-    }
-    gb = gnext;
   }
 }
 
@@ -2023,6 +2099,7 @@ struct nps_gs {
   int fwd_ppt = 1, bwd_ppt = 2, fwd_stage = 256, bwd_stage = 128;
   // raster form: 0 = one CTA per (tile, view), 1 = persistent warp-specialised kernel over a work queue
   int fwd_form = 0, bwd_form = 0;
+  bool raster_auto = true;  // no variant was chosen: the pixels per thread follow the grid's size (default_variant)
   uint32_t tile = 16;  // tile edge in pixels (8, 16, 32); form 0 and the deterministic backward need 16
   DevBuf tile_last, ws_order_f, ws_order_b, ws_q;  // per-item last contributor, work queues, queue control
   DevBuf det_part, det_keys, det_pos;
@@ -2496,6 +2573,26 @@ constexpr int kNumTiles = 3;
 // per tile in the autotuner's times: binning, then the forward and backward time of each variant
 constexpr int kTuneStride = 1 + 2 * kNumVariants;
 
+// Form 0's variant for a grid of nitems tiles while none was chosen.  A grid of few
+// tiles is bound by the latency of the chain from pair to pair and by how many warps
+// are resident, and 1 pixel per thread has the shorter chain and twice the warps;
+// a grid that fills the device several times over is bound by issue, where 2 pixels
+// per thread share a pair's loads and its reduction.  Forward / backward in us at
+// (1, 256) and at (2, 128), one view: 16 tiles 22 / 43 and 32 / 70; 256 tiles 39 / 64
+// and 50 / 101; 784 tiles 46 / 85 and 45 / 92; 1024 tiles 48 / 101 and 51 / 101; 1936
+// tiles 71 / 151 and 73 / 123; 2500 tiles 83 / 171 and 79 / 146; 6084 tiles 157 / 333
+// and 132 / 241.
+static RasterVariant default_variant(const nps_gs* o, bool bwd, uint32_t nitems) {
+  const uint32_t per_sm = bwd ? 6 : 12;
+  return nitems <= per_sm * (uint32_t)o->ctx->sm_count ? RasterVariant{0, 1, 256} : RasterVariant{0, 2, 128};
+}
+static RasterVariant raster_variant(const nps_gs* o, bool bwd) {
+  if (o->raster_auto && o->tile == 16)
+    return default_variant(o, bwd, div_up(o->w, 16u) * div_up(o->h, 16u) * o->nv);
+  return bwd ? RasterVariant{o->bwd_form, o->bwd_ppt, o->bwd_stage}
+             : RasterVariant{o->fwd_form, o->fwd_ppt, o->fwd_stage};
+}
+
 // Resident CTAs of a persistent kernel on the device (queried once per kernel).
 template <class K>
 static int persistent_grid(nps_gs* o, K kernel, int threads, int* cache) {
@@ -2802,7 +2899,8 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     o->sorted_vals = vs;
     if (M == 0 || cap > 0) {
       StageTimer t_fwd(o, ST_FWD);
-      NPS_TRY(launch_fwd_raster(o, o->fwd_form, o->fwd_ppt, o->fwd_stage, cleared));
+      const RasterVariant va = raster_variant(o, false);
+      NPS_TRY(launch_fwd_raster(o, va.form, va.ppt, va.stage, cleared));
       NPS_CHECK_LAUNCH();
     }
     if (capture || M == 0) break;
@@ -2915,7 +3013,8 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
   const float4* dimg = dl_dimg ? (const float4*)dl_dimg : o->dimg.as<float4>();
   if (!o->deterministic) {
     StageTimer t(o, ST_BWD);
-    NPS_TRY(launch_bwd_raster(o, o->bwd_form, o->bwd_ppt, o->bwd_stage, dimg));
+    const RasterVariant va = raster_variant(o, true);
+    NPS_TRY(launch_bwd_raster(o, va.form, va.ppt, va.stage, dimg));
     NPS_CHECK_LAUNCH();
   } else if (o->pair_cap > 0) {
     if (o->tile != 16) {
@@ -3497,6 +3596,7 @@ int nps_gs_set_raster(nps_gs* o, int fwd_form, int fwd_ppt, int fwd_stage, int b
               fwd_form, fwd_ppt, fwd_stage, bwd_form, bwd_ppt, bwd_stage, o->tile, o->tile);
     return NPS_ERR_INVALID;
   }
+  o->raster_auto = false;
   o->fwd_form = fwd_form;
   o->fwd_ppt = fwd_ppt;
   o->fwd_stage = fwd_stage;
@@ -3522,6 +3622,7 @@ int nps_gs_set_tile(nps_gs* o, uint32_t tile) {
     return NPS_ERR_STATE;
   }
   o->tile = tile;
+  if (tile != 16) o->raster_auto = false;
   // keep the raster variants if they serve the new tile, else its default persistent ones
   const RasterVariant def = tile == 8 ? RasterVariant{1, 1, 128} : tile == 32 ? RasterVariant{1, 4, 128}
                                                                               : RasterVariant{1, 2, 128};
@@ -3613,6 +3714,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
             valid_variant((uint32_t)a[0], a[4], a[5], a[6])) {
           found = true;
           o->tile = (uint32_t)a[0];
+          o->raster_auto = false;
           o->fwd_form = a[1], o->fwd_ppt = a[2], o->fwd_stage = a[3];
           o->bwd_form = a[4], o->bwd_ppt = a[5], o->bwd_stage = a[6];
         }
@@ -3634,6 +3736,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
   NPS_CUDA(cudaEventCreate(&e1));
   float best_total = 1e30f;
   uint32_t best_tile = o->tile;
+  o->raster_auto = false;
   RasterVariant best_pick[2] = {{o->fwd_form, o->fwd_ppt, o->fwd_stage}, {o->bwd_form, o->bwd_ppt, o->bwd_stage}};
   constexpr int kReps = 3;
   int rc = NPS_OK;

@@ -289,42 +289,9 @@ __global__ void __launch_bounds__(TS * TS / PPT + 32) k_fwd_ws(
         if (jj < m.nb) h = !rec_misses_box(sr[jj].a, sr[jj].b.x, sr[jj].c, wx0, wy0, TL::kStripW, TL::kStripH);
         hit[qq] = __ballot_sync(0xffffffffu, h);
       }
-      bool done = mine;
 #pragma unroll
       for (int qq = 0; qq < SB / 32; ++qq)
-        for (uint32_t mk = hit[qq]; mk != 0u && !done;) {
-          const int bit = __ffs(mk) - 1;
-          mk &= mk - 1u;
-          const uint32_t j = qq * 32 + bit;
-          const float4 a = sr[j].a;
-          const float4 c4 = sr[j].c;
-          const float4 b = sr[j].b;
-          const float dx = a.x - fx, pmin = -0.5f * c4.y;
-#pragma unroll
-          for (int k = 0; k < PPT; ++k) {
-            if (dn[k]) continue;
-            const float dy = a.y - (float)(py + k);
-            float cu, cw;
-            const float power = gs_power(a, b.x, dx, dy, cu, cw);
-            if (power > 0.0f || power < pmin) continue;  // alpha < 1/255 below pmin
-            const float alpha = fminf(kAlphaMax, b.y * exp_raster(power));
-            if (alpha < kAlphaMin) continue;
-            const float test_T = T[k] * (1.0f - alpha);
-            if (test_T < kTMin) {
-              dn[k] = true;
-              continue;
-            }
-            const float w = alpha * T[k];
-            C0[k] += b.z * w;
-            C1[k] += b.w * w;
-            C2[k] += c4.x * w;
-            T[k] = test_T;
-            last[k] = m.off + j + 1;
-          }
-          done = true;
-#pragma unroll
-          for (int k = 0; k < PPT; ++k) done = done && dn[k];
-        }
+        fwd_pairs<PPT>(sr + qq * 32, hit[qq], m.off + qq * 32, fx, (float)py, T, C0, C1, C2, last, dn);
     }
     if (!reported) {
       bool all = true;
@@ -356,7 +323,7 @@ __global__ void __launch_bounds__(TS * TS / PPT + 32) k_fwd_ws(
 
 // ------------------------------------------------------------ backward
 template <int TS, int PPT, int SB>
-__global__ void __launch_bounds__(TS * TS / PPT + 32) k_bwd_ws(
+__global__ void __launch_bounds__(TS * TS / PPT + 32, TS == 32 ? 2 : 1) k_bwd_ws(
     const Rec* __restrict__ recs, const uint32_t* __restrict__ vals, const uint32_t* __restrict__ rstart,
     const uint32_t* __restrict__ tile_last, const uint32_t* __restrict__ order, uint32_t* __restrict__ qctl,
     uint32_t W, uint32_t H, uint32_t tiles_x, uint32_t num_tiles, float3 bg, const float4* __restrict__ img,
@@ -368,6 +335,7 @@ __global__ void __launch_bounds__(TS * TS / PPT + 32) k_bwd_ws(
   __shared__ __align__(16) Rec s_rec[S][SB];
   __shared__ uint32_t s_g[S][SB];
   __shared__ float s_acc[S][SB][9];
+  __shared__ __align__(16) float s_red[NW][9 * kRedStride];
   __shared__ __align__(8) uint64_t s_full[S];
   __shared__ __align__(8) uint64_t s_empty[S];
   __shared__ WsMeta s_meta[S];
@@ -477,19 +445,11 @@ __global__ void __launch_bounds__(TS * TS / PPT + 32) k_bwd_ws(
           const int bit = 31 - __clz(mk);
           mk &= ~(1u << bit);
           const int j = qq * 32 + bit;  // descending within the batch
-          const float4 a = sr[j].a;
-          const float4 c4 = sr[j].c;
-          const float4 b = sr[j].b;
-          const uint32_t cur = m.off + (uint32_t)j;
           float gv[9];
-#pragma unroll
-for (int k = 0; k < 9; ++k) gv[k] = 0.0f;
-          bool any = false;
-#pragma unroll
-          for (int k = 0; k < PPT; ++k) any |= pix_bwd_pair(p[k], a, b, c4, cur, gv);
+          const bool any = pixels_bwd<PPT>(p, sr[j], m.off + (uint32_t)j, gv);
           if (__any_sync(0xffffffffu, any)) {
-            const float tot = warp_sum9(gv, lane);
-            const uint32_t k = warp_sum9_index(lane);
+            const float tot = warp_total9(gv, lane, s_red[warp]);
+            const uint32_t k = lane >> 1;
             if ((lane & 1) == 0 && k < 9) atomicAdd(&acc[j][k], tot * bwd_term_scale(k));
           }
         }

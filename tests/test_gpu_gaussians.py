@@ -325,6 +325,32 @@ def test_deterministic_mode_is_bit_reproducible(trainer_cls, tmp_path):
     np.testing.assert_array_equal(r.read_state()["adam_v"], runs[0].read_state()["adam_v"])
 
 
+@pytest.mark.parametrize("w,h,views", [(64, 50, 1), (640, 400, 1), (400, 320, 4), (800, 639, 1)])
+def test_default_raster_follows_the_grid_size(trainer_cls, w, h, views):
+    """Without a chosen variant a pass takes 1 pixel per thread on a grid of
+    few tiles and 2 on one of many (16, 1000, 2000 and 2000 tiles: below, between
+    and above the lines of the two passes): the same images and gradients as a
+    chosen variant with 4, to the bounds of the variants among themselves (1e-6
+    per value, 1e-5 relative L2)."""
+    p = gs_scene(1500, 71, deg=1, log_scale_mean=-3.2)
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0), (-2.0, 0.5, 3.0), (0.5, -2.0, 3.5))[:views])
+    t = trainer_cls(1500, sh_degree=1, params=p)
+    t.set_targets(gs_targets(views, w, h, 72))
+    out = []
+    for chosen in (False, True):
+        if chosen:
+            t.set_raster((0, 4, 64), (0, 4, 64))
+        else:
+            assert t.raster() == dict(tile=16, fwd=(0, 1, 256), bwd=(0, 2, 128))
+        t.set_views(vp, vpi)
+        t.forward()
+        t.loss()
+        t.backward()
+        out.append((t.read_image(with_grad=False)[0], t.read_state()["grads"].astype(np.float64)))
+    np.testing.assert_allclose(out[0][0], out[1][0], atol=1e-6, rtol=0)
+    assert np.linalg.norm(out[0][1] - out[1][1]) / np.linalg.norm(out[1][1]) < 1e-5
+
+
 def test_raster_variants_agree_and_autotune(trainer_cls, tmp_path):
     """Forward images agree across tile sizes (8, 16, 32) and the raster
     variants of both forms (one CTA per tile; persistent warp-specialised)
