@@ -17,7 +17,7 @@
 //                  (block-wide vote ends the tile), final T and last
 //                  contributor stored per pixel (O(pixels) state, no
 //                  per-pair state)
-//   k_ssim_fwd2 / k_ssim_bwd2 / k_loss_reduce: (1 - l) L1 + l (1 - SSIM), 11x11
+//   k_ssim_fwd / k_ssim_bwd / k_loss_reduce: (1 - l) L1 + l (1 - SSIM), 11x11
 //                  Gaussian window (sigma 1.5), l = 0.2, and dL/dimage
 //   k_bwd2         reverse traversal replaying transmittance from the final
 //                  T, two pixels per thread, per-Gaussian gradients summed
@@ -56,6 +56,10 @@ constexpr int kSsimWin = 11;
 constexpr float kSsimC1 = 0.01f * 0.01f, kSsimC2 = 0.03f * 0.03f;
 
 __constant__ float c_ssim_w[kSsimWin];
+// 1, which the compiler cannot see: a packed product added to a sum becomes one
+// fused operation whatever the rounding modifiers, and multiplying the rounded product by
+// this keeps the two roundings that the means are defined with
+__constant__ float c_ssim_one = 1.0f;
 
 // 1 / x on the special-function unit for x well inside the normal range
 // (__fdividef(1, x)'s bits without its scaling for extreme x)
@@ -801,243 +805,272 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 4 : PPT == 2 ? 9 : 1) k_
 
 // ------------------------------------------------------------ loss
 // (1 - l) * mean|x - y| + l * (1 - mean SSIM), averaged over views.
-// k_ssim_fwd2 writes, per pixel and channel, the three maps whose Gaussian
+// k_ssim_fwd writes, per pixel and channel, the three maps whose Gaussian
 // correlation gives dL/dx, plus per-block partial sums of |x - y| and SSIM;
-// k_ssim_bwd2 correlates the maps and adds the L1 term.
+// k_ssim_bwd correlates the maps and adds the L1 term.  Zero padding outside the
+// image.
 //
-// 32 x 32 output tiles (input span 42 x 42), zero padding outside the image,
-// register-blocked separable window: the horizontal pass runs 4 consecutive
-// outputs of a row from 14 inputs held in registers, the vertical pass 4
-// consecutive rows of a column.  The gradient maps are planar (V x 9 x H x W)
-// so the backward's halo loads are coalesced.
+// A warp takes one channel of a strip 32 columns wide and walks down its rows,
+// with no block barrier: it stages a row (and five columns on either side) in its
+// own row of shared memory, loading the next one meanwhile, sums the window
+// along the row, one column per lane, and keeps the sums of the last eleven rows in
+// registers, where the sum down the columns reads them (the loop is unrolled by
+// eleven, so that every register index is fixed).  Tiles that put the row sums through
+// shared memory instead read seventeen words per output for the second pass
+// and recompute 31% of the first one (both kernels 348 -> 321 us at 8 views of 800 x 800, 1084 -> 895
+// at 8 views of 1920 x 1080).  Values that share a weight (x and y, xx and yy) are added
+// in packed pairs (forward 203 us without).  The forward is bound by issue and the FMA
+// pipe, the backward by shared-memory bandwidth and issue.
 constexpr int kHalo = kSsimWin / 2;
-constexpr int kLT = 32, kLI = kLT + 2 * kHalo, kLS = kLI + 1;  // 32, 42, row stride 43
-constexpr int kHS = kLT + 1;                                    // row stride of the horizontal sums
-constexpr size_t kSsimFwdSmem = sizeof(float) * (2 * 3 * kLI * kLS + 5 * kLI * kHS);
-constexpr size_t kSsimBwdSmem = sizeof(float) * (3 * kLI * kLS + 3 * kLI * kHS);
+constexpr int kSsimCols = 32, kSsimRow = kSsimCols + 2 * kHalo;  // outputs of a row, staged columns
 
-__global__ void __launch_bounds__(256) k_ssim_fwd2(const float4* __restrict__ img, const float4* __restrict__ tgt,
-                                                   const uint32_t* __restrict__ tgt_ids, uint32_t W, uint32_t H,
-                                                   float lambda, float inv_norm, float* __restrict__ maps,
-                                                   float* __restrict__ partial) {
-  extern __shared__ float sm[];
-  float* sx = sm;                        // [3][kLI][kLS]
-  float* sy = sx + 3 * kLI * kLS;        // [3][kLI][kLS]
-  float* hm = sy + 3 * kLI * kLS;        // [5][kLI][kHS]
-  __shared__ float red[2][8];
-  const uint32_t v = blockIdx.z, tid = threadIdx.x;
-  const int ox = blockIdx.x * kLT - kHalo, oy = blockIdx.y * kLT - kHalo;
-  const float4* im = img + (size_t)v * W * H;
-  const float4* tg = tgt + (size_t)tgt_ids[v] * W * H;
-  // staging in two halves, each issuing all its loads before its stores, so
-  // the load latency is paid twice rather than once per element
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    constexpr int kIt = (kLI * kLI + 511) / 512;  // 4 elements per thread per half
-    float4 a[kIt], b[kIt];
-#pragma unroll
-    for (int i = 0; i < kIt; ++i) {
-      const int e = tid + (half * kIt + i) * 256;
-      const int ly = e / kLI, lx = e - ly * kLI;
-      const int gx = ox + lx, gy = oy + ly;
-      a[i] = b[i] = make_float4(0, 0, 0, 0);
-      if (e < kLI * kLI && gx >= 0 && gy >= 0 && gx < (int)W && gy < (int)H) {
-        a[i] = im[(size_t)gy * W + gx];
-        b[i] = tg[(size_t)gy * W + gx];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kIt; ++i) {
-      const int e = tid + (half * kIt + i) * 256;
-      if (e >= kLI * kLI) continue;
-      const int ly = e / kLI, lx = e - ly * kLI;
-      const int o = ly * kLS + lx;
-      sx[o] = a[i].x; sx[kLI * kLS + o] = a[i].y; sx[2 * kLI * kLS + o] = a[i].z;
-      sy[o] = b[i].x; sy[kLI * kLS + o] = b[i].y; sy[2 * kLI * kLS + o] = b[i].z;
-    }
+// the three channels' warps of one strip of up to `rows` output rows
+struct SsimStrip {
+  int c, lane, px, gx0, gx1, y0, rows;  // channel; output column; the lane's staged columns; first row, rows
+  __device__ SsimStrip(uint32_t W, uint32_t H, uint32_t strip_rows)
+      : c(threadIdx.x >> 5), lane(threadIdx.x & 31), px(blockIdx.x * kSsimCols + (threadIdx.x & 31)),
+        gx0(px - kHalo), gx1(px - kHalo + kSsimCols), y0(blockIdx.y * strip_rows),
+        rows(min((int)strip_rows, (int)H - (int)(blockIdx.y * strip_rows))) {
+    if (gx0 >= (int)W) gx0 = -1;
+    if (lane >= 2 * kHalo || gx1 >= (int)W) gx1 = -1;  // the second column of lanes 0 .. 9 only
   }
-  __syncthreads();
-  const int col = tid & 31, rg = tid >> 5;  // vertical pass: column, 4-row group
-  const int px = blockIdx.x * kLT + col;
+};
+
+// copies of one row into shared memory, zeros where it is outside the image (size 0)
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src, bool inside) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(BYTES), "r"(inside ? BYTES : 0)
+               : "memory");
+}
+constexpr int kSsimRing = 4;  // rows of a warp in shared memory: one in use, three on their way
+// after it the row to be read next has landed for every lane, and the one before it may be overwritten
+__device__ __forceinline__ void ssim_row_ready() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kSsimRing - 2) : "memory");
+  __syncwarp();
+}
+__device__ __forceinline__ void ssim_row_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+__device__ __forceinline__ float2 ssim_fma2(float w, float2 v, float2 acc) {
+  return __ffma2_rn(make_float2(w, w), v, acc);
+}
+
+__global__ void __launch_bounds__(96) k_ssim_fwd(const float4* __restrict__ img, const float4* __restrict__ tgt,
+                                                 const uint32_t* __restrict__ tgt_ids, uint32_t W, uint32_t H,
+                                                 uint32_t strip_rows, float lambda, float inv_norm,
+                                                 float2* __restrict__ map_ab, float* __restrict__ map_c,
+                                                 float* __restrict__ partial) {
+  __shared__ float2 s_row[3][kSsimRing][kSsimRow];
+  __shared__ float red[2][3];
+  const SsimStrip st(W, H, strip_rows);
+  const uint32_t v = blockIdx.z;
+  const size_t plane = (size_t)W * H;
+  const float* im = reinterpret_cast<const float*>(img + v * plane) + st.c;
+  const float* tg = reinterpret_cast<const float*>(tgt + tgt_ids[v] * plane) + st.c;
+  float2* mab = map_ab + ((size_t)v * 3 + st.c) * plane;
+  float* mc = map_c + ((size_t)v * 3 + st.c) * plane;
+  float w[kHalo + 1];  // the window is symmetric
+#pragma unroll
+  for (int k = 0; k <= kHalo; ++k) w[k] = c_ssim_w[k];
+  const float2 one = make_float2(c_ssim_one, c_ssim_one);
+  const int nrows = st.rows + 2 * kHalo;
+  auto fetch = [&](int r) {  // staged row r: image row y0 + r - 5
+    const int gy = st.y0 + r - kHalo;
+    const bool in = r < nrows && gy >= 0 && gy < (int)H;
+    const size_t o = in ? 4 * ((size_t)gy * W) : 0;
+    float* d = reinterpret_cast<float*>(&s_row[st.c][r % kSsimRing][st.lane]);
+    const bool in0 = in && st.gx0 >= 0, in1 = in && st.gx1 >= 0;
+    const size_t o0 = in0 ? o + 4 * st.gx0 : 0, o1 = in1 ? o + 4 * st.gx1 : 0;
+    cp_async<4>(d, im + o0, in0);
+    cp_async<4>(d + 1, tg + o0, in0);
+    if (st.lane < 2 * kHalo) {
+      cp_async<4>(d + 2 * kSsimCols, im + o1, in1);
+      cp_async<4>(d + 2 * kSsimCols + 1, tg + o1, in1);
+    }
+    ssim_row_commit();
+  };
+  float2 hm[kSsimWin], hs[kSsimWin];  // row sums of (x, y) and (xx, yy), by row modulo 11
+  float hx[kSsimWin];                 // of xy
   float l1 = 0.0f, ss = 0.0f;
-  for (int c = 0; c < 3; ++c) {
-    const float* X = sx + c * kLI * kLS;
-    const float* Y = sy + c * kLI * kLS;
-    for (int r = tid; r < kLI * (kLT / 4); r += 256) {
-      const int row = r >> 3, x0 = (r & 7) * 4;
-      float xv[14], yv[14];
+  const float dLds = -lambda * inv_norm;
+  for (int r = 0; r < kSsimRing - 1; ++r) fetch(r);
+  for (int base = 0; base < nrows; base += kSsimWin) {
 #pragma unroll
-      for (int j = 0; j < 14; ++j) {
-        xv[j] = X[row * kLS + x0 + j];
-        yv[j] = Y[row * kLS + x0 + j];
-      }
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        float m0 = 0, m1 = 0, m2 = 0, m3 = 0, m4 = 0;
+    for (int i = 0; i < kSsimWin; ++i) {
+      const int r = base + i;  // staged row, image row y0 + r - 5
+      if (r < nrows) {
+        ssim_row_ready();
+        const float2* row = s_row[st.c][r % kSsimRing];
+        fetch(r + kSsimRing - 1);
+        float2 m = make_float2(0.0f, 0.0f), q = m, mid;
+        float xy = 0.0f;
 #pragma unroll
         for (int k = 0; k < kSsimWin; ++k) {
-          const float w = c_ssim_w[k], x = xv[o + k], y = yv[o + k];
-          m0 += w * x; m1 += w * y; m2 += w * x * x; m3 += w * y * y; m4 += w * x * y;
+          const float wk = w[k <= kHalo ? k : 2 * kHalo - k];
+          const float2 p = row[st.lane + k], wp = __fmul2_rn(make_float2(wk, wk), p);
+          if (k == kHalo) mid = p;
+          m = __ffma2_rn(wp, one, m);  // the rounded product, as in xx and yy (see c_ssim_one)
+          q = __ffma2_rn(wp, p, q);
+          xy = fmaf(wp.x, p.y, xy);
         }
-        const int q = row * kHS + x0 + o;
-        hm[q] = m0; hm[kLI * kHS + q] = m1; hm[2 * kLI * kHS + q] = m2;
-        hm[3 * kLI * kHS + q] = m3; hm[4 * kLI * kHS + q] = m4;
+        hm[i] = m;
+        hs[i] = q;
+        hx[i] = xy;
+        if (r >= kHalo && r < st.rows + kHalo && st.px < (int)W) l1 += fabsf(mid.x - mid.y);
+        if (r >= 2 * kHalo) {
+          float2 em = make_float2(0.0f, 0.0f), eq = em;
+          float exy = 0.0f;
+#pragma unroll
+          for (int k = 0; k < kSsimWin; ++k) {
+            const float wk = w[k <= kHalo ? k : 2 * kHalo - k];
+            const int slot = (i + 1 + k) % kSsimWin;  // rows r - 10 .. r
+            em = ssim_fma2(wk, hm[slot], em);
+            eq = ssim_fma2(wk, hs[slot], eq);
+            exy = fmaf(wk, hx[slot], exy);
+          }
+          if (st.px < (int)W) {
+            const float mx = em.x, my = em.y;
+            const float sxx = eq.x - mx * mx, syy = eq.y - my * my, sxy = exy - mx * my;
+            const float A1 = 2.0f * mx * my + kSsimC1, A2 = 2.0f * sxy + kSsimC2;
+            const float B1 = mx * mx + my * my + kSsimC1, B2 = sxx + syy + kSsimC2;
+            // two fast reciprocals instead of five divisions (B1, B2 >= C1, C2 > 0)
+            const float iB1 = rcp_normal(B1), iB2 = rcp_normal(B2), iB = iB1 * iB2;
+            const float sv = (A1 * A2) * iB;
+            ss += sv;
+            const float ds_dmx = (2.0f * my * A2) * iB - sv * 2.0f * mx * iB1;
+            const float ds_dsxx = -sv * iB2;
+            const float ds_dsxy = 2.0f * A1 * iB;
+            const float dm = dLds * ds_dmx, d2 = dLds * ds_dsxx, dxy = dLds * ds_dsxy;
+            const size_t pix = (size_t)(st.y0 + r - 2 * kHalo) * W + st.px;
+            mab[pix] = make_float2(dm - 2.0f * mx * d2 - my * dxy, d2);
+            mc[pix] = dxy;
+          }
+        }
       }
     }
-    __syncthreads();
-    float mo[4][5];
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      float hv[14];
-#pragma unroll
-      for (int j = 0; j < 14; ++j) hv[j] = hm[q * kLI * kHS + (rg * 4 + j) * kHS + col];
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kSsimWin; ++k) acc += c_ssim_w[k] * hv[o + k];
-        mo[o][q] = acc;
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-      const int py = blockIdx.y * kLT + rg * 4 + o;
-      if (px >= (int)W || py >= (int)H) continue;
-      const float mx = mo[o][0], my = mo[o][1];
-      const float sxx = mo[o][2] - mx * mx, syy = mo[o][3] - my * my, sxy = mo[o][4] - mx * my;
-      const float A1 = 2.0f * mx * my + kSsimC1, A2 = 2.0f * sxy + kSsimC2;
-      const float B1 = mx * mx + my * my + kSsimC1, B2 = sxx + syy + kSsimC2;
-      // two fast reciprocals instead of five divisions (B1, B2 >= C1, C2 > 0)
-      const float iB1 = rcp_normal(B1), iB2 = rcp_normal(B2), iB = iB1 * iB2;
-      const float sv = (A1 * A2) * iB;
-      ss += sv;
-      const float dLds = -lambda * inv_norm;
-      const float ds_dmx = (2.0f * my * A2) * iB - sv * 2.0f * mx * iB1;
-      const float ds_dsxx = -sv * iB2;
-      const float ds_dsxy = 2.0f * A1 * iB;
-      const float dm = dLds * ds_dmx, d2 = dLds * ds_dsxx, dxy = dLds * ds_dsxy;
-      const size_t plane = (size_t)W * H, pix = (size_t)py * W + px;
-      float* mp = maps + ((size_t)v * 9 + 3 * c) * plane + pix;
-      mp[0] = dm - 2.0f * mx * d2 - my * dxy;
-      mp[plane] = d2;
-      mp[2 * plane] = dxy;
-      const int cy = rg * 4 + o + kHalo, cx = col + kHalo;
-      l1 += fabsf(X[cy * kLS + cx] - Y[cy * kLS + cx]);
-    }
-    __syncthreads();  // before the next channel overwrites the horizontal sums
   }
   for (int o = 16; o > 0; o >>= 1) {
     l1 += __shfl_xor_sync(0xffffffffu, l1, o);
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
   }
-  if ((tid & 31) == 0) {
-    red[0][tid >> 5] = l1;
-    red[1][tid >> 5] = ss;
+  if (st.lane == 0) {
+    red[0][st.c] = l1;
+    red[1][st.c] = ss;
   }
   __syncthreads();
-  if (tid == 0) {
-    float a = 0, b = 0;
-    for (int w = 0; w < 8; ++w) { a += red[0][w]; b += red[1][w]; }
+  if (threadIdx.x == 0) {
     const size_t bi = ((size_t)v * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    partial[2 * bi] = a;
-    partial[2 * bi + 1] = b;
+    partial[2 * bi] = red[0][0] + red[0][1] + red[0][2];
+    partial[2 * bi + 1] = red[1][0] + red[1][1] + red[1][2];
   }
 }
 
-// four blocks per SM (at most 64 registers; five fit in shared memory)
-__global__ void __launch_bounds__(256, 4) k_ssim_bwd2(const float4* __restrict__ img, const float4* __restrict__ tgt,
-                                                   const uint32_t* __restrict__ tgt_ids,
-                                                   const float* __restrict__ maps, uint32_t W, uint32_t H,
-                                                   float lambda, float inv_norm, float4* __restrict__ dimg) {
-  extern __shared__ float sm[];
-  float* mp = sm;                    // [3][kLI][kLS]
-  float* hm = mp + 3 * kLI * kLS;    // [3][kLI][kHS]
-  const uint32_t v = blockIdx.z, tid = threadIdx.x;
-  const int ox = blockIdx.x * kLT - kHalo, oy = blockIdx.y * kLT - kHalo;
+// The channels' gradients of up to eleven rows meet in shared memory, so that a
+// pixel's leaves in one 16-byte store.
+__global__ void __launch_bounds__(96) k_ssim_bwd(const float4* __restrict__ img, const float4* __restrict__ tgt,
+                                                 const uint32_t* __restrict__ tgt_ids,
+                                                 const float2* __restrict__ map_ab, const float* __restrict__ map_c,
+                                                 uint32_t W, uint32_t H, uint32_t strip_rows, float lambda,
+                                                 float inv_norm, float4* __restrict__ dimg) {
+  __shared__ float2 s_ab[3][2][kSsimRow];
+  __shared__ float s_c[3][2][kSsimRow];
+  __shared__ float s_out[kSsimWin][3][kSsimCols];
+  const SsimStrip st(W, H, strip_rows);
+  const uint32_t v = blockIdx.z;
   const size_t plane = (size_t)W * H;
-  const int col = tid & 31, rg = tid >> 5;
-  const int px = blockIdx.x * kLT + col;
-  // the image and target are read per channel where they are used (they
-  // come from L2), so no registers hold them across the kernel
-  const float* imf = reinterpret_cast<const float*>(img + (size_t)v * plane);
-  const float* tgf = reinterpret_cast<const float*>(tgt + (size_t)tgt_ids[v] * plane);
+  const float* im = reinterpret_cast<const float*>(img + v * plane) + st.c;
+  const float* tg = reinterpret_cast<const float*>(tgt + tgt_ids[v] * plane) + st.c;
+  const float2* mab = map_ab + ((size_t)v * 3 + st.c) * plane;
+  const float* mc = map_c + ((size_t)v * 3 + st.c) * plane;
+  float w[kHalo + 1];
+#pragma unroll
+  for (int k = 0; k <= kHalo; ++k) w[k] = c_ssim_w[k];
   const float l1w = (1.0f - lambda) * inv_norm;
-  float d[4][3];
-  for (int c = 0; c < 3; ++c) {
-    const float* mv = maps + ((size_t)v * 9 + 3 * c) * plane;
-    {  // stage the channel's three maps: every load issued before the stores
-      constexpr int kIt = (kLI * kLI + 255) / 256;  // 7 elements per thread
-      float m0[kIt], m1[kIt], m2[kIt];
+  const int nrows = st.rows + 2 * kHalo;
+  struct Row {  // a staged row's values of this lane's columns, on their way
+    float2 ab0, ab1;
+    float c0, c1;
+  };
+  auto fetch = [&](int r) {  // staged row r: image row y0 + r - 5
+    Row n{make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), 0.0f, 0.0f};
+    const int gy = st.y0 + r - kHalo;
+    if (r >= nrows || gy < 0 || gy >= (int)H) return n;
+    const size_t o = (size_t)gy * W;
+    if (st.gx0 >= 0) {
+      n.ab0 = __ldg(mab + o + st.gx0);
+      n.c0 = __ldg(mc + o + st.gx0);
+    }
+    if (st.gx1 >= 0) {
+      n.ab1 = __ldg(mab + o + st.gx1);
+      n.c1 = __ldg(mc + o + st.gx1);
+    }
+    return n;
+  };
+  float x = 0.0f, y = 0.0f;
+  auto fetch_xy = [&](int r) {  // the pixel that row r completes
+    if (r >= 2 * kHalo && r < nrows && st.px < (int)W) {
+      const size_t o = 4 * ((size_t)(st.y0 + r - 2 * kHalo) * W + st.px);
+      x = __ldg(im + o);
+      y = __ldg(tg + o);
+    }
+  };
+  float2 hab[kSsimWin];
+  float hc[kSsimWin];
+  Row n0 = fetch(0), n1 = fetch(1);
+  for (int base = 0; base < nrows; base += kSsimWin) {
 #pragma unroll
-      for (int i = 0; i < kIt; ++i) {
-        const int e = tid + i * 256;
-        const int ly = e / kLI, lx = e - ly * kLI;
-        const int gx = ox + lx, gy = oy + ly;
-        const bool ok = e < kLI * kLI && gx >= 0 && gy >= 0 && gx < (int)W && gy < (int)H;
-        const size_t g = ok ? (size_t)gy * W + gx : 0;
-        m0[i] = ok ? mv[g] : 0.0f;
-        m1[i] = ok ? mv[plane + g] : 0.0f;
-        m2[i] = ok ? mv[2 * plane + g] : 0.0f;
-      }
+    for (int i = 0; i < kSsimWin; ++i) {
+      const int r = base + i;
+      if (r < nrows) {
+        float2* rab = s_ab[st.c][r & 1];
+        float* rc = s_c[st.c][r & 1];
+        rab[st.lane] = n0.ab0;
+        rc[st.lane] = n0.c0;
+        if (st.lane < 2 * kHalo) {
+          rab[kSsimCols + st.lane] = n0.ab1;
+          rc[kSsimCols + st.lane] = n0.c1;
+        }
+        __syncwarp();  // the other buffer was read before this point, so one per row is enough
+        n0 = n1;
+        n1 = fetch(r + 2);
+        const bool out = r >= 2 * kHalo && st.px < (int)W;
+        const float cx = x, cy = y;
+        fetch_xy(r + 1);
+        float2 ab = make_float2(0.0f, 0.0f);
+        float cc = 0.0f;
 #pragma unroll
-      for (int i = 0; i < kIt; ++i) {
-        const int e = tid + i * 256;
-        if (e >= kLI * kLI) continue;
-        const int ly = e / kLI, lx = e - ly * kLI;
-        const int o = ly * kLS + lx;
-        mp[o] = m0[i];
-        mp[kLI * kLS + o] = m1[i];
-        mp[2 * kLI * kLS + o] = m2[i];
+        for (int k = 0; k < kSsimWin; ++k) {
+          const float wk = w[k <= kHalo ? k : 2 * kHalo - k];
+          ab = ssim_fma2(wk, rab[st.lane + k], ab);
+          cc = fmaf(wk, rc[st.lane + k], cc);
+        }
+        hab[i] = ab;
+        hc[i] = cc;
+        if (out) {
+          float2 e = make_float2(0.0f, 0.0f);
+          float ec = 0.0f;
+#pragma unroll
+          for (int k = 0; k < kSsimWin; ++k) {
+            const float wk = w[k <= kHalo ? k : 2 * kHalo - k];
+            const int slot = (i + 1 + k) % kSsimWin;
+            e = ssim_fma2(wk, hab[slot], e);
+            ec = fmaf(wk, hc[slot], ec);
+          }
+          const float diff = cx - cy;
+          const float sgn = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
+          s_out[i][st.c][st.lane] = e.x + 2.0f * cx * e.y + cy * ec + l1w * sgn;
+        }
       }
     }
     __syncthreads();
-    for (int r = tid; r < 3 * kLI * (kLT / 4); r += 256) {
-      const int q = r / (kLI * (kLT / 4)), rr = r - q * (kLI * (kLT / 4));
-      const int row = rr >> 3, x0 = (rr & 7) * 4;
-      float mvv[14];
-#pragma unroll
-      for (int j = 0; j < 14; ++j) mvv[j] = mp[q * kLI * kLS + row * kLS + x0 + j];
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kSsimWin; ++k) acc += c_ssim_w[k] * mvv[o + k];
-        hm[q * kLI * kHS + row * kHS + x0 + o] = acc;
+    if (st.px < (int)W)
+      for (int i = st.c; i < kSsimWin; i += 3) {
+        const int r = base + i;
+        if (r >= 2 * kHalo && r < nrows)
+          dimg[v * plane + (size_t)(st.y0 + r - 2 * kHalo) * W + st.px] =
+              make_float4(s_out[i][0][st.lane], s_out[i][1][st.lane], s_out[i][2][st.lane], 0.0f);
       }
-    }
     __syncthreads();
-    float cv[4][3];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      float hv[14];
-#pragma unroll
-      for (int j = 0; j < 14; ++j) hv[j] = hm[q * kLI * kHS + (rg * 4 + j) * kHS + col];
-#pragma unroll
-      for (int o = 0; o < 4; ++o) {
-        float acc = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kSsimWin; ++k) acc += c_ssim_w[k] * hv[o + k];
-        cv[o][q] = acc;
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < 4; ++o) {
-      const int py = blockIdx.y * kLT + rg * 4 + o;
-      const bool in = px < (int)W && py < (int)H;
-      const size_t pix = in ? (size_t)py * W + px : 0;
-      const float x = in ? __ldg(imf + 4 * pix + c) : 0.0f;
-      const float y = in ? __ldg(tgf + 4 * pix + c) : 0.0f;
-      const float diff = x - y;
-      const float sgn = diff > 0.0f ? 1.0f : (diff < 0.0f ? -1.0f : 0.0f);
-      d[o][c] = cv[o][0] + 2.0f * x * cv[o][1] + y * cv[o][2] + l1w * sgn;
-    }
-    __syncthreads();  // before the next channel overwrites the staged maps
-  }
-#pragma unroll
-  for (int o = 0; o < 4; ++o) {
-    const int py = blockIdx.y * kLT + rg * 4 + o;
-    if (px < (int)W && py < (int)H)
-      dimg[(size_t)v * plane + (size_t)py * W + px] = make_float4(d[o][0], d[o][1], d[o][2], 0.0f);
   }
 }
 
@@ -2257,15 +2290,6 @@ int nps_gs_create(nps_ctx* ctx, uint32_t capacity, uint32_t sh_degree, nps_gs** 
   o->ctx = ctx;
   o->cap = capacity;
   o->n = 0;
-  // kernels with more than 48 KB of dynamic shared memory (set outside any capture)
-  if (cudaFuncSetAttribute(gs::k_ssim_fwd2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs::kSsimFwdSmem) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(gs::k_ssim_bwd2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs::kSsimBwdSmem) !=
-          cudaSuccess) {
-    delete o;
-    set_error("nps_gs_create: cannot raise the loss kernels' shared-memory limit");
-    return NPS_ERR_CUDA;
-  }
   o->sh_deg = (int)sh_degree;
   const size_t pb = sizeof(float) * gsm::kP * (size_t)capacity;
   int rc = NPS_OK;
@@ -2933,6 +2957,25 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
   return NPS_OK;
 }
 
+// Rows per strip of an SSIM kernel of which `resident` blocks run at once: the
+// blocks of a launch take equally long, so its time is the number of waves times the
+// rows of a strip and the ten that it shares with its neighbours (and about four
+// rows' time to start).  The least of that product over the strip counts gives one wave of
+// long strips where they fill the device and eight rows or more on small images.
+static uint32_t ssim_strip_rows(uint32_t columns, uint32_t H, uint32_t resident) {
+  uint32_t best = H;
+  uint64_t least = ~0ull;
+  for (uint32_t strips = 1; strips <= div_up(H, 8); ++strips) {
+    const uint32_t rows = div_up(H, strips);
+    const uint64_t t = (uint64_t)div_up((size_t)columns * div_up(H, rows), resident) * (rows + 14);
+    if (t < least) {
+      least = t;
+      best = rows;
+    }
+  }
+  return best;
+}
+
 extern "C" {
 
 int nps_gs_forward(nps_gs* o, float* out_rgba) {
@@ -2967,17 +3010,21 @@ int nps_gs_loss(nps_gs* o, float* loss3_host) {
                                                  (float)nv / (float)lv, o->loss.as<float>());
     NPS_CHECK_LAUNCH();
   } else {
-    const dim3 grid(div_up(W, gs::kLT), div_up(H, gs::kLT), nv);
-    const uint32_t nblocks = grid.x * grid.y * grid.z;
+    static int resident_fwd = 0, resident_bwd = 0;
+    const uint32_t columns = div_up(W, gs::kSsimCols);
+    const uint32_t rows_f = ssim_strip_rows(columns * nv, H, persistent_grid(o, gs::k_ssim_fwd, 96, &resident_fwd));
+    const uint32_t rows_b = ssim_strip_rows(columns * nv, H, persistent_grid(o, gs::k_ssim_bwd, 96, &resident_bwd));
+    const dim3 grid_f(columns, div_up(H, rows_f), nv), grid_b(columns, div_up(H, rows_b), nv);
+    const uint32_t nblocks = grid_f.x * grid_f.y * grid_f.z;
     NPS_TRY(o->maps.ensure(sizeof(float) * 9 * npix));
     NPS_TRY(o->partial.ensure(sizeof(float) * 2 * nblocks));
     StageTimer t(o, ST_LOSS);
-    gs::k_ssim_fwd2<<<grid, 256, gs::kSsimFwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids(), W, H,
-                                                       o->lambda, inv_norm, o->maps.as<float>(),
-                                                       o->partial.as<float>());
-    gs::k_ssim_bwd2<<<grid, 256, gs::kSsimBwdSmem, s>>>(o->img.as<float4>(), o->tgt, o->tids(),
-                                                       o->maps.as<float>(), W, H, o->lambda, inv_norm,
-                                                       o->dimg.as<float4>());
+    float2* map_ab = o->maps.as<float2>();
+    float* map_c = o->maps.as<float>() + 6 * npix;
+    gs::k_ssim_fwd<<<grid_f, 96, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids(), W, H, rows_f, o->lambda, inv_norm,
+                                         map_ab, map_c, o->partial.as<float>());
+    gs::k_ssim_bwd<<<grid_b, 96, 0, s>>>(o->img.as<float4>(), o->tgt, o->tids(), map_ab, map_c, W, H, rows_b,
+                                         o->lambda, inv_norm, o->dimg.as<float4>());
     gs::k_loss_reduce<<<1, gs::kThreads, 0, s>>>(o->partial.as<float>(), nblocks, o->loss_kind, o->lambda,
                                                  inv_norm, (float)nv / (float)lv, o->loss.as<float>());
     NPS_CHECK_LAUNCH();

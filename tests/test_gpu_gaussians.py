@@ -325,6 +325,24 @@ def test_deterministic_mode_is_bit_reproducible(trainer_cls, tmp_path):
     np.testing.assert_array_equal(r.read_state()["adam_v"], runs[0].read_state()["adam_v"])
 
 
+@pytest.mark.parametrize("w,h,views", [(5, 3, 1), (31, 9, 1), (32, 8, 2), (33, 11, 1), (64, 32, 1), (27, 203, 1), (530, 75, 3),
+                                       (200, 1001, 2)])
+def test_ssim_strips_match_oracle(trainer_cls, w, h, views):
+    """Loss and image gradient where the 32-column strips and their row ranges
+    are ragged, shorter than the window, or several to a column.  Bounds as above;
+    the gradient as relative L2 (1e-4)."""
+    p = gs_scene(600, 81, deg=0, log_scale_mean=-2.6)
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0), (-2.0, 0.5, 3.0))[:views])
+    tg = gs_targets(views, w, h, 82)
+    tids = np.arange(views, dtype=np.uint32)
+    t, img, l3, _ = run_gpu(trainer_cls, p, 0, vp, vpi, tg, tids)
+    rl3, rdimg = orc.gs_loss(img, tg, tids)
+    np.testing.assert_allclose(l3[:2], rl3[:2], rtol=1e-5, atol=1e-7)
+    assert abs(l3[2] - rl3[2]) < 2e-5, (l3, rl3)
+    d, r = t.read_image()[1][..., :3].astype(np.float64), rdimg[..., :3].astype(np.float64)
+    assert np.linalg.norm(d - r) / np.linalg.norm(r) < 1e-4
+
+
 @pytest.mark.parametrize("w,h,views", [(64, 50, 1), (640, 400, 1), (400, 320, 4), (800, 639, 1)])
 def test_default_raster_follows_the_grid_size(trainer_cls, w, h, views):
     """Without a chosen variant a pass takes 1 pixel per thread on a grid of
