@@ -1338,7 +1338,7 @@ __global__ void __launch_bounds__(kThreads) k_bwd(const Rec* __restrict__ recs, 
 struct PixBwd {
   float T;          // transmittance in front of the pair being replayed
   float nbg;        // -T_final (background . dL/dpixel)
-  float last_alpha, acc_dot, last_dot;
+  float acc_dot;    // colour behind it . dL/dpixel
   float dC[3];
   float fx, fy;
   uint32_t last;    // contributors of the pixel; 0 outside the image
@@ -1362,7 +1362,7 @@ __device__ __forceinline__ void pix_bwd_init(PixBwd& s, uint32_t px, uint32_t py
     s.dC[0] = d.x; s.dC[1] = d.y; s.dC[2] = d.z;
   }
   s.nbg = -s.T * (bg.x * s.dC[0] + bg.y * s.dC[1] + bg.z * s.dC[2]);
-  s.last_alpha = s.acc_dot = s.last_dot = 0.0f;
+  s.acc_dot = 0.0f;
 }
 
 // Scale of gradient term k that pix_bwd_apply leaves out of its per-pixel sums
@@ -1396,31 +1396,30 @@ __device__ __forceinline__ PairAt pix_bwd_prep(const PixBwd& s, const float4& a,
   return r;
 }
 
-// advances the replay state past a contributing pair of colour (b.z, b.w, cx) and
-// adds this pixel's gradient with respect to it to gv[0..8] (terms 0..4 without
-// their bwd_term_scale)
+// advances the replay state past the pair, of colour (b.z, b.w, cx), if it
+// contributes, and adds this pixel's gradient with respect to it to gv[0..8]
+// (terms 0..4 without their bwd_term_scale).  Selections instead of a branch, for
+// the reason above (922 -> 870 us); what a pair that does not contribute would add is
+// never added, so that a NaN stays with the pixels and Gaussians it belongs to.
 __device__ __forceinline__ void pix_bwd_apply(PixBwd& s, const PairAt& r, const float4& b, float cx, float (&gv)[9]) {
-  if (!r.ok) return;
-  s.T = s.T * r.inv1ma;
+  s.T = r.ok ? s.T * r.inv1ma : s.T;
   const float wgt = r.alpha * s.T;
-  // colour behind this pair, dotted with dL/dpixel: last_alpha * last + (1 - last_alpha) * acc
-  const float cdot = fmaf(cx, s.dC[2], fmaf(b.w, s.dC[1], b.z * s.dC[0]));
-  s.acc_dot = fmaf(s.last_alpha, s.last_dot - s.acc_dot, s.acc_dot);
-  s.last_dot = cdot;
-  s.last_alpha = r.alpha;
-  const float dL_dalpha = fmaf(s.nbg, r.inv1ma, (cdot - s.acc_dot) * s.T);
+  // this pair's colour less the colour behind it, dotted with dL/dpixel
+  const float d = fmaf(cx, s.dC[2], fmaf(b.w, s.dC[1], b.z * s.dC[0])) - s.acc_dot;
+  const float dL_dalpha = fmaf(s.nbg, r.inv1ma, d * s.T);
+  s.acc_dot = r.ok ? fmaf(r.alpha, d, s.acc_dot) : s.acc_dot;
 #pragma unroll
-  for (int c = 0; c < 3; ++c) gv[6 + c] = fmaf(wgt, s.dC[c], gv[6 + c]);
-  if (r.araw <= kAlphaMax) {
-    // dL/dG = opacity dL/dalpha; h = G dL/dG
-    const float h = r.araw * dL_dalpha, hx = h * r.dx, hy = h * r.dy;
-    gv[0] = fmaf(h, r.u, gv[0]);          // d/du:  -h u
-    gv[1] = fmaf(h, r.w, gv[1]);          // d/dv:  -h w
-    gv[2] = fmaf(hx, r.dx, gv[2]);        // d/d conic a: -h dx dx / 2
-    gv[3] = fmaf(hx, r.dy, gv[3]);        // d/d conic b: -h dx dy
-    gv[4] = fmaf(hy, r.dy, gv[4]);        // d/d conic c: -h dy dy / 2
-    gv[5] = fmaf(r.G, dL_dalpha, gv[5]);  // d/d opacity
-  }
+  for (int c = 0; c < 3; ++c) gv[6 + c] = r.ok ? fmaf(wgt, s.dC[c], gv[6 + c]) : gv[6 + c];
+  // dL/dG = opacity dL/dalpha; h = G dL/dG
+  const bool in = r.ok && r.araw <= kAlphaMax;
+  const float h = in ? r.araw * dL_dalpha : 0.0f;
+  const float hx = h * r.dx, hy = h * r.dy;
+  gv[0] = fmaf(h, r.u, gv[0]);                             // d/du:  -h u
+  gv[1] = fmaf(h, r.w, gv[1]);                             // d/dv:  -h w
+  gv[2] = fmaf(hx, r.dx, gv[2]);                           // d/d conic a: -h dx dx / 2
+  gv[3] = fmaf(hx, r.dy, gv[3]);                           // d/d conic b: -h dx dy
+  gv[4] = fmaf(hy, r.dy, gv[4]);                           // d/d conic c: -h dy dy / 2
+  gv[5] = in ? fmaf(r.G, dL_dalpha, gv[5]) : gv[5];        // d/d opacity
 }
 
 // gv: the gradient of PPT pixels with respect to the pair; returns whether it
@@ -1452,10 +1451,10 @@ __device__ __forceinline__ bool pixels_bwd(PixBwd (&p)[PPT], const Rec& rec, uin
 // compare-and-swap loop in shared memory per warp and pair and a scattered flush
 // per batch (1240 -> 1195 us at 200k Gaussians, 8 views of 800 x 800).  PPT is the
 // autotuned variant.  Issue-bound at 2 pixels per thread (77% of the issue slots):
-// 72 registers, seven 128-thread blocks per SM (eight give 1020 us where seven give
-// 965).  One pixel per thread serves small grids, which are bound by the latency of
+// 72 registers, seven 128-thread blocks per SM (eight give 152 -> 160 us at 57k Gaussians
+// and the same at 200k).  One pixel per thread serves small grids, which are bound by the latency of
 // the chain from pair to pair: two pairs are evaluated and reduced together
-// (65 -> 43 us at 16 tiles, with 80 registers).
+// (65 -> 37 us at 16 tiles, with 80 registers).
 template <int PPT, int SPS, bool kOrd>
 __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_bwd2(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
                                                     const uint32_t* __restrict__ rstart,
@@ -2602,12 +2601,12 @@ constexpr int kTuneStride = 1 + 2 * kNumVariants;
 // are resident, and 1 pixel per thread has the shorter chain and twice the warps;
 // a grid that fills the device several times over is bound by issue, where 2 pixels
 // per thread share a pair's loads and its reduction.  Forward / backward in us at
-// (1, 256) and at (2, 128), one view: 16 tiles 22 / 43 and 32 / 70; 256 tiles 39 / 64
-// and 50 / 101; 784 tiles 46 / 85 and 45 / 92; 1024 tiles 48 / 101 and 51 / 101; 1936
-// tiles 71 / 151 and 73 / 123; 2500 tiles 83 / 171 and 79 / 146; 6084 tiles 157 / 333
-// and 132 / 241.
+// (1, 256) and at (2, 128): 16 tiles 22 / 37 and 32 / 54; 256 tiles 32 / 58 and 50 /
+// 77; 512 tiles of eight views 90 / 156 and 117 / 178; 576 tiles 42 / 85 and 49 / 84;
+// 784 tiles 45 / 83 and 45 / 78; 1024 tiles 48 / 100 and 50 / 86; 1936 tiles 73 / 147
+// and 72 / 114; 2500 tiles 85 / 171 and 80 / 136; 6084 tiles 161 / 332 and 135 / 222.
 static RasterVariant default_variant(const nps_gs* o, bool bwd, uint32_t nitems) {
-  const uint32_t per_sm = bwd ? 6 : 12;
+  const uint32_t per_sm = bwd ? 4 : 12;
   return nitems <= per_sm * (uint32_t)o->ctx->sm_count ? RasterVariant{0, 1, 256} : RasterVariant{0, 2, 128};
 }
 static RasterVariant raster_variant(const nps_gs* o, bool bwd) {
