@@ -164,25 +164,27 @@ __device__ __forceinline__ float warp_sum16(float (&v)[16], uint32_t lane) {
 
 // Sums of 9 values over the warp through shared memory (sm: one 9 x kRedStride
 // array per warp): each lane stores its values, then lanes 2k and 2k + 1 each add
-// half of row k in packed pairs and exchange their halves.  Returns value k's
-// total in lanes 2k, 2k + 1 (k < 9).  27 warp instructions; a reduce-scatter by
-// shuffles takes 12 shuffles and 40 selects and additions (50% more instructions
-// in a kernel bound by issue: backward 1020 -> 965 us at 200k Gaussians, 8 views of
-// 800 x 800).  A row of 36 words keeps the 16-byte loads of eight lanes, and the
+// half of row k, the even or the odd lanes' values, in packed pairs and exchange
+// their halves.  Returns value k's total in lanes 2k, 2k + 1 (k < 9).  The additions form
+// the tree of a butterfly over lane distances 16, 8, 4, 2, 1, as in warp_sum9x2.  27
+// warp instructions; a reduce-scatter by shuffles takes 12 shuffles and 40 selects and
+// additions (5% of the backward at 200k Gaussians, 8 views of 800 x 800, where it is
+// bound by issue).  A row of 36 words keeps the 16-byte loads of eight lanes, and the
 // stores, free of bank conflicts.
 constexpr int kRedStride = 36;
 __device__ __forceinline__ float warp_total9(const float (&v)[9], uint32_t lane, float* sm) {
+  const uint32_t at = (lane & 1u) * 16u + (lane >> 1);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) sm[k * kRedStride + lane] = v[k];
+  for (int k = 0; k < 9; ++k) sm[k * kRedStride + at] = v[k];
   __syncwarp();
   const uint32_t l = min(lane, 17u);
   const float4* c = reinterpret_cast<const float4*>(sm + (l >> 1) * kRedStride + (l & 1u) * 16u);
   const float4 q0 = c[0], q1 = c[1], q2 = c[2], q3 = c[3];
-  const float2 s01 = __fadd2_rn(__fadd2_rn(make_float2(q0.x, q0.y), make_float2(q0.z, q0.w)),
-                                __fadd2_rn(make_float2(q1.x, q1.y), make_float2(q1.z, q1.w)));
-  const float2 s23 = __fadd2_rn(__fadd2_rn(make_float2(q2.x, q2.y), make_float2(q2.z, q2.w)),
-                                __fadd2_rn(make_float2(q3.x, q3.y), make_float2(q3.z, q3.w)));
-  const float2 s = __fadd2_rn(s01, s23);
+  const float2 a = __fadd2_rn(make_float2(q0.x, q0.y), make_float2(q2.x, q2.y));
+  const float2 b = __fadd2_rn(make_float2(q0.z, q0.w), make_float2(q2.z, q2.w));
+  const float2 d = __fadd2_rn(make_float2(q1.x, q1.y), make_float2(q3.x, q3.y));
+  const float2 e = __fadd2_rn(make_float2(q1.z, q1.w), make_float2(q3.z, q3.w));
+  const float2 s = __fadd2_rn(__fadd2_rn(a, d), __fadd2_rn(b, e));
   const float half = s.x + s.y;
   const float t = half + __shfl_xor_sync(0xffffffffu, half, 1);
   __syncwarp();  // sm may be written again
@@ -1399,7 +1401,7 @@ __device__ __forceinline__ PairAt pix_bwd_prep(const PixBwd& s, const float4& a,
 // advances the replay state past the pair, of colour (b.z, b.w, cx), if it
 // contributes, and adds this pixel's gradient with respect to it to gv[0..8]
 // (terms 0..4 without their bwd_term_scale).  Selections instead of a branch, for
-// the reason above (922 -> 870 us); what a pair that does not contribute would add is
+// the reason above (5% of the backward); what a pair that does not contribute would add is
 // never added, so that a NaN stays with the pixels and Gaussians it belongs to.
 __device__ __forceinline__ void pix_bwd_apply(PixBwd& s, const PairAt& r, const float4& b, float cx, float (&gv)[9]) {
   s.T = r.ok ? s.T * r.inv1ma : s.T;
@@ -1445,16 +1447,16 @@ __device__ __forceinline__ bool pixels_bwd(PixBwd (&p)[PPT], const Rec& rec, uin
 // Backward raster, PPT vertically adjacent pixels per thread (256 / PPT
 // threads per 16 x 16 tile): one warp reduction serves 32·PPT pixels.  The warp
 // first ballots the staged pairs that meet its strip and that some of its pixels
-// reached, then walks them in reverse order and adds each pair's warp totals to
-// the (view, Gaussian) record with one coalesced instruction of global
-// additions: nothing waits for them, where sums kept per block cost a
-// compare-and-swap loop in shared memory per warp and pair and a scattered flush
-// per batch (1240 -> 1195 us at 200k Gaussians, 8 views of 800 x 800).  PPT is the
+// reached, then walks them in reverse order and adds each pair's warp totals in
+// shared memory; a batch's sums leave in runs of nine words, one run per (view,
+// Gaussian) record.  (Adding the warp totals to the records directly is 4%
+// faster, and where a large Gaussian's terms cancel the longer sums lose digits
+// to it, so the block's share is summed first.)  PPT is the
 // autotuned variant.  Issue-bound at 2 pixels per thread (77% of the issue slots):
-// 72 registers, seven 128-thread blocks per SM (eight give 152 -> 160 us at 57k Gaussians
-// and the same at 200k).  One pixel per thread serves small grids, which are bound by the latency of
+// 72 registers, seven 128-thread blocks per SM (eight are 5% slower at 57k Gaussians
+// and the same at 200k); 1240 -> 921 us at 200k Gaussians, 8 views of 800 x 800.  One pixel per thread serves small grids, which are bound by the latency of
 // the chain from pair to pair: two pairs are evaluated and reduced together
-// (65 -> 37 us at 16 tiles, with 80 registers).
+// (65 -> 40 us at 16 tiles, with 80 registers).
 template <int PPT, int SPS, bool kOrd>
 __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_bwd2(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
                                                     const uint32_t* __restrict__ rstart,
@@ -1468,8 +1470,11 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_
   constexpr int NT = 256 / PPT, SB = NT * SPS;
   static_assert(SB <= 256, "staging buffers beyond the static shared-memory budget");
   __shared__ __align__(16) Rec s_rec[2][SB];
-  __shared__ uint32_t s_g[2][SB];
-  __shared__ __align__(16) float s_red[PPT == 1 ? 1 : NT / 32][9 * kRedStride];
+  __shared__ uint32_t s_g[3][SB];
+  __shared__ float s_acc[2][SB * 9];
+  // the largest stage leaves no room for the warps' arrays, and one pixel per thread does not use them
+  constexpr bool kShared = PPT > 1 && SB * (2 * sizeof(Rec) + 18 * 4 + 12) + NT / 32 * 9 * kRedStride * 4 <= 47 * 1024;
+  __shared__ __align__(16) float s_red[kShared ? NT / 32 : 1][9 * kRedStride];
   __shared__ __align__(8) uint64_t s_bar[2];
   __shared__ uint32_t s_max;
   uint32_t tx = blockIdx.x, ty = blockIdx.y, v = blockIdx.z;
@@ -1504,6 +1509,7 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_
     mbar_init(&s_bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  for (uint32_t r = tid; r < (uint32_t)(2 * SB * 9); r += NT) (&s_acc[0][0])[r] = 0.0f;
   __syncthreads();
   atomicMax(&s_max, mylast);
   __syncthreads();
@@ -1521,19 +1527,25 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_
     const uint32_t b0 = bstart_of(0);
     stage_batch(recs, vals, b0, start + maxlast - b0, s_rec[0], &s_bar[0], s_g[0]);
   }
-  // One CTA barrier per batch: it orders the re-staging of s_rec[bi & 1] (issued at
-  // batch bi + 1, after the barrier of batch bi) after every read of it.
+  // One CTA barrier per batch: batch bi accumulates into s_acc[bi & 1]; after
+  // the barrier the threads flush and clear that buffer while others may already
+  // walk batch bi + 1 into the other one.  The barrier also orders the re-staging of
+  // s_rec[bi & 1] (issued at batch bi + 1, after the barrier of batch bi) after
+  // every read of it, and the record ids rotate through three buffers so that
+  // staging batch bi + 2 never overwrites the ids the flush of batch bi is still
+  // reading.
+  uint32_t gb = 0;  // bi % 3
   for (uint32_t bi = 0; bi < nbatch; ++bi) {
-    const uint32_t buf = bi & 1u;
+    const uint32_t buf = bi & 1u, gnext = gb == 2u ? 0u : gb + 1u;
     const uint32_t bend = start + maxlast - bi * SB, bstart = bstart_of(bi);
     const uint32_t nb = bend - bstart;
     if (bi + 1 < nbatch) {
       const uint32_t nbs = bstart_of(bi + 1);
-      stage_batch(recs, vals, nbs, bstart - nbs, s_rec[buf ^ 1u], &s_bar[buf ^ 1u], s_g[buf ^ 1u]);
+      stage_batch(recs, vals, nbs, bstart - nbs, s_rec[buf ^ 1u], &s_bar[buf ^ 1u], s_g[gnext]);
     }
     if (!mbar_wait(&s_bar[buf], (bi >> 1) & 1u)) s_abort = 1u;  // the batch is undefined: end the tile below
     const Rec* sr = s_rec[buf];
-    const uint32_t* sg = s_g[buf];
+    float* acc = s_acc[buf];
     uint32_t hit[SB / 32];
 #pragma unroll
     for (int qq = 0; qq < SB / 32; ++qq) {
@@ -1564,15 +1576,23 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_
             const uint32_t k = warp_sum9x2_index(lane);
             const bool second = lane & 8u;
             if (k < 9 && (two || !second))
-              atomicAdd(g2 + (size_t)sg[second ? j2 : j] * kG2 + k, tot * bwd_term_scale(k));
+              atomicAdd(acc + (second ? j2 : j) * 9 + k, tot * bwd_term_scale(k));
           }
         } else {
           float gv[9];
           const bool any = pixels_bwd<PPT>(p, sr[j], cur, gv);
           if (__any_sync(0xffffffffu, any)) {
-            const float tot = warp_total9(gv, lane, s_red[tid >> 5]);
-            const uint32_t k = lane >> 1;
-            if ((lane & 1) == 0 && k < 9) atomicAdd(g2 + (size_t)sg[j] * kG2 + k, tot * bwd_term_scale(k));
+            float tot;
+            uint32_t k;
+            if constexpr (kShared) {
+              tot = warp_total9(gv, lane, s_red[tid >> 5]);
+              k = (lane & 1) == 0 ? lane >> 1 : 15u;
+            } else {
+              const float none[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+              tot = warp_sum9x2(gv, none, lane);
+              k = (lane & 8) == 0 ? warp_sum9x2_index(lane) : 15u;
+            }
+            if (k < 9) atomicAdd(acc + j * 9 + k, tot * bwd_term_scale(k));
           }
         }
       }
@@ -1587,6 +1607,15 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_
       }
       return;
     }
+    for (uint32_t e = tid; e < nb * 9u; e += NT) {
+      const float x = acc[e];
+      if (x != 0.0f) {
+        const uint32_t r = e / 9u;
+        atomicAdd(g2 + (size_t)s_g[gb][r] * kG2 + (e - 9u * r), x);
+        acc[e] = 0.0f;
+      }
+    }
+    gb = gnext;
   }
 }
 
@@ -2601,10 +2630,10 @@ constexpr int kTuneStride = 1 + 2 * kNumVariants;
 // are resident, and 1 pixel per thread has the shorter chain and twice the warps;
 // a grid that fills the device several times over is bound by issue, where 2 pixels
 // per thread share a pair's loads and its reduction.  Forward / backward in us at
-// (1, 256) and at (2, 128): 16 tiles 22 / 37 and 32 / 54; 256 tiles 32 / 58 and 50 /
-// 77; 512 tiles of eight views 90 / 156 and 117 / 178; 576 tiles 42 / 85 and 49 / 84;
-// 784 tiles 45 / 83 and 45 / 78; 1024 tiles 48 / 100 and 50 / 86; 1936 tiles 73 / 147
-// and 72 / 114; 2500 tiles 85 / 171 and 80 / 136; 6084 tiles 161 / 332 and 135 / 222.
+// (1, 256) and at (2, 128): 16 tiles 22 / 40 and 32 / 62; 256 tiles 32 / 60 and 50 /
+// 90; 512 tiles of eight views 90 / 173 and 117 / 197; 576 tiles 43 / 87 and 48 / 93;
+// 784 tiles 42 / 85 and 45 / 87; 1024 tiles 49 / 101 and 51 / 94; 1936 tiles 73 / 150
+// and 73 / 118; 2500 tiles 84 / 175 and 79 / 149; 6084 tiles 159 / 339 and 133 / 236.
 static RasterVariant default_variant(const nps_gs* o, bool bwd, uint32_t nitems) {
   const uint32_t per_sm = bwd ? 4 : 12;
   return nitems <= per_sm * (uint32_t)o->ctx->sm_count ? RasterVariant{0, 1, 256} : RasterVariant{0, 2, 128};
