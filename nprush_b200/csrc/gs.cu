@@ -249,6 +249,14 @@ __device__ __forceinline__ float exp_half(float q) {
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
 // ------------------------------------------------------------ preprocess
+// an asynchronous copy into shared memory of 4, 8 or 16 bytes, zeros if they are not to be read
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src, bool inside) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src), "n"(BYTES), "r"(inside ? BYTES : 0)
+               : "memory");
+}
+
 // What binning needs of a projected record: its tile rectangle (x0 | x1 << 16,
 // y0 | y1 << 16), the mask of the rectangle's tiles that get a pair (rectangles
 // of at most 32 tiles) and the number of pairs.  One 16-byte word, because the
@@ -264,7 +272,8 @@ __device__ __forceinline__ uint32_t rect_tiles(uint32_t x, uint32_t y) {
 // memory, once for all views, and the projected ones leave through it, in whole
 // lines.  The shared strides (17 and 3 float4) keep 16-byte accesses free of
 // bank conflicts.  200k Gaussians, SH3, 8 views: 110 -> 78 us; 1M: 500 -> 336 us
-// (bytes that it cannot do without: 36 and 181 us).
+// (bytes that it cannot do without: 36 and 181 us).  The copies are asynchronous, so that
+// a block of one view, which has few threads to stage with, waits for them once.
 constexpr uint32_t kPreStride = 17;  // float4 per staged parameter record (16 and a pad)
 constexpr size_t pre_smem(uint32_t group, uint32_t threads) {
   return (size_t)group * kPreStride * 16 + (size_t)threads * sizeof(Rec);
@@ -284,7 +293,8 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
     const float4* src = reinterpret_cast<const float4*>(params) + (size_t)i0 * (kP / 4);
     const uint32_t have = min(group, n - i0) * (kP / 4);
     for (uint32_t e = threadIdx.x; e < have; e += blockDim.x)
-      if ((e & 15u) < kUsed4) sm_pre[(e >> 4) * kPreStride + (e & 15u)] = __ldg(src + e);
+      if ((e & 15u) < kUsed4) cp_async<16>(sm_pre + (e >> 4) * kPreStride + (e & 15u), src + e, true);
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   __syncthreads();
   if (v >= nv || i0 + (gi & ~31u) >= n) return;  // whole warps
@@ -838,13 +848,6 @@ struct SsimStrip {
   }
 };
 
-// copies of one row into shared memory, zeros where it is outside the image (size 0)
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* dst, const void* src, bool inside) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-               "l"(src), "n"(BYTES), "r"(inside ? BYTES : 0)
-               : "memory");
-}
 constexpr int kSsimRing = 4;  // rows of a warp in shared memory: one in use, three on their way
 // after it the row to be read next has landed for every lane, and the one before it may be overwritten
 __device__ __forceinline__ void ssim_row_ready() {
