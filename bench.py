@@ -36,13 +36,13 @@ N_GAUSS, N_TEACHER, WIDTH, HEIGHT, VIEWS, CAMS, SH_DEG = 200_000, 250_000, 800, 
 P_USED = 59          # floats per Gaussian used by the model
 # DRAM traffic of one backward-raster launch (dram__bytes_read.sum + dram__bytes_write.sum) from one
 # 1-pass ncu capture of this workload (11,433,806 pairs): scaled to a launch by its pair count.
-BWD_TRAFFIC_BYTES, BWD_TRAFFIC_PAIRS = 239_281_152 + 18_662_144, 11_433_806
+BWD_TRAFFIC_BYTES, BWD_TRAFFIC_PAIRS = 239_885_824 + 18_334_720, 11_433_806
 S_REC = 36           # algorithmic projected-record bytes (mean2d, conic, rgb, opacity)
 # Warp instructions issued by one launch of each raster kernel (smsp__inst_executed.sum) in a 1-pass
 # ncu capture of this workload with the variant named, and that launch's pair count: scaled to a
 # launch by its pair count.  Key: (stage, form, pixels per thread, records per stage) at 16 x 16 tiles.
-RASTER_INST = {("raster_fwd", 2, 2, 128): (548_836_695, 11_433_806),
-               ("raster_bwd", 2, 2, 128): (1_183_662_764, 11_433_806)}
+RASTER_INST = {("raster_fwd", 2, 2, 128): (438_749_453, 11_433_806),
+               ("raster_bwd", 2, 2, 128): (772_862_980, 11_433_806)}
 SMS, ISSUE_PER_SM_CLK = 148, 4  # B200: 148 SMs, four warp schedulers each issuing one instruction per clock
 
 

@@ -223,7 +223,7 @@ int nps_bezier_opt_set_target(nps_bezier_opt* opt, const float* target_rgba, con
 int nps_bezier_opt_dispatch(nps_bezier_opt* opt);
 /* The stages of dispatch separately; backward optionally writes the composite
  * (num_views*h*w*4: r, g, b, reciprocal depth) to out_rgbd (device).  Its
- * work memory includes 37 KB of transmittance checkpoints per (view, 16 x 16
+ * work memory includes 43 KB of transmittance checkpoints per (view, 16 x 16
  * tile). */
 int nps_bezier_opt_backward(nps_bezier_opt* opt, float* out_rgbd_device);
 int nps_bezier_opt_step(nps_bezier_opt* opt);
