@@ -28,6 +28,7 @@
 //   k_project_bwd  up to eight lanes per Gaussian over the views: screen-space
 //                  gradients -> parameter gradients, ADC statistics
 //   k_adam         fused Adam over the 59 parameters of every Gaussian
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -2684,7 +2685,7 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool clear
   uint32_t* err = o->stepst.as<uint32_t>() + 6;
   if (form == 1) {
     uint32_t* q = o->ws_q.as<uint32_t>();
-    gs::k_order_items<false><<<1, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(), q);
+    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(), q);
     NPS_CHECK_LAUNCH();
 #define NPS_FWD_WS(TS, PPT, SB)                                                                                \
   do {                                                                                                         \
@@ -2719,7 +2720,7 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool clear
   }
   const bool ord = form == 2;
   if (ord) {
-    gs::k_order_items<false><<<1, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(),
+    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(),
                                                 o->ws_q.as<uint32_t>());
     NPS_CHECK_LAUNCH();
   }
@@ -2758,7 +2759,7 @@ static int launch_bwd_raster(nps_gs* o, int form, int ppt, int stage, const floa
   if (form == 1) {
     NPS_TRY(ensure_ws_buffers(o, nitems));
     uint32_t* q = o->ws_q.as<uint32_t>() + 2;
-    gs::k_order_items<true><<<1, 1024, 0, s>>>(nullptr, nullptr, o->tile_last.as<uint32_t>(), nitems,
+    gs::k_order_items<true><<<gs::kOrderBlocks, 1024, 0, s>>>(nullptr, nullptr, o->tile_last.as<uint32_t>(), nitems,
                                                o->ws_order_b.as<uint32_t>(), q);
     NPS_CHECK_LAUNCH();
 #define NPS_BWD_WS(TS, PPT, SB)                                                                                \
@@ -2796,7 +2797,7 @@ static int launch_bwd_raster(nps_gs* o, int form, int ppt, int stage, const floa
   if (form == 2) {
     NPS_TRY(ensure_ws_buffers(o, nitems));
     uint32_t* q = o->ws_q.as<uint32_t>() + 2;
-    gs::k_order_items<true><<<1, 1024, 0, s>>>(nullptr, nullptr, o->tile_last.as<uint32_t>(), nitems,
+    gs::k_order_items<true><<<gs::kOrderBlocks, 1024, 0, s>>>(nullptr, nullptr, o->tile_last.as<uint32_t>(), nitems,
                                                o->ws_order_b.as<uint32_t>(), q);
     NPS_CHECK_LAUNCH();
 #define NPS_BWD2O(PPT, SPS)                                                                                   \

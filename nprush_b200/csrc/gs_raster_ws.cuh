@@ -80,48 +80,74 @@ __device__ __forceinline__ uint32_t ws_length_class(uint32_t len) {
 
 // Orders the work items longest first (by length class; within a class in
 // no particular order, which does not change any result) into order[] and
-// resets the queue: qctl[0] = items queued, qctl[1] = 0 (the head).  One CTA.
+// resets the queue: qctl[0] = items queued, qctl[1] = 0 (the head).
 // kBwd: the length is the tile's last contributor over its pixels (from the
 // forward), and tiles without contributors are left out; otherwise the tile
 // list's length.
+// One cluster: each block counts the classes of its share, reads the others' counts
+// through distributed shared memory and places its share.  The few classes that
+// most items have would serialise the counters, so a warp counts each of its
+// classes once.  (One block without that: 21 + 16 us at 20,000 items, forward + backward,
+// and 73 + 47 us at 65,280; this: 7 + 7 and 12 + 11 us.)
+constexpr uint32_t kOrderBlocks = 8;
 template <bool kBwd>
-__global__ void __launch_bounds__(1024) k_order_items(const uint32_t* __restrict__ rstart,
-                                                      const uint32_t* __restrict__ rend,
-                                                      const uint32_t* __restrict__ tile_last, uint32_t nitems,
-                                                      uint32_t* __restrict__ order, uint32_t* __restrict__ qctl) {
+__global__ void __cluster_dims__(kOrderBlocks, 1, 1) __launch_bounds__(1024)
+    k_order_items(const uint32_t* __restrict__ rstart, const uint32_t* __restrict__ rend,
+                  const uint32_t* __restrict__ tile_last, uint32_t nitems, uint32_t* __restrict__ order,
+                  uint32_t* __restrict__ qctl) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
   __shared__ uint32_t hist[64];
   __shared__ uint32_t offs[64];
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, rank = cluster.block_rank();
   if (tid < 64) hist[tid] = 0;
   __syncthreads();
-  for (uint32_t it = tid; it < nitems; it += blockDim.x) {
+  // whole warps, so that every lane takes part in the votes; 64: no item
+  const uint32_t end = (nitems + 31u) & ~31u, stride = kOrderBlocks * 1024u;
+  auto length_class = [&](uint32_t it) {
+    if (it >= nitems) return 64u;
     const uint32_t len = kBwd ? tile_last[it] : rend[it] - rstart[it];
-    if (kBwd && len == 0) continue;
-    atomicAdd(&hist[ws_length_class(len)], 1u);
+    return kBwd && len == 0 ? 64u : ws_length_class(len);
+  };
+  for (uint32_t it = rank * 1024u + tid; it < end; it += stride) {
+    const uint32_t c = length_class(it), same = __match_any_sync(0xffffffffu, c);
+    if (c < 64u && lane == (uint32_t)__ffs(same) - 1u) atomicAdd(&hist[c], (uint32_t)__popc(same));
   }
-  __syncthreads();
+  cluster.sync();
   if (tid < 32) {
-    // exclusive scan of 64 counts, two per lane
-    const uint32_t a = hist[2 * tid], b = hist[2 * tid + 1];
-    uint32_t inc = a + b;
+    // exclusive scan of 64 counts, two per lane, and the counts of the blocks before this one
+    uint32_t n[2] = {0, 0}, before[2] = {0, 0};
+    for (uint32_t r = 0; r < kOrderBlocks; ++r) {
+      const uint32_t* h = cluster.map_shared_rank(hist, r);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t x = h[2 * tid + k];
+        n[k] += x;
+        if (r < rank) before[k] += x;
+      }
+    }
+    uint32_t inc = n[0] + n[1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
       if ((int)tid >= o) inc += y;
     }
-    const uint32_t ex = inc - a - b;
-    offs[2 * tid] = ex;
-    offs[2 * tid + 1] = ex + a;
-    if (tid == 31) {
+    const uint32_t ex = inc - n[0] - n[1];
+    offs[2 * tid] = ex + before[0];
+    offs[2 * tid + 1] = ex + n[0] + before[1];
+    if (rank == 0 && tid == 31) {
       qctl[0] = inc;
       qctl[1] = 0u;
     }
   }
-  __syncthreads();
-  for (uint32_t it = tid; it < nitems; it += blockDim.x) {
-    const uint32_t len = kBwd ? tile_last[it] : rend[it] - rstart[it];
-    if (kBwd && len == 0) continue;
-    order[atomicAdd(&offs[ws_length_class(len)], 1u)] = it;
+  cluster.sync();  // the offsets are ready, and no block leaves while its counts are read
+  for (uint32_t it = rank * 1024u + tid; it < end; it += stride) {
+    const uint32_t c = length_class(it), same = __match_any_sync(0xffffffffu, c);
+    const int first = __ffs(same) - 1;
+    uint32_t at = 0;
+    if (c < 64u && (int)lane == first) at = atomicAdd(&offs[c], (uint32_t)__popc(same));
+    at = __shfl_sync(0xffffffffu, at, first) + (uint32_t)__popc(same & ((1u << lane) - 1u));
+    if (c < 64u) order[at] = it;
   }
 }
 

@@ -369,6 +369,29 @@ def test_default_raster_follows_the_grid_size(trainer_cls, w, h, views):
     assert np.linalg.norm(out[0][1] - out[1][1]) / np.linalg.norm(out[1][1]) < 1e-5
 
 
+@pytest.mark.parametrize("w,h,views", [(16, 16, 1), (31 * 16, 16, 1), (33 * 16, 16, 1), (1024, 2048, 1), (1040, 2048, 1),
+                                       (700, 900, 4)])
+def test_ordered_items_are_all_drawn(trainer_cls, w, h, views):
+    """Longest-first order of 1, 31, 33, 8192, 8320 and 10032 items (around a warp
+    and one round of the ordering blocks): every tile drawn once, so the images are
+    those of the plain grid (1e-6 as between any two variants) and the gradients
+    agree (1e-5 relative L2)."""
+    p = gs_scene(400, 91, deg=0, log_scale_mean=-2.6)
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0), (-2.0, 0.5, 3.0), (0.5, -2.0, 3.5))[:views])
+    t = trainer_cls(400, sh_degree=0, params=p)
+    t.set_targets(gs_targets(views, w, h, 92))
+    out = []
+    for form in (0, 2):
+        t.set_raster((form, 2, 128), (form, 2, 128))
+        t.set_views(vp, vpi)
+        t.forward()
+        t.loss()
+        t.backward()
+        out.append((t.read_image(with_grad=False)[0], t.read_state()["grads"].astype(np.float64)))
+    np.testing.assert_allclose(out[0][0], out[1][0], atol=1e-6, rtol=0)
+    assert np.linalg.norm(out[0][1] - out[1][1]) / np.linalg.norm(out[0][1]) < 1e-5
+
+
 def test_raster_variants_agree_and_autotune(trainer_cls, tmp_path):
     """Forward images agree across tile sizes (8, 16, 32) and the raster
     variants of both forms (one CTA per tile; persistent warp-specialised)
