@@ -424,8 +424,14 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
   return at;
 }
 
+// Whether a bounded wait gave up since the last step or report (st: the step
+// state, see k_adam_prep).  What a sort or an emission then left unwritten may
+// hold any key and any record.
+__device__ __forceinline__ bool wait_gave_up(const volatile uint32_t* st) { return st[6] != st[7]; }
+
 // Writes the pairs of the depth-sorted (view, Gaussian) entries in their order,
-// positions beyond cap dropped, and their number to *total: one kernel
+// positions beyond cap dropped, their number to total[0] and to total[1] how many
+// of them the tile lists are made of (none after a wait that gave up): one kernel
 // gathers the entries' records, scans their counts and emits (instead of a
 // gather, three scan kernels, a host round trip for the total and an emit that
 // gathers again; with the clears in one launch, the status written by Adam's
@@ -444,16 +450,18 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
 //
 // Status words as in the sort (flag and 32-bit count), cleared beforehand.  The
 // look-back is bounded: after spin_limit polls of an unpublished tile the
-// block counts a timeout in *err and carries on; positions stay below cap.
-// host (page-locked, may be null) gets the total and *err for the host.
+// block counts a timeout (in st[6]) and carries on; positions stay below cap.  A
+// depth sort that gave up leaves places of sorted_g unwritten: an id of no
+// record (m or more) is an entry without pairs.
+// host (page-locked, may be null) gets the total and the timeouts for the host.
 constexpr uint32_t kBinTile = 1024;
 __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
                                                   uint32_t m, uint32_t n, uint32_t tiles_x, uint32_t num_tiles,
                                                   uint32_t cap, uint32_t* __restrict__ keys,
                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ total,
                                                   unsigned long long* __restrict__ status,
-                                                  uint32_t* __restrict__ counter, uint32_t* __restrict__ err,
-                                                  uint32_t spin_limit, volatile uint32_t* host) {
+                                                  uint32_t* __restrict__ counter, uint32_t* st, uint32_t spin_limit,
+                                                  volatile uint32_t* host) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32;
   __shared__ uint32_t s_tile, s_excl, s_warp[8];
@@ -472,14 +480,27 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
     if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
-    if (tile >= tiles) return;
+    if (tile >= tiles) {
+      // the last block to leave: every tile is emitted, every timeout counted
+      if (tile == tiles + gridDim.x - 1 && threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t sum = (uint32_t)load_status(tiles - 1);
+        total[0] = sum;
+        total[1] = wait_gave_up(st) ? 0u : min(sum, cap);
+        if (host) {
+          host[0] = sum;
+          host[1] = *(volatile uint32_t*)(st + 6);
+        }
+      }
+      return;
+    }
     const uint32_t first = tile * kBinTile + warp * 128u + lane;
     uint32_t g[4], off[4];
     uint4 b[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) g[q] = first + 32 * q < m ? sorted_g[first + 32 * q] : 0u;
+    for (int q = 0; q < 4; ++q) g[q] = first + 32 * q < m ? sorted_g[first + 32 * q] : 0xffffffffu;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) b[q] = first + 32 * q < m ? bins[g[q]] : make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < 4; ++q) b[q] = g[q] < m ? bins[g[q]] : make_uint4(0u, 0u, 0u, 0u);
     uint32_t run = 0;  // pairs of the warp's entries so far
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -513,7 +534,10 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
           const uint32_t take = inc ? inc ^ (inc - 1u) : kFull;  // up to the nearest inclusive prefix
           if (none & take) {
             if (++polls > spin_limit) {
-              if (lane == 0) atomicAdd(err, 1u);
+              if (lane == 0) {
+                atomicAdd(st + 6, 1u);
+                __threadfence();  // before this block's last claim (see above)
+              }
               break;
             }
             continue;
@@ -526,13 +550,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
       }
       if (lane == 0) {
         s_excl = excl;
-        if (tile == tiles - 1) {
-          *total = excl + sum;
-          if (host) {
-            host[0] = excl + sum;
-            host[1] = *(volatile uint32_t*)err;
-          }
-        }
+        if (tile == tiles - 1) __threadfence();
       }
     }
     __syncthreads();
@@ -592,10 +610,14 @@ __global__ void __launch_bounds__(256) k_clear(ClearList c) {
 }
 
 // Four consecutive sorted keys per thread from one 16-byte load (the key
-// buffers are 256-byte aligned), with the neighbours on either side.
-__global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ total, uint32_t cap,
-                         uint32_t* __restrict__ rstart, uint32_t* __restrict__ rend) {
-  const uint32_t K = min(*total, cap);
+// buffers are 256-byte aligned), with the neighbours on either side.  After a
+// wait that gave up every tile's list stays empty, so that no raster follows a
+// key or a record that was never written (the call reports NPS_ERR_TIMEOUT).
+__global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ count, uint32_t cap,
+                         const uint32_t* __restrict__ st, uint32_t* __restrict__ rstart,
+                         uint32_t* __restrict__ rend) {
+  if (wait_gave_up(st)) return;
+  const uint32_t K = min(*count, cap);
   const uint32_t n4 = (K + 3) / 4;
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x) {
     const uint32_t p0 = 4 * q;
@@ -1635,10 +1657,12 @@ __global__ void k_det_prep(const uint32_t* __restrict__ sorted_vals, const uint3
   }
 }
 
-// deterministic mode: each record's pair sums added in sorted-pair order
+// deterministic mode: each record's pair sums added in sorted-pair order (none
+// after a wait that gave up: the records and positions may be unwritten)
 __global__ void k_det_segsum(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pos,
-                             const uint32_t* __restrict__ total, uint32_t cap, const float* __restrict__ part,
-                             float* __restrict__ g2) {
+                             const uint32_t* __restrict__ total, uint32_t cap, const uint32_t* __restrict__ st,
+                             const float* __restrict__ part, float* __restrict__ g2) {
+  if (wait_gave_up(st)) return;
   const uint32_t K = min(*total, cap);
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < K; p += gridDim.x * blockDim.x) {
     const uint32_t k = keys[p];
@@ -2871,7 +2895,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
   uint32_t* rstart = o->ranges.as<uint32_t>();
   uint32_t* rend = rstart + nitems;
   uint32_t* total = o->total.as<uint32_t>();
-  uint32_t* err = o->stepst.as<uint32_t>() + 6;
+  uint32_t* st = o->stepst.as<uint32_t>();
   int bits = 1;
   while ((1ull << bits) < (uint64_t)nitems) ++bits;
   void *dclear = nullptr, *tclear = nullptr;
@@ -2938,16 +2962,16 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
       gs::k_bin_emit<<<std::min<uint32_t>(bin_tiles, 8u * kNumSMs), 256, 0, s>>>(
           dv, o->bins.as<uint4>(), (uint32_t)M, n, tiles_x, num_tiles, cap, o->keys.as<uint32_t>(),
           o->vals.as<uint32_t>(), total, reinterpret_cast<unsigned long long*>(o->bin_status.as<char>() + 16),
-          o->bin_status.as<uint32_t>(), err, o->sw_tile.spin_limit, capture ? nullptr : o->h_fwd);
+          o->bin_status.as<uint32_t>(), st, o->sw_tile.spin_limit, capture ? nullptr : o->h_fwd);
       NPS_CHECK_LAUNCH(); }
       if (!capture) NPS_CUDA(cudaEventRecord(o->fwd_counted, s));
       if (cap > 0) {
         uint32_t *ks = nullptr, *vv = nullptr;
         { StageTimer t(o, ST_TSORT);
-        NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total, cap, bits, o->sw_tile, s, &ks,
-                               &vv, false, cleared && tbytes > 0)); }
+        NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total + 1, cap, bits, o->sw_tile, s,
+                               &ks, &vv, false, cleared && tbytes > 0)); }
         { StageTimer t(o, ST_RANGES);
-        gs::k_ranges<<<std::min(16u * kNumSMs, div_up(cap, 1024)), 256, 0, s>>>(ks, total, cap, rstart, rend);
+        gs::k_ranges<<<std::min(16u * kNumSMs, div_up(cap, 1024)), 256, 0, s>>>(ks, total + 1, cap, st, rstart, rend);
         NPS_CHECK_LAUNCH(); }
         vs = vv;
       }
@@ -2966,7 +2990,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     if (tmo != o->timeouts_seen) {
       // reported here: the next Adam step must not skip for it again
       o->timeouts_seen = tmo;
-      k_set_u32<<<1, 1, 0, s>>>(o->stepst.as<uint32_t>() + 7, tmo);
+      k_set_u32<<<1, 1, 0, s>>>(st + 7, tmo);
       o->fwd_valid = o->loss_valid = false;
       set_error("gs_forward: a bounded device wait (sort look-back or raster staging) gave up in this or an "
                 "earlier call; its results were incomplete and no update used them");
@@ -2976,9 +3000,6 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     const uint32_t want = K + K / 4 + 4096;
     NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)want));
     NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)want));
-    // slots that an emission which gave up waiting leaves unwritten hold valid keys and records
-    NPS_CUDA(cudaMemsetAsync(o->keys.p, 0, sizeof(uint32_t) * (size_t)want, s));
-    NPS_CUDA(cudaMemsetAsync(o->vals.p, 0, sizeof(uint32_t) * (size_t)want, s));
     o->pair_cap = want;
   }
   o->K = K;
@@ -3110,7 +3131,7 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
         o->recs.as<gs::Rec>(), o->sorted_vals, rstart, rend, W, H, tiles_x, num_tiles, bg, o->img.as<float4>(),
         o->ncontrib.as<uint32_t>(), dimg, nullptr, o->det_part.as<float>());
     NPS_CHECK_LAUNCH();
-    const uint32_t* total = o->total.as<uint32_t>();
+    const uint32_t* total = o->total.as<uint32_t>() + 1;  // the pairs that the lists are made of
     gs::k_det_prep<<<4 * kNumSMs, 256, 0, s>>>(o->sorted_vals, total, cap, o->det_keys.as<uint32_t>(),
                                                o->det_pos.as<uint32_t>());
     NPS_CHECK_LAUNCH();
@@ -3119,7 +3140,8 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
     uint32_t *ko = nullptr, *vo = nullptr;
     NPS_TRY(radix_sort_u32(o->det_keys.as<uint32_t>(), o->det_pos.as<uint32_t>(), total, cap, bits, o->sw_det, s,
                            &ko, &vo));
-    gs::k_det_segsum<<<4 * kNumSMs, 256, 0, s>>>(ko, vo, total, cap, o->det_part.as<float>(), o->g2.as<float>());
+    gs::k_det_segsum<<<4 * kNumSMs, 256, 0, s>>>(ko, vo, total, cap, o->stepst.as<uint32_t>(), o->det_part.as<float>(),
+                                                 o->g2.as<float>());
     NPS_CHECK_LAUNCH();
   }
   if (n > 0) {

@@ -569,3 +569,47 @@ def test_sort_lookback_timeout_is_reported(trainer_cls):
             t.train_step()
         runs.append(t.read_state()["params"])
     np.testing.assert_array_equal(runs[0], runs[1])
+
+
+@pytest.mark.parametrize("deterministic", [True, False])
+def test_lookback_timeout_with_pair_buffers_from_earlier_calls(trainer_cls, deterministic):
+    """A depth sort that gives up (as above) on more records than any call before
+    had, with pair buffers that an earlier call sized: the ids that it leaves
+    unwritten are in memory that no call has written.  Each call reports it once, no
+    parameter moves, and the next forward and backward are those of a fresh trainer
+    (images bit for bit; gradients too in deterministic mode, else to 1e-5 relative
+    L2, the bound between two raster variants)."""
+    from nprush_b200._lib import NpsError
+    n, w, h = 20000, 256, 256
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0), (-2.0, 0.5, 3.0), (0.5, -2.0, 3.5)))
+    tg = gs_targets(4, w, h, 104)
+    ids = np.arange(4, dtype=np.uint32)
+    t = trainer_cls(n, sh_degree=0, params=gs_scene(n, 103, deg=0, log_scale_mean=-3.5))
+    t.set_deterministic(deterministic)
+    t.set_targets(tg)
+    t.set_views(vp[:1], vpi[:1], ids[:1])
+    t.train_step()
+    params = t.read_state()["params"]
+    t.set_views(vp, vpi, ids)
+    t.set_sort_guard(1000, 2)
+    for call in (t.train_step, t.forward):
+        with pytest.raises(NpsError) as e:
+            call()
+        assert e.value.code == -5
+    t.set_sort_guard()
+    fresh = trainer_cls(n, sh_degree=0, params=params)
+    fresh.set_deterministic(deterministic)
+    fresh.set_targets(tg)
+    fresh.set_views(vp, vpi, ids)
+    for u in (t, fresh):
+        u.forward()
+        u.loss()
+        u.backward()
+    np.testing.assert_array_equal(t.read_image(with_grad=False)[0], fresh.read_image(with_grad=False)[0])
+    s0, s1 = t.read_state(), fresh.read_state()
+    np.testing.assert_array_equal(s0["params"], params)
+    if deterministic:
+        np.testing.assert_array_equal(s0["grads"], s1["grads"])
+    else:
+        d = s0["grads"].astype(np.float64) - s1["grads"]
+        assert np.linalg.norm(d) / np.linalg.norm(s1["grads"].astype(np.float64)) < 1e-5
