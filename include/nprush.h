@@ -308,8 +308,9 @@ int nps_gs_backward(nps_gs* gs, const float* dl_dimage_device);
 int nps_gs_backward_host(nps_gs* gs, const float* dl_dimage_host);
 int nps_gs_adam(nps_gs* gs);
 /* forward + loss + backward + Adam.  In graph mode the first call (and any
- * call after the step's shape changed: Gaussian count, views, image size,
- * targets) runs eagerly to size every buffer and then captures the whole
+ * call after the step changed: Gaussian count, views, image size, targets,
+ * an option, a learning rate, the background, or a buffer that an eager call
+ * in between replaced) runs eagerly to size every buffer and then captures the whole
  * step as one CUDA graph; later calls replay it with no host synchronisation
  * inside the step.  A replay whose tile pairs exceed the captured capacity
  * (25% above the capturing step's) skips its parameter update; the next call

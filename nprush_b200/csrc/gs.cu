@@ -32,6 +32,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -2242,8 +2243,9 @@ struct nps_gs {
   uint32_t* h_fwd = nullptr;     // pinned: pair count and timeouts of the last eager forward
   cudaEvent_t fwd_counted = nullptr;
   bool g2_cleared = false;       // the forward cleared the backward's accumulators too
-  uint64_t gkey = 0;
-  uint32_t gcap = 0, skipped = 0;
+  std::array<uint64_t, 96> gkey{};  // what the captured step holds by value (step_key)
+  bool gvalid = false;              // the captured step may be replayed while its key is the current one
+  uint32_t skipped = 0;
   uint32_t graph_kernels = 0;  // kernel nodes of the captured step (launches per replay)
   uint32_t timeouts_seen = 0;  // bounded-wait timeouts already reported (device counter stepst[6])
   // optional per-stage timing with CUDA events on the context stream
@@ -3297,8 +3299,40 @@ static int gs_capture(nps_gs* o) {
     set_error("graph instantiate failed: %s", cudaGetErrorString(ie));
     return NPS_ERR_CUDA;
   }
-  o->gcap = o->pair_cap;
   return NPS_OK;
+}
+
+// What a captured step holds by value: sizes, options, learning rates and the
+// address of every buffer that its kernels use.  An eager call with more views,
+// pairs or Gaussians between two replays frees and replaces buffers, a call
+// that sets an option changes what the step computes: either makes another key.
+static decltype(nps_gs::gkey) step_key(const nps_gs* o) {
+  decltype(nps_gs::gkey) key{};
+  size_t at = 0;
+  auto num = [&](uint64_t v) { key[at++] = v; };
+  auto flt = [&](float f) { num(__builtin_bit_cast(uint32_t, f)); };
+  auto ptr = [&](const void* p) { num((uint64_t)(uintptr_t)p); };
+  for (uint32_t v : {o->n, o->nv, o->w, o->h, o->loss_views, o->tile, o->pair_cap}) num(v);
+  for (int v : {o->sh_deg, o->loss_kind, o->fwd_form, o->fwd_ppt, o->fwd_stage, o->bwd_form, o->bwd_ppt, o->bwd_stage})
+    num((uint64_t)v);
+  for (bool v : {o->accumulate, o->deterministic, o->raster_auto}) num(v);
+  flt(o->lambda);
+  for (float f : o->bg) flt(f);
+  for (float f : o->lr) flt(f);
+  ptr(o->tgt);
+  ptr(o->h_status);
+  for (const DevBuf* b :
+       {&o->params, &o->grads, &o->am, &o->av, &o->adc_grad, &o->adc_denom, &o->stepst, &o->views, &o->recs, &o->counts,
+        &o->bins, &o->dkeys, &o->dvals, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->bin_status, &o->img,
+        &o->ncontrib, &o->maps, &o->partial, &o->loss, &o->dimg, &o->g2, &o->tile_last, &o->ws_order_f, &o->ws_order_b,
+        &o->ws_q, &o->det_part, &o->det_keys, &o->det_pos})
+    ptr(b->p);
+  for (const SortWork* w : {&o->sw_depth, &o->sw_tile, &o->sw_det}) {
+    for (const DevBuf* b : {&w->partial, &w->lookback, &w->keys_alt, &w->vals_alt}) ptr(b->p);
+    num(w->spin_limit);
+    num(w->stall_tile);
+  }
+  return key;
 }
 
 extern "C" {
@@ -3320,10 +3354,6 @@ int nps_gs_train_step(nps_gs* o, float* loss3_host) {
   if (!o->graph_mode) {
     NPS_TRY(gs_step_eager(o));
   } else {
-    // shape of the captured step; anything else in it reads device memory
-    const uint64_t key = ((uint64_t)o->n * 1000003ull) ^ ((uint64_t)o->nv << 40) ^ ((uint64_t)o->w << 20) ^
-                         ((uint64_t)o->h << 4) ^ (uint64_t)o->sh_deg ^ ((uint64_t)(uintptr_t)o->tgt << 7) ^
-                         ((uint64_t)__builtin_bit_cast(uint32_t, o->bg[0]) << 3) ^ (uint64_t)o->lambda * 131ull;
     if (o->gexec) {
       // at most two replays in flight (one while stage timers are read, since
       // their event nodes are shared by all replays)
@@ -3334,7 +3364,7 @@ int nps_gs_train_step(nps_gs* o, float* loss3_host) {
         // a replay overflowed its pair buffers and skipped its update
         o->skipped += sk - o->skip_seen;
         o->skip_seen = sk;
-        o->gkey = 0;
+        o->gvalid = false;
       }
       if (o->h_status[2] != o->timeouts_seen) {
         o->timeouts_seen = o->h_status[2];
@@ -3343,7 +3373,7 @@ int nps_gs_train_step(nps_gs* o, float* loss3_host) {
         return NPS_ERR_TIMEOUT;
       }
     }
-    if (!o->gexec || key != o->gkey) {
+    if (!o->gexec || !o->gvalid || step_key(o) != o->gkey) {
       NPS_TRY(collect_graph_timers(o));
       NPS_TRY(gs_step_eager(o));  // sizes every buffer (and is this call's step)
       NPS_TRY(gs_capture(o));
@@ -3351,7 +3381,8 @@ int nps_gs_train_step(nps_gs* o, float* loss3_host) {
       o->skip_seen = o->h_status[1] = 0;
       o->h_status[2] = o->timeouts_seen;  // what the replays report until a wait gives up
       NPS_CUDA(cudaMemsetAsync(o->stepst.as<uint32_t>() + 4, 0, sizeof(uint32_t), s));
-      o->gkey = key;
+      o->gkey = step_key(o);
+      o->gvalid = true;
     } else {
       NPS_CUDA(cudaGraphLaunch(o->gexec, s));
       std::swap(o->gdone, o->gprev);
@@ -3453,7 +3484,7 @@ int adc_apply(nps_gs* o, const gs::AdcParams& a, uint32_t* counts4) {
   std::swap(o->params, o->p_alt);
   std::swap(o->am, o->m_alt);
   std::swap(o->av, o->v_alt);
-  o->gkey = 0;  // a captured step holds the old buffers and count
+  o->gvalid = false;  // a captured step holds the old buffers and count
   NPS_CUDA(cudaMemsetAsync(o->adc_grad.p, 0, sizeof(float) * o->cap, s));
   NPS_CUDA(cudaMemsetAsync(o->adc_denom.p, 0, sizeof(float) * o->cap, s));
   if (counts4) {
@@ -3679,7 +3710,7 @@ int nps_gs_load(nps_gs* o, const char* path) {
   o->timeouts_seen = 0;
   o->loss_kind = h.reserved[0] <= (uint32_t)gs::kLossL2 ? (int)h.reserved[0] : gs::kLossL1Dssim;
   o->fwd_valid = o->loss_valid = false;
-  o->gkey = 0;
+  o->gvalid = false;
   o->skip_seen = 0;
   if (o->h_status) o->h_status[1] = o->h_status[2] = 0;
   return NPS_OK;
@@ -3704,7 +3735,7 @@ int nps_gs_set_raster(nps_gs* o, int fwd_form, int fwd_ppt, int fwd_stage, int b
   o->bwd_form = bwd_form;
   o->bwd_ppt = bwd_ppt;
   o->bwd_stage = bwd_stage;
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -3732,7 +3763,7 @@ int nps_gs_set_tile(nps_gs* o, uint32_t tile) {
   if (!valid_variant(tile, o->bwd_form, o->bwd_ppt, o->bwd_stage))
     o->bwd_form = def.form, o->bwd_ppt = def.ppt, o->bwd_stage = def.stage;
   o->fwd_valid = o->loss_valid = false;
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -3821,7 +3852,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
         }
       std::fclose(f);
       if (found) {
-        o->gkey = 0;
+        o->gvalid = false;
         o->fwd_valid = o->loss_valid = false;
         return report(false);
       }
@@ -3893,7 +3924,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
   o->fwd_form = best_pick[0].form, o->fwd_ppt = best_pick[0].ppt, o->fwd_stage = best_pick[0].stage;
   o->bwd_form = best_pick[1].form, o->bwd_ppt = best_pick[1].ppt, o->bwd_stage = best_pick[1].stage;
   o->fwd_valid = o->loss_valid = false;
-  o->gkey = 0;
+  o->gvalid = false;
   NPS_TRY(rc);
   NPS_TRY(report(true));
   if (cache_path) {
@@ -3932,7 +3963,7 @@ int nps_gs_set_loss(nps_gs* o, int kind, float ssim_weight) {
   o->loss_kind = kind;
   o->lambda = ssim_weight;
   o->loss_valid = false;
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -3942,7 +3973,7 @@ int nps_gs_set_sort_guard(nps_gs* o, uint32_t spin_limit, uint32_t stall_tile) {
     w->spin_limit = spin_limit ? spin_limit : (1u << 20);
     w->stall_tile = stall_tile;
   }
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -3950,7 +3981,7 @@ int nps_gs_set_deterministic(nps_gs* o, int enable) {
   NPS_TRY(check_gs(o));
   if (enable && o->tile != 16) NPS_TRY(nps_gs_set_tile(o, 16));  // the two-pass backward's tiles
   o->deterministic = enable != 0;
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -3958,7 +3989,7 @@ int nps_gs_set_accumulate(nps_gs* o, int accumulate, uint32_t loss_views) {
   NPS_TRY(check_gs(o));
   o->accumulate = accumulate != 0;
   o->loss_views = loss_views;
-  o->gkey = 0;
+  o->gvalid = false;
   return NPS_OK;
 }
 
@@ -4010,7 +4041,7 @@ int nps_gs_stats(nps_gs* o, nps_stats* out) {
     if (sk != o->skip_seen) {
       o->skipped += sk - o->skip_seen;
       o->skip_seen = sk;
-      o->gkey = 0;
+      o->gvalid = false;
     }
     o->stats.reserved[1] = o->skipped;
   }

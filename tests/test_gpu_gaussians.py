@@ -613,3 +613,53 @@ def test_lookback_timeout_with_pair_buffers_from_earlier_calls(trainer_cls, dete
     else:
         d = s0["grads"].astype(np.float64) - s1["grads"]
         assert np.linalg.norm(d) / np.linalg.norm(s1["grads"].astype(np.float64)) < 1e-5
+
+
+@pytest.mark.parametrize("between", ["more_views", "more_pairs", "more_gaussians", "background", "learning_rates", "loss"])
+def test_captured_step_after_eager_calls(trainer_cls, between):
+    """Calls between two captured steps that make the trainer replace buffers (a
+    forward of more views, of larger Gaussians, of more Gaussians) or that set what
+    the step holds by value (a colour of the background, learning rates, the weight
+    of the structural term): the steps after them are those of an eager trainer that
+    made the same calls, bit for bit (deterministic mode)."""
+    n, w, h = 6000, 160, 128
+    p = gs_scene(n, 105, deg=1, log_scale_mean=-3.5)
+    eyes = [(4.0 * np.cos(a), 0.5, 4.0 * np.sin(a)) for a in np.linspace(0.0, 5.5, 24)]
+    vp, vpi, _ = gs_views(w, h, eyes)
+    tg = gs_targets(24, w, h, 106)
+    ids = np.arange(24, dtype=np.uint32)
+    runs = []
+    for graph in (True, False):
+        t = trainer_cls(2 * n, sh_degree=1, params=p)
+        t.set_deterministic(True)
+        t.set_graph(graph)
+        t.set_targets(tg)
+        t.set_views(vp[:2], vpi[:2], ids[:2])
+        for _ in range(3):
+            t.train_step()
+        if between == "more_views":
+            t.set_views(vp, vpi, ids)
+            t.forward()
+            t.set_views(vp[:2], vpi[:2], ids[:2])
+        elif between in ("more_pairs", "more_gaussians"):
+            q = t.read_state()["params"][:n]
+            large = q.copy()
+            large[:, 3:6] += 1.5
+            if between == "more_pairs":
+                t.write_params(large)
+                t.forward()
+                t.write_params(q)
+            else:
+                t.write_params(large, first=n)
+                t.forward()
+                t.set_count(n)
+        elif between == "background":
+            t.set_background((0.0, 0.5, 0.25))
+        elif between == "learning_rates":
+            t.set_lr(2.0 * np.asarray(t.LR_DEFAULT, np.float32))
+        else:
+            t.set_loss("l1_dssim", 0.203)
+        for _ in range(3):
+            t.train_step()
+        runs.append(t.read_state()["params"][:n])
+    np.testing.assert_array_equal(runs[0], runs[1])
