@@ -449,13 +449,15 @@ __device__ __forceinline__ bool wait_gave_up(const volatile uint32_t* st) { retu
 // entry's fields are one 16-byte word and its slots need no integer division
 // (84 -> 52 us at 11.5 M pairs).
 //
-// Status words as in the sort (flag and 32-bit count), cleared beforehand.  The
-// look-back is bounded: after spin_limit polls of an unpublished tile the
+// Counts stay at kMostPairs once they reach it, beyond any cap (a sort takes fewer
+// than 2^30 pairs), so that a scene whose pairs pass 2^32 is not mistaken for a small one
+// (a sum of 32 entries is at most 2^31: an image has at most 2^26 tiles).  Status words as in
+// the sort (flag and 32-bit count), cleared beforehand.  The look-back is bounded: after spin_limit polls of an unpublished tile the
 // block counts a timeout (in st[6]) and carries on; positions stay below cap.  A
 // depth sort that gave up leaves places of sorted_g unwritten: an id of no
 // record (m or more) is an entry without pairs.
 // host (page-locked, may be null) gets the total and the timeouts for the host.
-constexpr uint32_t kBinTile = 1024;
+constexpr uint32_t kBinTile = 1024, kMostPairs = 0x7fffffffu;
 __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
                                                   uint32_t m, uint32_t n, uint32_t tiles_x, uint32_t num_tiles,
                                                   uint32_t cap, uint32_t* __restrict__ keys,
@@ -511,16 +513,16 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         const uint32_t y = __shfl_up_sync(kFull, inc, o);
         if ((int)lane >= o) inc += y;
       }
-      off[q] = run + inc - b[q].w;
-      run += __shfl_sync(kFull, inc, 31);
+      off[q] = min(run + inc - b[q].w, kMostPairs);
+      run = min(run + __shfl_sync(kFull, inc, 31), kMostPairs);
     }
     if (lane == 0) s_warp[warp] = run;
     __syncthreads();
     uint32_t before = 0, sum = 0;
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k) {
-      before += k < warp ? s_warp[k] : 0u;
-      sum += s_warp[k];
+      before = min(before + (k < warp ? s_warp[k] : 0u), kMostPairs);
+      sum = min(sum + s_warp[k], kMostPairs);
     }
     if (warp == 0) {
       uint32_t excl = 0;
@@ -543,11 +545,13 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
             }
             continue;
           }
-          excl += __reduce_add_sync(kFull, (take >> lane) & 1u ? (uint32_t)w : 0u);
+          const uint32_t c = (take >> lane) & 1u ? (uint32_t)w : 0u;  // summed in halves: 32 counts pass 2^32
+          const uint32_t lo = __reduce_add_sync(kFull, c & 0xffffu), hi = __reduce_add_sync(kFull, c >> 16);
+          excl = (uint32_t)min(((unsigned long long)hi << 16) + lo + excl, (unsigned long long)kMostPairs);
           if (inc) break;
           j -= 32;
         }
-        if (lane == 0) store_status(tile, kInc | (uint32_t)(excl + sum));
+        if (lane == 0) store_status(tile, kInc | min(excl + sum, kMostPairs));
       }
       if (lane == 0) {
         s_excl = excl;
@@ -555,12 +559,12 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
       }
     }
     __syncthreads();
-    const uint32_t warp0 = s_excl + before;
+    const uint32_t warp0 = min(s_excl + before, kMostPairs);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const uint32_t start = warp0 + __shfl_sync(kFull, off[q], 0);
-      const uint32_t end = warp0 + __shfl_sync(kFull, off[q] + b[q].w, 31);
-      if (start == end) continue;
+      const uint32_t end = min(warp0 + __shfl_sync(kFull, off[q] + b[q].w, 31), cap);
+      if (start >= end) continue;  // no pairs, or all beyond cap (of which 32 entries end below 2^32)
       // per entry: first slot, tile mask (all ones: every tile), key of its first tile and row width
       const uint32_t o = warp0 + off[q], x0 = b[q].x & 0xffffu, w = max((b[q].x >> 16) - x0, 1u);
       const uint32_t tm = rect_tiles(b[q].x, b[q].y) <= 32u ? b[q].z : 0xffffffffu;
@@ -578,7 +582,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         const uint32_t kL = __shfl_sync(kFull, key0, L), wL = __shfl_sync(kFull, w, L);
         const uint32_t tmL = __shfl_sync(kFull, tm, L);
         const float iwL = __shfl_sync(kFull, iw, L);
-        if (sl < end && sl < cap) {
+        if (sl < end) {
           const uint32_t k = sl - oL;
           // the tile's index in the box: the k-th of the mask, or the k-th
           const uint32_t local = tmL != 0xffffffffu ? nth_set_bit(tmL, k) : k;
@@ -2950,8 +2954,8 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     NPS_TRY(radix_sort_u32(o->dkeys.as<uint32_t>(), o->dvals.as<uint32_t>(), o->mcount.as<uint32_t>(), (uint32_t)M, 32,
                            o->sw_depth, s, &dk, &dv, true, true)); }
   }
-  // The rest depends on the pair buffers' capacity: a second round only where
-  // the count came back larger (or there were no buffers yet).
+  // The rest depends on the pair buffers' capacity: a second round, the last, only
+  // where the count came back larger (or there were no buffers yet).
   for (int round = 0;; ++round) {
     const bool cleared = round == 0;
     const uint32_t cap = o->pair_cap;
@@ -2999,10 +3003,17 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
       return NPS_ERR_TIMEOUT;
     }
     if (cap > 0 && K <= cap) break;
-    const uint32_t want = K + K / 4 + 4096;
+    const uint64_t want = (uint64_t)K + K / 4 + 4096;
+    if (round > 0 || want >= (1ull << 30)) {
+      o->fwd_valid = o->loss_valid = false;
+      set_error("gs_forward: %u or more tile pairs do not fit the %u that the sort takes", K,
+                round > 0 ? cap : (1u << 30) - 1u);
+      return NPS_ERR_INVALID;
+    }
+    o->pair_cap = 0;  // until both buffers are there
     NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)want));
     NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)want));
-    o->pair_cap = want;
+    o->pair_cap = (uint32_t)want;
   }
   o->K = K;
   if (out_rgba) NPS_CUDA(cudaMemcpyAsync(out_rgba, o->img.p, sizeof(float4) * npix, cudaMemcpyDeviceToDevice, s));

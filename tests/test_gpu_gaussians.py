@@ -663,3 +663,37 @@ def test_captured_step_after_eager_calls(trainer_cls, between):
             t.train_step()
         runs.append(t.read_state()["params"][:n])
     np.testing.assert_array_equal(runs[0], runs[1])
+
+
+@pytest.mark.parametrize("n", [70_000, 180_000, 230_000])
+def test_more_pairs_than_a_sort_takes(trainer_cls, n):
+    """Gaussians that each cover all 2500 tiles of 8 views (a fit that diverges):
+    1.4e9, 3.6e9 and 4.6e9 pairs, where a 25% margin on the count, and then the count
+    itself, pass 2^32.  The forward reports that they are too many, with pair
+    buffers from an earlier scene and without, and the handle then renders a small
+    scene as a fresh one does."""
+    from nprush_b200._lib import NpsError
+    w = h = 800
+    eyes = [(4.0 * np.cos(a), 0.5, 4.0 * np.sin(a)) for a in np.linspace(0.0, 5.5, 8)]
+    vp, vpi, _ = gs_views(w, h, eyes)
+    huge = gs_scene(n, 107, deg=0, log_scale_mean=3.5)
+    small = gs_scene(500, 108, deg=0, log_scale_mean=-3.0)
+    t = trainer_cls(n, sh_degree=0, params=huge)
+    t.set_image_size(w, h)
+    t.set_views(vp, vpi)
+    imgs = []
+    for _ in range(2):
+        t.write_params(huge)
+        with pytest.raises(NpsError) as e:
+            t.forward()
+        assert e.value.code == -1  # NPS_ERR_INVALID
+        t.write_params(small)
+        t.set_count(500)
+        t.forward()
+        imgs.append(t.read_image(with_grad=False)[0])
+    u = trainer_cls(500, sh_degree=0, params=small)
+    u.set_image_size(w, h)
+    u.set_views(vp, vpi)
+    u.forward()
+    for img in imgs:
+        np.testing.assert_array_equal(img, u.read_image(with_grad=False)[0])
