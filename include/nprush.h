@@ -381,6 +381,9 @@ int nps_gs_autotune(nps_gs* gs, const char* cache_path, int* choice4, float* tim
  * status is treated as never published, which makes a look-back run out on a
  * normal input. */
 int nps_gs_set_sort_guard(nps_gs* gs, uint32_t spin_limit, uint32_t stall_tile);
+/* The same for the look-back of the pair emission between the two sorts, whose
+ * tiles are 1024 (view, Gaussian) records in depth order. */
+int nps_gs_set_bin_guard(nps_gs* gs, uint32_t spin_limit, uint32_t stall_tile);
 /* Deterministic mode: the backward reduces each (view, Gaussian) gradient in
  * two passes (per-pair tile sums stored, then summed per record in sorted-pair
  * order) instead of with float atomics, so repeated runs are bit-identical.

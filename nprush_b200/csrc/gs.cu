@@ -457,6 +457,7 @@ __device__ __forceinline__ bool wait_gave_up(const volatile uint32_t* st) { retu
 // depth sort that gave up leaves places of sorted_g unwritten: an id of no
 // record (m or more) is an entry without pairs.
 // host (page-locked, may be null) gets the total and the timeouts for the host.
+// stall_tile: see nps_gs_set_bin_guard.
 constexpr uint32_t kBinTile = 1024, kMostPairs = 0x7fffffffu;
 __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
                                                   uint32_t m, uint32_t n, uint32_t tiles_x, uint32_t num_tiles,
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ total,
                                                   unsigned long long* __restrict__ status,
                                                   uint32_t* __restrict__ counter, uint32_t* st, uint32_t spin_limit,
-                                                  volatile uint32_t* host) {
+                                                  uint32_t stall_tile, volatile uint32_t* host) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32;
   __shared__ uint32_t s_tile, s_excl, s_warp[8];
@@ -532,7 +533,8 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         if (lane == 0) store_status(tile, kAgg | sum);
         uint32_t j = tile, polls = 0;  // tiles below j are still to be added
         while (j > 0) {
-          const unsigned long long w = lane < j ? load_status(j - 1 - lane) : kInc;
+          unsigned long long w = lane < j ? load_status(j - 1 - lane) : kInc;
+          if (lane < j && j - 1 - lane == stall_tile) w = 0ull;
           const uint32_t inc = __ballot_sync(kFull, (w & kInc) != 0ull), none = __ballot_sync(kFull, (w >> 32) == 0ull);
           const uint32_t take = inc ? inc ^ (inc - 1u) : kFull;  // up to the nearest inclusive prefix
           if (none & take) {
@@ -2216,6 +2218,7 @@ struct nps_gs {
   // forward state
   DevBuf recs, counts, bins, dkeys, dvals, total, mcount, keys, vals, ranges;
   DevBuf bin_status;             // k_bin_emit: tile counter, then one status word per tile
+  uint32_t bin_spin = 1u << 20, bin_stall = 0xffffffffu;  // its look-back (nps_gs_set_bin_guard)
   DevBuf img, ncontrib;
   DevBuf maps, partial, loss, dimg, g2;
   SortWork sw_depth, sw_tile;
@@ -2968,7 +2971,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
       gs::k_bin_emit<<<std::min<uint32_t>(bin_tiles, 8u * kNumSMs), 256, 0, s>>>(
           dv, o->bins.as<uint4>(), (uint32_t)M, n, tiles_x, num_tiles, cap, o->keys.as<uint32_t>(),
           o->vals.as<uint32_t>(), total, reinterpret_cast<unsigned long long*>(o->bin_status.as<char>() + 16),
-          o->bin_status.as<uint32_t>(), st, o->sw_tile.spin_limit, capture ? nullptr : o->h_fwd);
+          o->bin_status.as<uint32_t>(), st, o->bin_spin, o->bin_stall, capture ? nullptr : o->h_fwd);
       NPS_CHECK_LAUNCH(); }
       if (!capture) NPS_CUDA(cudaEventRecord(o->fwd_counted, s));
       if (cap > 0) {
@@ -3327,6 +3330,8 @@ static decltype(nps_gs::gkey) step_key(const nps_gs* o) {
   for (int v : {o->sh_deg, o->loss_kind, o->fwd_form, o->fwd_ppt, o->fwd_stage, o->bwd_form, o->bwd_ppt, o->bwd_stage})
     num((uint64_t)v);
   for (bool v : {o->accumulate, o->deterministic, o->raster_auto}) num(v);
+  num(o->bin_spin);
+  num(o->bin_stall);
   flt(o->lambda);
   for (float f : o->bg) flt(f);
   for (float f : o->lr) flt(f);
@@ -3985,6 +3990,13 @@ int nps_gs_set_sort_guard(nps_gs* o, uint32_t spin_limit, uint32_t stall_tile) {
     w->stall_tile = stall_tile;
   }
   o->gvalid = false;
+  return NPS_OK;
+}
+
+int nps_gs_set_bin_guard(nps_gs* o, uint32_t spin_limit, uint32_t stall_tile) {
+  NPS_TRY(check_gs(o));
+  o->bin_spin = spin_limit ? spin_limit : (1u << 20);
+  o->bin_stall = stall_tile;
   return NPS_OK;
 }
 

@@ -240,6 +240,10 @@ class GaussianTrainer:
         (tests) is a tile whose status is treated as never published."""
         call("nps_gs_set_sort_guard", self._h, int(spin_limit), int(stall_tile))
 
+    def set_bin_guard(self, spin_limit: int = 0, stall_tile: int = 0xFFFFFFFF):
+        """The same for the look-back of the pair emission (tiles of 1024 records)."""
+        call("nps_gs_set_bin_guard", self._h, int(spin_limit), int(stall_tile))
+
     def set_deterministic(self, enable: bool):
         """Two-pass backward reduction without float atomics (bit-reproducible)."""
         call("nps_gs_set_deterministic", self._h, int(bool(enable)))

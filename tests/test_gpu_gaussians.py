@@ -572,10 +572,12 @@ def test_sort_lookback_timeout_is_reported(trainer_cls):
 
 
 @pytest.mark.parametrize("deterministic", [True, False])
-def test_lookback_timeout_with_pair_buffers_from_earlier_calls(trainer_cls, deterministic):
+@pytest.mark.parametrize("guard", ["set_sort_guard", "set_bin_guard"])
+def test_lookback_timeout_with_pair_buffers_from_earlier_calls(trainer_cls, guard, deterministic):
     """A depth sort that gives up (as above) on more records than any call before
     had, with pair buffers that an earlier call sized: the ids that it leaves
-    unwritten are in memory that no call has written.  Each call reports it once, no
+    unwritten are in memory that no call has written.  The same for the pair
+    emission (tile 2 of its tiles of 1024 records).  Each call reports it once, no
     parameter moves, and the next forward and backward are those of a fresh trainer
     (images bit for bit; gradients too in deterministic mode, else to 1e-5 relative
     L2, the bound between two raster variants)."""
@@ -591,12 +593,13 @@ def test_lookback_timeout_with_pair_buffers_from_earlier_calls(trainer_cls, dete
     t.train_step()
     params = t.read_state()["params"]
     t.set_views(vp, vpi, ids)
-    t.set_sort_guard(1000, 2)
+    getattr(t, guard)(1000, 2)
     for call in (t.train_step, t.forward):
+        before = t.stats()["staging_timeouts"]
         with pytest.raises(NpsError) as e:
             call()
-        assert e.value.code == -5
-    t.set_sort_guard()
+        assert e.value.code == -5 and t.stats()["staging_timeouts"] > before
+    getattr(t, guard)()
     fresh = trainer_cls(n, sh_degree=0, params=params)
     fresh.set_deterministic(deterministic)
     fresh.set_targets(tg)
