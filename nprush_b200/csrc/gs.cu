@@ -2999,6 +2999,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     if (tmo != o->timeouts_seen) {
       // reported here: the next Adam step must not skip for it again
       o->timeouts_seen = tmo;
+      if (o->h_status) o->h_status[2] = tmo;  // nor a captured step report it (none is in flight here)
       k_set_u32<<<1, 1, 0, s>>>(st + 7, tmo);
       o->fwd_valid = o->loss_valid = false;
       set_error("gs_forward: a bounded device wait (sort look-back or raster staging) gave up in this or an "

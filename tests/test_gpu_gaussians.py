@@ -700,3 +700,35 @@ def test_more_pairs_than_a_sort_takes(trainer_cls, n):
     u.forward()
     for img in imgs:
         np.testing.assert_array_equal(img, u.read_image(with_grad=False)[0])
+
+
+def test_emission_timeout_in_captured_steps(trainer_cls):
+    """The pair emission's look-back made to run out with captured steps: the call
+    that captures anew reports it and moves nothing, and later steps are those of a
+    trainer that never stalled, bit for bit (deterministic mode)."""
+    from nprush_b200._lib import NpsError
+    n, w, h = 8000, 128, 128
+    p = gs_scene(n, 109, deg=0, log_scale_mean=-3.5)
+    vp, vpi, _ = gs_views(w, h)
+    tg = gs_targets(1, w, h, 110)
+    runs = []
+    for stall in (True, False):
+        t = trainer_cls(n, sh_degree=0, params=p)
+        t.set_deterministic(True)
+        t.set_graph(True)
+        t.set_targets(tg)
+        t.set_views(vp, vpi)
+        for _ in range(3):
+            t.train_step()
+        if stall:
+            before = t.read_state()["params"]
+            t.set_bin_guard(1000, 2)
+            with pytest.raises(NpsError) as e:
+                t.train_step()
+            assert e.value.code == -5
+            np.testing.assert_array_equal(t.read_state()["params"], before)
+            t.set_bin_guard()
+        for _ in range(3):
+            t.train_step()
+        runs.append(t.read_state()["params"])
+    np.testing.assert_array_equal(runs[0], runs[1])
