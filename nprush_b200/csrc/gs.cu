@@ -432,7 +432,9 @@ __device__ __forceinline__ bool wait_gave_up(const volatile uint32_t* st) { retu
 
 // Writes the pairs of the depth-sorted (view, Gaussian) entries in their order,
 // positions beyond cap dropped, their number to total[0] and to total[1] how many
-// of them the tile lists are made of (none after a wait that gave up): one kernel
+// of them the tile lists are made of: none after a wait that gave up, and none beyond
+// cap where the host repeats the emission with larger buffers (host is not null), so
+// that the sort and the raster of a list cut short cost nothing; one kernel
 // gathers the entries' records, scans their counts and emits (instead of a
 // gather, three scan kernels, a host round trip for the total and an emit that
 // gathers again; with the clears in one launch, the status written by Adam's
@@ -481,19 +483,23 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
   };
   for (;;) {
     __syncthreads();  // the tile before is done with the shared words
-    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
+    if (threadIdx.x == 0)
+      asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], 1;" : "=r"(s_tile) : "l"(counter) : "memory");
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= tiles) {
-      // the last block to leave: every tile is emitted, every timeout counted
+      // the last block to leave: every tile is claimed and left, every timeout counted
       if (tile == tiles + gridDim.x - 1 && threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t sum = (uint32_t)load_status(tiles - 1);
+        const uint32_t gave_up = *(volatile uint32_t*)(st + 6);
+        const bool complete = !wait_gave_up(st);
+        unsigned long long w = load_status(tiles - 1);
+        for (uint32_t polls = 0; (w & kInc) == 0ull && polls < spin_limit; ++polls) w = load_status(tiles - 1);
+        const uint32_t sum = (uint32_t)w;
         total[0] = sum;
-        total[1] = wait_gave_up(st) ? 0u : min(sum, cap);
+        total[1] = !complete ? 0u : sum <= cap ? sum : host ? 0u : cap;
         if (host) {
           host[0] = sum;
-          host[1] = *(volatile uint32_t*)(st + 6);
+          host[1] = gave_up;
         }
       }
       return;
@@ -541,7 +547,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
             if (++polls > spin_limit) {
               if (lane == 0) {
                 atomicAdd(st + 6, 1u);
-                __threadfence();  // before this block's last claim (see above)
+                __threadfence();  // before this block's next claim, so that the last block sees it
               }
               break;
             }
@@ -555,10 +561,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         }
         if (lane == 0) store_status(tile, kInc | min(excl + sum, kMostPairs));
       }
-      if (lane == 0) {
-        s_excl = excl;
-        if (tile == tiles - 1) __threadfence();
-      }
+      if (lane == 0) s_excl = excl;
     }
     __syncthreads();
     const uint32_t warp0 = min(s_excl + before, kMostPairs);
@@ -2897,6 +2900,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
   NPS_TRY(o->img.ensure(sizeof(float4) * npix));
   NPS_TRY(o->ncontrib.ensure(sizeof(uint32_t) * npix));
   if (train) NPS_TRY(o->g2.ensure(sizeof(float) * gs::kG2 * (M + 1)));
+  // here and not in nps_gs_create: after set_views has page-locked its staging these words are 0.02 ms, before it 2.5 ms
   if (!capture && !o->h_fwd) {
     NPS_CUDA(cudaMallocHost((void**)&o->h_fwd, 16));
     NPS_CUDA(cudaEventCreateWithFlags(&o->fwd_counted, cudaEventDisableTiming));

@@ -732,3 +732,39 @@ def test_emission_timeout_in_captured_steps(trainer_cls):
             t.train_step()
         runs.append(t.read_state()["params"])
     np.testing.assert_array_equal(runs[0], runs[1])
+
+
+@pytest.mark.parametrize("n", [700, 9000, 60000])
+def test_forward_that_outgrows_its_pair_buffers(trainer_cls, n):
+    """Pairs that outgrow the buffers of an earlier scene (by more than the margin of
+    a quarter), for sorts of one block, of short tiles and of long ones: image, loss and
+    gradients of the repeated emission are those of a fresh handle (bit for bit in
+    deterministic mode), and so is a step that finds them outgrown."""
+    w, h = 400, 320
+    p = gs_scene(n, 111, deg=0, log_scale_mean=-4.5)
+    q = p.copy()
+    q[:, 3:6] += 2.0
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0)))
+    tg = gs_targets(2, w, h, 112)
+    out = []
+    for before, after in ((p, q), (q, q)):
+        for step in (False, True):
+            t = trainer_cls(n, sh_degree=0, params=before)
+            t.set_deterministic(True)
+            t.set_targets(tg)
+            t.set_views(vp, vpi)
+            t.forward()
+            pairs = t.stats()["pairs"]
+            t.write_params(after)
+            if step:
+                loss = t.train_step(read_loss=True)
+                out.append((loss, t.read_state()["params"]))
+            else:
+                t.forward()
+                loss = t.loss()
+                t.backward()
+                out.append((loss, t.read_image()[0], t.read_state()["grads"]))
+                assert before is q or t.stats()["pairs"] > 1.3 * pairs
+    for grown, fresh in ((out[0], out[2]), (out[1], out[3])):
+        for a, b in zip(grown, fresh):
+            np.testing.assert_array_equal(a, b)
