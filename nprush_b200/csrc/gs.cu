@@ -428,7 +428,7 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t k) {
 // Whether a bounded wait gave up since the last step or report (st: the step
 // state, see k_adam_prep).  What a sort or an emission then left unwritten may
 // hold any key and any record.
-__device__ __forceinline__ bool wait_gave_up(const volatile uint32_t* st) { return st[6] != st[7]; }
+__device__ __forceinline__ bool wait_gave_up(const uint32_t* st) { return __ldg(st + 6) != __ldg(st + 7); }
 
 // Writes the pairs of the depth-sorted (view, Gaussian) entries in their order,
 // positions beyond cap dropped, their number to total[0] and to total[1] how many
@@ -490,8 +490,9 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
     if (tile >= tiles) {
       // the last block to leave: every tile is claimed and left, every timeout counted
       if (tile == tiles + gridDim.x - 1 && threadIdx.x == 0) {
-        const uint32_t gave_up = *(volatile uint32_t*)(st + 6);
-        const bool complete = !wait_gave_up(st);
+        const volatile uint32_t* now = st;  // other blocks of this kernel count here
+        const uint32_t gave_up = now[6];
+        const bool complete = gave_up == now[7];
         unsigned long long w = load_status(tiles - 1);
         for (uint32_t polls = 0; (w & kInc) == 0ull && polls < spin_limit; ++polls) w = load_status(tiles - 1);
         const uint32_t sum = (uint32_t)w;
@@ -626,8 +627,7 @@ __global__ void __launch_bounds__(256) k_clear(ClearList c) {
 __global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ count, uint32_t cap,
                          const uint32_t* __restrict__ st, uint32_t* __restrict__ rstart,
                          uint32_t* __restrict__ rend) {
-  if (wait_gave_up(st)) return;
-  const uint32_t K = min(*count, cap);
+  const uint32_t K = wait_gave_up(st) ? 0u : min(*count, cap);
   const uint32_t n4 = (K + 3) / 4;
   for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n4; q += gridDim.x * blockDim.x) {
     const uint32_t p0 = 4 * q;
@@ -1672,8 +1672,7 @@ __global__ void k_det_prep(const uint32_t* __restrict__ sorted_vals, const uint3
 __global__ void k_det_segsum(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ pos,
                              const uint32_t* __restrict__ total, uint32_t cap, const uint32_t* __restrict__ st,
                              const float* __restrict__ part, float* __restrict__ g2) {
-  if (wait_gave_up(st)) return;
-  const uint32_t K = min(*total, cap);
+  const uint32_t K = wait_gave_up(st) ? 0u : min(*total, cap);
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < K; p += gridDim.x * blockDim.x) {
     const uint32_t k = keys[p];
     if (p > 0 && keys[p - 1] == k) continue;  // not the first pair of this record
