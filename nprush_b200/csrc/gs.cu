@@ -313,9 +313,11 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
   project<float>(view, mean, ls, q, (float)W, (float)H, kLowpass, P);
   uint32_t cnt = 0, ecnt = 0, tmask = 0;
   uint2 rect = make_uint2(0, 0);
-  // a record without pairs may stand anywhere in the depth order; at 2.0 it shares
-  // the top byte of every depth in [2, 8), and that digit's sort pass is free
-  uint32_t key = __float_as_uint(2.0f);
+  // positive floats order like their bit patterns; a record without pairs may stand
+  // anywhere in the depth order: at its own distance from the camera plane it has most
+  // likely the top byte of the visible ones (depths within a factor of four), and
+  // that digit's sort pass is free
+  const uint32_t key = __float_as_uint(fabsf(P.cw));
   Rec r;
   r.a = make_float4(0, 0, 0, 0);
   r.b = make_float4(0, 0, 0, 0);
@@ -335,7 +337,6 @@ __global__ void __launch_bounds__(256) k_preprocess(const float* __restrict__ pa
     if (x1 > x0 && y1 > y0) {
       cnt = (uint32_t)((x1 - x0) * (y1 - y0));
       rect = make_uint2((uint32_t)x0 | ((uint32_t)x1 << 16), (uint32_t)y0 | ((uint32_t)y1 << 16));
-      key = __float_as_uint(P.cw);  // positive floats order like their bit patterns
       // SH colour for the view direction
       const float dx = mean[0] - view[32], dy = mean[1] - view[33], dz = mean[2] - view[34];
       const float il = rsqrtf(fmaxf(dx * dx + dy * dy + dz * dz, 1e-20f));
