@@ -459,53 +459,48 @@ __device__ __forceinline__ bool wait_gave_up(const uint32_t* st) { return __ldg(
 // block counts a timeout (in st[6]) and carries on; positions stay below cap.  A
 // depth sort that gave up leaves places of sorted_g unwritten: an id of no
 // record (m or more) is an entry without pairs.
-// host (page-locked, may be null) gets the total and the timeouts for the host.
-// stall_tile: see nps_gs_set_bin_guard.
+// The claim counter's upper half counts the blocks that gave up, so that the last
+// one to leave knows.  host (page-locked, may be null) gets the total, the timeouts
+// so far and, where a block gave up later, those again for the host.
+// stall_tile publishes nothing (nps_gs_set_bin_guard).
 constexpr uint32_t kBinTile = 1024, kMostPairs = 0x7fffffffu;
 __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ sorted_g, const uint4* __restrict__ bins,
                                                   uint32_t m, uint32_t n, uint32_t tiles_x, uint32_t num_tiles,
                                                   uint32_t cap, uint32_t* __restrict__ keys,
                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ total,
                                                   unsigned long long* __restrict__ status,
-                                                  uint32_t* __restrict__ counter, uint32_t* st, uint32_t spin_limit,
+                                                  unsigned long long* __restrict__ counter, uint32_t* st, uint32_t spin_limit,
                                                   uint32_t stall_tile, volatile uint32_t* host) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32;
   __shared__ uint32_t s_tile, s_excl, s_warp[8];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t tiles = (m + kBinTile - 1) / kBinTile;
+  const volatile uint32_t* now = st;   // every block counts its timeouts there
+  unsigned long long gave_up = 0;      // thread 0: 2^32 if the block gave up since its last claim
   auto load_status = [&](uint32_t t) {
     unsigned long long w;
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(status + t) : "memory");
     return w;
   };
   auto store_status = [&](uint32_t t, unsigned long long w) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(status + t), "l"(w) : "memory");
+    if (t != stall_tile) asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(status + t), "l"(w) : "memory");
   };
   for (;;) {
     __syncthreads();  // the tile before is done with the shared words
-    if (threadIdx.x == 0)
-      asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], 1;" : "=r"(s_tile) : "l"(counter) : "memory");
+    if (threadIdx.x == 0) {
+      const unsigned long long claim = atomicAdd(counter, gave_up + 1ull);
+      s_tile = (uint32_t)claim;
+      // the last block to leave, after a timeout in any: the one that wrote host[1] may have missed it
+      if ((uint32_t)claim == tiles + gridDim.x - 1 && (claim + gave_up) >> 32 && host) {
+        __threadfence();
+        host[2] = now[6];
+      }
+      gave_up = 0;
+    }
     __syncthreads();
     const uint32_t tile = s_tile;
-    if (tile >= tiles) {
-      // the last block to leave: every tile is claimed and left, every timeout counted
-      if (tile == tiles + gridDim.x - 1 && threadIdx.x == 0) {
-        const volatile uint32_t* now = st;  // other blocks of this kernel count here
-        const uint32_t gave_up = now[6];
-        const bool complete = gave_up == now[7];
-        unsigned long long w = load_status(tiles - 1);
-        for (uint32_t polls = 0; (w & kInc) == 0ull && polls < spin_limit; ++polls) w = load_status(tiles - 1);
-        const uint32_t sum = (uint32_t)w;
-        total[0] = sum;
-        total[1] = !complete ? 0u : sum <= cap ? sum : host ? 0u : cap;
-        if (host) {
-          host[0] = sum;
-          host[1] = gave_up;
-        }
-      }
-      return;
-    }
+    if (tile >= tiles) return;
     const uint32_t first = tile * kBinTile + warp * 128u + lane;
     uint32_t g[4], off[4];
     uint4 b[4];
@@ -541,8 +536,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         if (lane == 0) store_status(tile, kAgg | sum);
         uint32_t j = tile, polls = 0;  // tiles below j are still to be added
         while (j > 0) {
-          unsigned long long w = lane < j ? load_status(j - 1 - lane) : kInc;
-          if (lane < j && j - 1 - lane == stall_tile) w = 0ull;
+          const unsigned long long w = lane < j ? load_status(j - 1 - lane) : kInc;
           const uint32_t inc = __ballot_sync(kFull, (w & kInc) != 0ull), none = __ballot_sync(kFull, (w >> 32) == 0ull);
           const uint32_t take = inc ? inc ^ (inc - 1u) : kFull;  // up to the nearest inclusive prefix
           if (none & take) {
@@ -550,6 +544,7 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
               if (lane == 0) {
                 atomicAdd(st + 6, 1u);
                 __threadfence();  // before this block's next claim, so that the last block sees it
+                gave_up = 1ull << 32;
               }
               break;
             }
@@ -563,7 +558,19 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
         }
         if (lane == 0) store_status(tile, kInc | min(excl + sum, kMostPairs));
       }
-      if (lane == 0) s_excl = excl;
+      if (lane == 0) {
+        s_excl = excl;
+        if (tile == tiles - 1) {
+          const uint32_t all = min(excl + sum, kMostPairs);
+          const uint32_t timeouts = now[6];
+          total[0] = all;
+          total[1] = timeouts != now[7] ? 0u : all <= cap ? all : host ? 0u : cap;
+          if (host) {
+            host[0] = all;
+            host[1] = timeouts;
+          }
+        }
+      }
     }
     __syncthreads();
     const uint32_t warp0 = min(s_excl + before, kMostPairs);
@@ -2971,11 +2978,12 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
         NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * nitems, s));
         NPS_CUDA(cudaMemsetAsync(o->bin_status.p, 0, 16 + 8 * (size_t)bin_tiles, s));
       }
+      if (!capture) o->h_fwd[2] = 0;  // the emission before has been waited for
       { StageTimer t(o, ST_EMIT);
       gs::k_bin_emit<<<std::min<uint32_t>(bin_tiles, 8u * kNumSMs), 256, 0, s>>>(
           dv, o->bins.as<uint4>(), (uint32_t)M, n, tiles_x, num_tiles, cap, o->keys.as<uint32_t>(),
           o->vals.as<uint32_t>(), total, reinterpret_cast<unsigned long long*>(o->bin_status.as<char>() + 16),
-          o->bin_status.as<uint32_t>(), st, o->bin_spin, o->bin_stall, capture ? nullptr : o->h_fwd);
+          o->bin_status.as<unsigned long long>(), st, o->bin_spin, o->bin_stall, capture ? nullptr : o->h_fwd);
       NPS_CHECK_LAUNCH(); }
       if (!capture) NPS_CUDA(cudaEventRecord(o->fwd_counted, s));
       if (cap > 0) {
@@ -2999,7 +3007,7 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
     if (capture || M == 0) break;
     NPS_CUDA(cudaEventSynchronize(o->fwd_counted));
     K = o->h_fwd[0];
-    const uint32_t tmo = o->h_fwd[1];
+    const uint32_t tmo = o->h_fwd[2] ? o->h_fwd[2] : o->h_fwd[1];
     if (tmo != o->timeouts_seen) {
       // reported here: the next Adam step must not skip for it again
       o->timeouts_seen = tmo;
