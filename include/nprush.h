@@ -348,7 +348,9 @@ int nps_gs_read_image(nps_gs* gs, float* rgba_host, float* dl_dimage_host);
  * nps_gs_set_variant selects form 0; nps_gs_set_tile changes the tile (and
  * switches to that tile's default persistent variants where the current ones
  * do not serve it); nps_gs_get_raster reports tile, forward form, ppt, stage,
- * backward form, ppt, stage (choice7).  nps_gs_autotune_raster bins the
+ * backward form, ppt, stage (choice7): what a pass over the current views and
+ * image size runs, the default included (before there are any, (0, 1, 256) and
+ * (0, 2, 128) while none was chosen).  nps_gs_autotune_raster bins the
  * current views at every tile size (timing the binning), times every variant
  * of each tile, forward and backward, and keeps the tile with the smallest
  * binning + fastest forward + fastest backward, with those variants; with

@@ -3799,9 +3799,14 @@ int nps_gs_set_tile(nps_gs* o, uint32_t tile) {
 int nps_gs_get_raster(nps_gs* o, int* choice7) {
   NPS_TRY(check_gs(o));
   if (!choice7) return NPS_ERR_INVALID;
+  RasterVariant f{o->fwd_form, o->fwd_ppt, o->fwd_stage}, b{o->bwd_form, o->bwd_ppt, o->bwd_stage};
+  if (o->nv > 0 && o->w > 0) {  // there is a grid: what a pass over it runs
+    f = raster_variant(o, false);
+    b = raster_variant(o, true);
+  }
   choice7[0] = (int)o->tile;
-  choice7[1] = o->fwd_form; choice7[2] = o->fwd_ppt; choice7[3] = o->fwd_stage;
-  choice7[4] = o->bwd_form; choice7[5] = o->bwd_ppt; choice7[6] = o->bwd_stage;
+  choice7[1] = f.form; choice7[2] = f.ppt; choice7[3] = f.stage;
+  choice7[4] = b.form; choice7[5] = b.ppt; choice7[6] = b.stage;
   return NPS_OK;
 }
 
@@ -3890,6 +3895,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
   if (times_ms99)
     for (int i = 0; i < kNumTiles * kTuneStride; ++i) times_ms99[i] = 0.0f;  // 0: not a variant of that tile
   cudaStream_t s = o->ctx->stream;
+  const bool was_auto = o->raster_auto;
   const uint32_t M = o->n * o->nv;
   NPS_TRY(o->g2.ensure(sizeof(float) * gs::kG2 * ((size_t)M + 1)));
   cudaEvent_t e0, e1;
@@ -3949,6 +3955,7 @@ int nps_gs_autotune_raster(nps_gs* o, const char* cache_path, int* choice7, floa
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  if (rc != NPS_OK) o->raster_auto = was_auto;  // nothing was chosen
   o->tile = best_tile;
   o->fwd_form = best_pick[0].form, o->fwd_ppt = best_pick[0].ppt, o->fwd_stage = best_pick[0].stage;
   o->bwd_form = best_pick[1].form, o->bwd_ppt = best_pick[1].ppt, o->bwd_stage = best_pick[1].stage;

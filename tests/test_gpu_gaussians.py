@@ -768,3 +768,35 @@ def test_forward_that_outgrows_its_pair_buffers(trainer_cls, n):
     for grown, fresh in ((out[0], out[2]), (out[1], out[3])):
         for a, b in zip(grown, fresh):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("tiles_x,tiles_y,views", [(4, 4, 1), (37, 16, 1), (593, 1, 1), (40, 25, 1), (37, 12, 4), (1777, 1, 1), (25, 20, 4)])
+def test_raster_reports_the_default_of_the_grid(trainer_cls, tiles_x, tiles_y, views):
+    """The default variant that runs is the one reported: 1 pixel per thread up to 4
+    (backward) and 12 (forward) tiles per SM, at, just above and around 592 and 1776
+    tiles on 148 SMs, 2 beyond; a chosen variant as chosen, whatever the grid.  Chosen
+    as reported, it gives the default's image bit for bit and its gradients to 1e-5."""
+    w, h = 16 * tiles_x, 16 * tiles_y
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    items = tiles_x * tiles_y * views
+    want = dict(tile=16, fwd=(0, 1, 256) if items <= 12 * sms else (0, 2, 128),
+                bwd=(0, 1, 256) if items <= 4 * sms else (0, 2, 128))
+    p = gs_scene(800, 113, deg=0, log_scale_mean=-3.0)
+    vp, vpi, _ = gs_views(w, h, ((0.0, 0.0, 4.0), (2.5, 1.0, 3.0), (-2.0, 0.5, 3.0), (0.5, -2.0, 3.5))[:views])
+    t = trainer_cls(800, sh_degree=0, params=p)
+    assert t.raster() == dict(tile=16, fwd=(0, 1, 256), bwd=(0, 2, 128))
+    t.set_targets(gs_targets(views, w, h, 114))
+    t.set_views(vp, vpi)
+    out = []
+    for chosen in (False, True):
+        assert t.raster() == want
+        t.forward()
+        t.loss()
+        t.backward()
+        out.append((t.read_image(with_grad=False)[0], t.read_state()["grads"].astype(np.float64)))
+        if not chosen:
+            t.set_raster(want["fwd"], want["bwd"])
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    assert np.linalg.norm(out[0][1] - out[1][1]) / np.linalg.norm(out[0][1]) < 1e-5
+    t.set_raster((0, 4, 64), (0, 4, 128))
+    assert t.raster() == dict(tile=16, fwd=(0, 4, 64), bwd=(0, 4, 128))
