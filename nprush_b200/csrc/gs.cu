@@ -1918,7 +1918,7 @@ struct AdamArgs {
 };
 
 // Step state in device memory (so that a captured graph advances it):
-// [0] step counter, [1] skip flag, [2], [3] bias corrections (f32 bits),
+// [0] step counter, [1] skip flag, [2], [3] 1 / bias corrections (f32 bits),
 // [4] steps skipped for pair overflow, [6] bounded device waits that gave up
 // (raster staging, sort look-back), [7] the value of [6] the last Adam step saw.
 // The step is skipped when the last forward produced more pairs than the
@@ -1927,9 +1927,19 @@ struct AdamArgs {
 // a bounded wait gave up since the last step (its results are incomplete).
 // host (page-locked, may be null): the pair count, [4] and [6] for the host,
 // written here because a graph's copy nodes cost a small step 6 us each.
+// Two threads, one for each bias correction: the 64-bit powers and divisions are
+// the kernel's time, and go side by side.
 __global__ void k_adam_prep(uint32_t* st, const uint32_t* total, uint32_t cap, volatile uint32_t* host) {
   const bool overflow = *total > cap;
   const bool timed_out = st[6] != st[7];
+  const uint32_t step = st[0] + 1;
+  if (!overflow && !timed_out) {
+    const double beta = threadIdx.x == 0 ? 0.9 : 0.999;
+    // rounded once (a 32-bit correction's reciprocal would be rounded twice)
+    st[2 + threadIdx.x] = __float_as_uint((float)(1.0 / (1.0 - pow(beta, (double)step))));
+  }
+  __syncwarp(3u);  // both have read the state
+  if (threadIdx.x == 1) return;
   st[7] = st[6];
   st[1] = (overflow || timed_out) ? 1u : 0u;
   if (overflow) st[4] += 1u;  // skipped steps so far (read by the host after graph replays)
@@ -1938,11 +1948,7 @@ __global__ void k_adam_prep(uint32_t* st, const uint32_t* total, uint32_t cap, v
     host[1] = st[4];
     host[2] = st[6];
   }
-  if (overflow || timed_out) return;
-  const uint32_t step = st[0] + 1;
-  st[0] = step;
-  st[2] = __float_as_uint((float)(1.0 - pow(0.9, (double)step)));
-  st[3] = __float_as_uint((float)(1.0 - pow(0.999, (double)step)));
+  if (!overflow && !timed_out) st[0] = step;
 }
 
 __device__ __forceinline__ float lr_of(const AdamArgs& a, int k) {
@@ -1951,15 +1957,17 @@ __device__ __forceinline__ float lr_of(const AdamArgs& a, int k) {
 
 // one thread per float4 of the parameter record (16 per Gaussian).  Was bound by
 // its four full divisions per value as much as by memory; the two bias corrections
-// are now products with their reciprocals: 1M Gaussians 420 -> 289 us, 200k 91 ->
-// 66 us (floors at the copy rate: 250 and 50).
+// are products with their reciprocals: 1M Gaussians 420 -> 285 us, 200k 91 ->
+// 64 us (floors at the copy rate: 250 and 50).
 __global__ void __launch_bounds__(256) k_adam(float4* __restrict__ p, const float4* __restrict__ g,
                                               float4* __restrict__ m, float4* __restrict__ v, uint32_t n4,
                                               AdamArgs a, const uint32_t* __restrict__ st) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n4 || st[1] != 0u) return;
+  if (t >= n4) return;
+  const uint4 state = __ldg(reinterpret_cast<const uint4*>(st));  // one load (three words apart: 68 us)
+  if (state.y != 0u) return;
   if ((t & 15u) * 4u >= (uint32_t)kUsed) return;  // floats 60-63: nothing to update, nothing to move
-  const float ibc1 = 1.0f / __uint_as_float(st[2]), ibc2 = 1.0f / __uint_as_float(st[3]);
+  const float ibc1 = __uint_as_float(state.z), ibc2 = __uint_as_float(state.w);
   const int k0 = (int)(t & 15u) * 4;
   float4 pp = p[t], gg = g[t], mm = m[t], vv = v[t];
   float* pf = &pp.x;
@@ -3232,7 +3240,7 @@ int nps_gs_adam(nps_gs* o) {
   a.eps = 1e-15f;
   const uint32_t n4 = o->n * 16;
   StageTimer t_adam(o, ST_ADAM);
-  gs::k_adam_prep<<<1, 1, 0, o->ctx->stream>>>(o->stepst.as<uint32_t>(), o->total.as<uint32_t>(),
+  gs::k_adam_prep<<<1, 2, 0, o->ctx->stream>>>(o->stepst.as<uint32_t>(), o->total.as<uint32_t>(),
                                                o->pair_cap ? o->pair_cap : 0xffffffffu,
                                                o->capturing ? o->h_status : nullptr);
   gs::k_adam<<<div_up(n4, 256), 256, 0, o->ctx->stream>>>(o->params.as<float4>(), o->grads.as<float4>(),

@@ -800,3 +800,38 @@ def test_raster_reports_the_default_of_the_grid(trainer_cls, tiles_x, tiles_y, v
     assert np.linalg.norm(out[0][1] - out[1][1]) / np.linalg.norm(out[0][1]) < 1e-5
     t.set_raster((0, 4, 64), (0, 4, 128))
     assert t.raster() == dict(tile=16, fwd=(0, 4, 64), bwd=(0, 4, 128))
+
+
+@pytest.mark.parametrize("step", [5, 20, 2000, 5000])
+def test_adam_bias_corrections_are_rounded_once(trainer_cls, step):
+    """An Adam step from zero parameters with given moments (the Gaussians stand behind
+    the camera: no gradient) against 64 bits.  A value's own roundings (up to about
+    2^-23, either way) average out over 300k values; what is left is the error of the two
+    corrections, m's and half of v's.  As 32-bit reciprocals of the exact corrections it is
+    known to 0.05 x 2^-24; a correction rounded before its reciprocal is off by 0.3 to 1
+    x 2^-24 at these steps."""
+    n = 5500
+    rng = np.random.default_rng(step)
+    p = np.zeros((n, 64), np.float32)
+    p[:, 2] = 100.0
+    m = rng.normal(0, 1e-3, (n, 64)).astype(np.float32)
+    v = np.square(rng.normal(0, 1e-3, (n, 64))).astype(np.float32) + np.float32(1e-8)
+    t = trainer_cls(n, sh_degree=3, params=p)
+    t.write_state(m, v, step - 1)
+    vp, vpi, _ = gs_views(32, 32)
+    t.set_targets(gs_targets(1, 32, 32, 115))
+    t.set_views(vp, vpi)
+    t.train_step()
+    s = t.read_state()
+    assert not s["grads"].any()
+    c = slice(3, 59)
+    lr = np.repeat(np.asarray(t.LR_DEFAULT, np.float32), [3, 3, 4, 2, 3, 44])[c].astype(np.float64)
+    mh = s["adam_m"][:, c].astype(np.float64) / (1 - 0.9 ** step)
+    vh = s["adam_v"][:, c].astype(np.float64) / (1 - 0.999 ** step)
+    want = -lr * mh / (np.sqrt(vh) + np.float64(np.float32(1e-15)))
+    used = np.arange(3, 59) != 11
+    got = s["params"][:, c].astype(np.float64)
+    err = float(np.mean((got / want - 1)[:, used])) * 2.0 ** 24
+    r1, r2 = 1 / (1 - 0.9 ** step), 1 / (1 - 0.999 ** step)
+    bias = ((np.float64(np.float32(r1)) / r1 - 1) - 0.5 * (np.float64(np.float32(r2)) / r2 - 1)) * 2.0 ** 24
+    assert abs(err - bias) < 0.05, (err, bias)
