@@ -737,7 +737,9 @@ __global__ void __launch_bounds__(kRasterThreads, 6) k_raster(RasterArgs a) {
       }
     }
   };
-  auto sum2 = [](float2 x) { return to_i32(x.x) + to_i32(x.y); };  // each term truncated on its own
+  // a sum of two terms wraps, as the shader's atomicAdd of each does
+  auto wrap_add = [](int32_t p, int32_t q) { return (int32_t)((uint32_t)p + (uint32_t)q); };
+  auto sum2 = [&](float2 x) { return wrap_add(to_i32(x.x), to_i32(x.y)); };  // each term truncated on its own
   uint32_t j = 0;
   for (; c == nch && j < nch; ++j) {
     const uint32_t q = nch + j, cc = nch - 1 - j, b = q & 1u;
@@ -788,8 +790,8 @@ __global__ void __launch_bounds__(kRasterThreads, 6) k_raster(RasterArgs a) {
       }
       const bool live = __any_sync(kFull, T_prev.x != 0.0f || T_prev.y != 0.0f);
       const PairCommon p = pair_common(f, bw, e, al, T_prev, dCr, dCg, dCb, dD, dT_C, dT_D);
-      const int32_t q13 = (v0 ? to_i32(p.d_shape_a.x * kFpPos) : 0) + (v1 ? to_i32(p.d_shape_a.y * kFpPos) : 0);
-      const int32_t q14 = (v0 ? to_i32(p.d_shape_b.x * kFpPos) : 0) + (v1 ? to_i32(p.d_shape_b.y * kFpPos) : 0);
+      const int32_t q13 = wrap_add(v0 ? to_i32(p.d_shape_a.x * kFpPos) : 0, v1 ? to_i32(p.d_shape_a.y * kFpPos) : 0);
+      const int32_t q14 = wrap_add(v0 ? to_i32(p.d_shape_b.x * kFpPos) : 0, v1 ? to_i32(p.d_shape_b.y * kFpPos) : 0);
       // lane jj collects the warp's sum of term jj: one shared atomic instruction adds them all
       int32_t sum = 0;
       auto collect = [&](int32_t q, uint32_t jj) {

@@ -322,3 +322,22 @@ def test_edge_target_and_dispatch_edge(mgr_cls):
     on_edge = np.abs(raw - np.floor(raw) - 0.5) < 1e-5 * 255
     assert np.all((got == np.rint(raw) / 255) | on_edge)
     m.close()
+
+
+@pytest.mark.parametrize("w,h,seed", [(33, 47, 5), (64, 50, 6), (16, 16, 7)])
+def test_saturated_terms_wrap(mgr_cls, w, h, seed):
+    """Targets of -1e8 and 1e8: every term of those colours' gradients saturates, and
+    their i32 sums (an odd number of terms, down to pairs of pixels) wrap as the shader's
+    atomicAdd does, exactly."""
+    s = splat_scene(1, seed, spread=0.1)
+    s[:, 7] = 0.9
+    s[:, [3, 12, 15]] = 0.3
+    vp, vpi = camera(w, h)
+    tgt, depth = targets(w, h, seed)
+    tgt[..., 0], tgt[..., 1] = -1e8, 1e8
+    ref = orc.splat_backward(s, vp, vpi, tgt, depth)
+    g, _, _ = run_backward(mgr_cls, s, [vp], [vpi], [tgt], [depth])
+    n = int(ref["terms"][0])
+    wrap = lambda t: (t * n + 2 ** 31) % 2 ** 32 - 2 ** 31  # noqa: E731
+    assert ref["grads_q"][0, 4:6].tolist() == [wrap(2147483520), wrap(-2 ** 31)]
+    np.testing.assert_array_equal(g[0, 4:6], ref["grads_q"][0, 4:6])
