@@ -45,6 +45,7 @@ constexpr int kChunk = 32;
 constexpr int kSlots = 16;      // pairs of a chunk differentiated per replay (k_raster)
 constexpr int kThreads = 256;
 constexpr int kRasterThreads = 128;  // k_raster: two pixels of a 16 x 16 tile each
+constexpr uint32_t kStrip = 8;       // k_raster: a warp's pixels are kStrip x kStrip
 constexpr float kFpPos = 10000.0f, kFpCol = 100000.0f;  // constants.ts:36-37
 constexpr float kOpacityKill = 0.05f, kVolumeKill = 1e-7f, kGradThresh = 0.00005f, kAdcPeriod = 25.0f;
 
@@ -590,7 +591,7 @@ __device__ __forceinline__ uint2 strip_masks(const float (*fwd)[kFwd], uint32_t 
 //    radius, so most tile pairs miss most warps: of the pairs of 200k splats,
 //    800 x 800, 60% have alpha 0 over the warp and 82% no alpha of 0.001
 //    (dispatch 33.1 -> 22.9 ms; 512 splats, 512 x 512: 1.60 -> 1.07 ms);
-//  * a warp whose 32 pixels all reached T == 0 stops compositing: a pair
+//  * a warp whose 64 pixels all reached T == 0 stops compositing: a pair
 //    then adds T * alpha * c = 0 and leaves T at 0 (for finite colours and
 //    depths, which the step keeps inside their boxes);
 //  * a chunk that starts at T == 0 for the whole warp is not replayed;
@@ -605,7 +606,8 @@ __global__ void __launch_bounds__(kRasterThreads, 6) k_raster(RasterArgs a) {
 
   const uint32_t tx = blockIdx.x, ty = blockIdx.y, v = blockIdx.z;
   const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t px = tx * 16 + 8 * (warp & 1u) + (lane & 7u), py = ty * 16 + 8 * (warp >> 1) + 2 * (lane >> 3);
+  const uint32_t px = tx * 16 + kStrip * (warp & 1u) + lane % kStrip;
+  const uint32_t py = ty * 16 + kStrip * (warp >> 1) + 2 * (lane / kStrip);
   const bool in0 = px < a.w && py < a.h, in1 = px < a.w && py + 1 < a.h;
   const float aspect = (float)a.w / (float)a.h;
   const float ppx = pixel_px(px, a.w, aspect);
