@@ -224,7 +224,8 @@ __device__ __forceinline__ void walk(const float4* seg, const float* len2, uint3
 // pixel's closest one where every segment is farther than r and alpha is 0
 // whichever segment is taken: leaving it out changes no alpha.  Returns the
 // mask of curves with a segment left; lane k gets curve k's segments.
-// A coordinate that is not a number keeps its segments.
+// A coordinate that is not a number keeps its segments; a curve whose colour is
+// not finite keeps all of them, since it makes the composite NaN even at alpha 0.
 __device__ __forceinline__ uint32_t strip_segments(const RasterSmem& S, uint32_t cnt, uint32_t lane, float x0,
                                                    float x1, float y0, float y1, uint32_t* own) {
   constexpr unsigned kFull = 0xffffffffu;
@@ -239,6 +240,7 @@ __device__ __forceinline__ uint32_t strip_segments(const RasterSmem& S, uint32_t
   if (lane < cnt) {
     const float* f = S.fwd[lane];
     r = (fabsf(f[12]) + fabsf(f[13])) * 1.001f + 1e-6f;
+    if (!(fabsf(f[15]) + fabsf(f[16]) + fabsf(f[17]) <= 3e38f)) r = __int_as_float(0x7f800000);
     // the curve lies in the hull of its control points
     hit = !far_box(fminf(fminf(f[0], f[2]), fminf(f[4], f[6])), fmaxf(fmaxf(f[0], f[2]), fmaxf(f[4], f[6])),
                    fminf(fminf(f[1], f[3]), fminf(f[5], f[7])), fmaxf(fmaxf(f[1], f[3]), fmaxf(f[5], f[7])), r);

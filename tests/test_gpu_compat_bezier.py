@@ -217,3 +217,29 @@ def test_separate_vp_writes_equal_the_combined_write(cls):
     for st in states[1:]:
         for k in ("beziers", "adam_m", "adam_v", "grad_accum"):
             np.testing.assert_array_equal(st[k], states[0][k])
+
+
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("channel", [16, 18])
+def test_colour_that_is_not_finite(cls, channel, value):
+    """A curve whose colour is not finite makes every pixel of its tiles NaN or
+    infinite, near or far from the curve, as the reference's composite does (T * 0 * inf);
+    the pattern equals the oracle's, and so do the gradient sums (a NaN term is 0)."""
+    n, w, h = 60, 48, 32
+    b = bezier_scene(n, 7)
+    b[5, channel] = value
+    vp, vpi = camera(w, h, dist=1.4)
+    tgt, depth, bg, bgd, nrm = bezier_textures(w, h, 8)
+    m = cls(n, init=b)
+    m.write_vp(vp, vpi)
+    m.write_mode(1.0)
+    m.set_backward_target(tgt, depth, bg, bgd, nrm, w, h)
+    img = torch.zeros((1, h, w, 4), device="cuda")
+    m.backward(out_rgbd=img)
+    ref = orc.bezier_backward(b, vp, uni6(1.0, 0.0, 0, 0, 0.0), tgt, depth, bg, bgd, nrm,
+                              loss_accum=np.zeros(n, np.float32))
+    got = img.cpu().numpy()[0]
+    assert np.isnan(ref["image"]).any()
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(ref["image"]))
+    np.testing.assert_allclose(got, ref["image"], atol=1e-5, rtol=0, equal_nan=True)
+    np.testing.assert_array_equal(m.read_state()["grads"], ref["grads_q"])
