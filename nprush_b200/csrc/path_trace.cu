@@ -379,13 +379,17 @@ constexpr uint32_t kNoRef = 0xffffffffu;  // a leaf of seven triangles: none has
 
 // Closest hit by front-to-back traversal: both children of a node are tested
 // at once, the nearer is entered and the other one waits on the stack with its
-// entry distance.  It finds the triangle that scene_hit finds: the leaves'
-// boxes reach 1e-4 beyond their triangles (bvh.ts:66), so with coordinates
-// within kOrderedReach (rounding below 2e-5) the box of the closest triangle
-// is entered before that triangle's distance and is never left out, in
-// whatever order the boxes come; between hits at equal distance scene_hit
-// keeps the one it meets first, which is the one first in BVH order.
-// (94 M paths over 30 scenes: the same radiances, bit for bit.)
+// entry distance.  It finds the triangle that scene_hit finds where that hit's
+// distance lies within its leaf's box: the boxes reach 1e-4 beyond their
+// triangles (bvh.ts:66), so with coordinates within kOrderedReach (rounding below
+// 2e-5) the box of the closest triangle is entered before that triangle's
+// distance and is never left out, in whatever order the boxes come; between hits
+// at equal distance scene_hit keeps the one it meets first, which is the one first
+// in BVH order.  Not bounded is the distance of a triangle seen nearly edge-on,
+// whose U, V and W are mostly rounding: it may be that of any point of the
+// triangle, before its box is entered, and a hit between the two then prunes the
+// box in one order and not in the other.  Not seen in 94 M paths over 30 scenes:
+// the same radiances, bit for bit.
 //
 // The bound is instruction issue at a few active lanes (bounced rays part).  1024
 // x 768, 12k triangles, per frame, from the reference's order at 0.764 ms: 0.565
@@ -615,10 +619,11 @@ __global__ void k_pt_resolve(const float4* __restrict__ accum, float4* __restric
 }
 
 // Pair records of a built tree, 16 floats per inner node in node order: per
-// axis both children's lo planes, then both hi planes; then their references.  Returns the root's reference and whether the
-// front-to-back traversal may stand in for the reference's: no path deeper than
-// its stack (the reference drops subtrees beyond 64 entries) and no
-// coordinate beyond kOrderedReach.
+// axis both children's lo planes, then both hi planes; then their references.
+// Returns the root's reference and whether the front-to-back traversal may stand
+// in for the reference's: an inner node at the root (a single leaf's box would not
+// be tested), no path deeper than its stack (the reference drops subtrees beyond 64
+// entries) and no coordinate beyond kOrderedReach.
 constexpr float kOrderedReach = 64.0f;
 bool pack_pairs(const Bvh& b, std::vector<float>& pairs, uint32_t* root) {
   const size_t n = b.nodes.size() / 8;
@@ -631,9 +636,11 @@ bool pack_pairs(const Bvh& b, std::vector<float>& pairs, uint32_t* root) {
   uint32_t inner = 0;
   bool ok = b.tris.size() / 3 <= kLeafFirstMask;
   for (size_t i = 0; i < n; ++i) {
-    if (word(i, 7) & kLeafFlag) rec[i] = kLeafFlag | ((word(i, 7) & 7u) << kLeafCountShift) | (word(i, 3) & kLeafFirstMask);
+    if (word(i, 7) & kLeafFlag)
+      rec[i] = kLeafFlag | ((word(i, 7) & 7u) << kLeafCountShift) | (word(i, 3) & kLeafFirstMask);
     else rec[i] = inner++;
   }
+  ok = ok && inner > 0;
   pairs.assign((size_t)std::max(1u, inner) * 16, 0.0f);
   for (size_t i = 0; i < n; ++i) {  // pre-order: parents before children
     for (int k = 0; k < 3; ++k)
@@ -749,7 +756,8 @@ int nps_pt_create(nps_ctx* ctx, const float* vertices, uint32_t n_vertices, cons
   std::vector<float> pairs;
   o->ordered = pt::pack_pairs(o->bvh, pairs, &o->root);
   int rc = NPS_OK;
-  if ((rc = o->nodes.ensure(n_nodes * 32)) || (rc = o->pairs.ensure(pairs.size() * 4)) || (rc = o->tri_pos.ensure(pos.size() * 4 + 16)) ||
+  if ((rc = o->nodes.ensure(n_nodes * 32)) || (rc = o->pairs.ensure(pairs.size() * 4)) ||
+      (rc = o->tri_pos.ensure(pos.size() * 4 + 16)) ||
       (rc = o->tri_idx.ensure((size_t)n_tris * 12 + 16)) || (rc = o->verts.ensure((size_t)n_vertices * 48 + 16)) ||
       (rc = o->env.ensure(16)) || (rc = o->stats.ensure(16))) {
     delete o;
