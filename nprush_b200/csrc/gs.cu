@@ -3153,7 +3153,7 @@ int nps_gs_backward(nps_gs* o, const float* dl_dimg) {
     const RasterVariant va = raster_variant(o, true);
     NPS_TRY(launch_bwd_raster(o, va.form, va.ppt, va.stage, dimg));
     NPS_CHECK_LAUNCH();
-  } else if (o->pair_cap > 0) {
+  } else if (o->pair_cap > 0 && M > 0) {  // (without records the pair count is an earlier call's)
     if (o->tile != 16) {
       set_error("gs_backward: the deterministic backward needs 16 x 16 tiles (tile is %u)", o->tile);
       return NPS_ERR_STATE;

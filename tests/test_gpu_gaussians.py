@@ -835,3 +835,29 @@ def test_adam_bias_corrections_are_rounded_once(trainer_cls, step):
     r1, r2 = 1 / (1 - 0.9 ** step), 1 / (1 - 0.999 ** step)
     bias = ((np.float64(np.float32(r1)) / r1 - 1) - 0.5 * (np.float64(np.float32(r2)) / r2 - 1)) * 2.0 ** 24
     assert abs(err - bias) < 0.05, (err, bias)
+
+
+@pytest.mark.parametrize("deterministic", [True, False])
+def test_no_gaussians_after_some(trainer_cls, deterministic):
+    """A trainer whose count goes to zero (the pair count and buffers are an earlier
+    call's): a background image, no gradients, and the Gaussians' step again after."""
+    n, w, h = 3000, 96, 80
+    p = gs_scene(n, 116, deg=0, log_scale_mean=-3.0)
+    vp, vpi, _ = gs_views(w, h)
+    tg = gs_targets(1, w, h, 117)
+    t = trainer_cls(n, sh_degree=0, params=p)
+    t.set_deterministic(deterministic)
+    t.set_background((0.25, 0.5, 0.75))
+    t.set_targets(tg)
+    t.set_views(vp, vpi)
+    t.forward()
+    img = t.read_image(with_grad=False)[0]
+    t.set_count(0)
+    t.forward()
+    t.loss()
+    t.backward()
+    assert (t.read_image()[0][..., :3] == np.float32([0.25, 0.5, 0.75])).all()
+    t.train_step()
+    t.set_count(n)
+    t.forward()
+    np.testing.assert_array_equal(t.read_image(with_grad=False)[0], img)
