@@ -8,7 +8,8 @@
 //   scan, emit, stable radix sort, ranges (as for splats; 1024 cap at :166)
 //   k_bz_raster   one CTA per (tile, view): the closest-point walk over the
 //                 segments (of 16) within reach of a warp's pixels, pressure,
-//                 analytic coverage, composite over the background (:196-269), luma / contrast / depth / edge loss (:271-320),
+//                 analytic coverage, composite over the background
+//                 (:196-269), luma / contrast / depth / edge loss (:271-320),
 //                 reverse backward through the closest segment with the width,
 //                 softness and direction-regulariser terms (:325-563),
 //                 transmittance replayed exactly from per-24-curve
@@ -34,7 +35,7 @@ namespace bz {
 constexpr int kRecF = 20;      // forward record floats
 constexpr int kRecB = 24;      // backward record floats (per control point: d screen / d world, 2 x 3)
 constexpr uint32_t kCap = 1024;  // BEZIER_MAX_TILE_BEZIERS, constants.ts:20
-constexpr int kChunk = 24;       // 73 KB of shared memory per CTA: three per SM
+constexpr int kChunk = 24;       // 69,120 bytes of shared memory per CTA: three per SM
 constexpr int kMaxChunks = (kCap + kChunk - 1) / kChunk;  // transmittance checkpoints per pixel
 constexpr int kThreads = 256;
 constexpr uint32_t kNSeg = 16;   // bezier_backward.wgsl:52
@@ -327,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_bz_raster(RasterArgs A) {
   const float sx0 = bin::pixel_px(wx, A.w, aspect), sx1 = bin::pixel_px(wx + 7, A.w, aspect);
   const float sy0 = bin::pixel_py(wy + 3, A.h), sy1 = bin::pixel_py(wy, A.h);
   const uint32_t key = v * A.num_tiles + ty * A.tiles_x + tx;
-  // the checkpoints are this CTA's own (32 KB-scale, global memory kept in L2
+  // the checkpoints are this CTA's own (43 KB, global memory kept in L2
   // between the forward's write and the backward's read; in shared memory they
   // held residency at two CTAs per SM, here three fit)
   float* ckpt = A.ckpt + (size_t)key * kMaxChunks * kThreads;

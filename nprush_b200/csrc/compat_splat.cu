@@ -81,7 +81,9 @@ __device__ __forceinline__ float4 mulv(const float* m, float x, float y, float z
 }
 
 struct f3 { float x, y, z; };
-__device__ __forceinline__ f3 cross3(f3 a, f3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
+__device__ __forceinline__ f3 cross3(f3 a, f3 b) {
+  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
 // splat_backward.wgsl:42-45
 __device__ __forceinline__ f3 quat_rotate(float qw, float qx, float qy, float qz, f3 v) {
   f3 u{qx, qy, qz};
@@ -1181,7 +1183,8 @@ struct RenderWork {
   SortWork sw;
   uint32_t pair_cap = 0;
   void release() {
-    for (DevBuf* b : {&rec, &counts, &offsets, &rects, &total, &cam, &keys, &vals, &ranges, &tabs, &sw.partial, &sw.lookback, &sw.keys_alt, &sw.vals_alt})
+    for (DevBuf* b : {&rec, &counts, &offsets, &rects, &total, &cam, &keys, &vals, &ranges, &tabs, &sw.partial,
+                      &sw.lookback, &sw.keys_alt, &sw.vals_alt})
       b->release();
   }
 };
@@ -1282,7 +1285,8 @@ int nps_splat_opt_destroy(nps_splat_opt* o) {
   for (DevBuf* b : {&o->params, &o->grads, &o->am, &o->av, &o->gacc, &o->views, &o->tgt_rgba_own,
                     &o->tgt_depth_own, &o->fwd, &o->bwd, &o->counts, &o->kept, &o->offsets, &o->rects, &o->total,
                     &o->grid, &o->cutoff, &o->tile_len, &o->ckbuf,
-                    &o->keys, &o->vals, &o->ranges, &o->tabs, &o->dead, &o->stat, &o->tstat, &o->sw.partial, &o->sw.lookback, &o->sw.keys_alt, &o->sw.vals_alt})
+                    &o->keys, &o->vals, &o->ranges, &o->tabs, &o->dead, &o->stat, &o->tstat, &o->sw.partial,
+                    &o->sw.lookback, &o->sw.keys_alt, &o->sw.vals_alt})
     b->release();
   if (o->rw) {
     o->rw->release();

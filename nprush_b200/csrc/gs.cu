@@ -7,23 +7,24 @@
 //                  tile rectangle of the alpha >= 1/255 ellipse, SH colour,
 //                  depth key
 //   radix sort     32-bit depth keys of all (view, Gaussian) records
-//   k_bin_emit     (view * tiles + tile, record) pairs written in depth order
+//   k_bin_emit     (view * tiles + tile, record) pairs written in depth order,
+//                  and their number
 //   radix sort     stable by tile key -> every tile list is depth ordered
 //   k_ranges       tile list bounds
 //   k_fwd          one CTA per (tile, view): records staged in shared memory
-//                  256 at a time, warps skip records whose footprint misses
-//                  their two pixel rows, front-to-back compositing with alpha
-//                  clamp 0.99, 1/255 skip and early termination at T < 1e-4
-//                  (block-wide vote ends the tile), final T and last
-//                  contributor stored per pixel (O(pixels) state, no
-//                  per-pair state)
+//                  in batches, warps ballot out the records whose footprint
+//                  misses their strip of pixels, front-to-back compositing
+//                  with alpha clamp 0.99, 1/255 skip and early termination at
+//                  T < 1e-4 (block-wide vote ends the tile), final T and last
+//                  contributor stored per pixel (O(pixels) state, no per-pair
+//                  state)
 //   k_ssim_fwd / k_ssim_bwd / k_loss_reduce: (1 - l) L1 + l (1 - SSIM), 11x11
 //                  Gaussian window (sigma 1.5), l = 0.2, and dL/dimage
 //   k_bwd2         reverse traversal replaying transmittance from the final
-//                  T, two pixels per thread, per-Gaussian gradients summed
-//                  over the warp by a 16-shuffle reduce-scatter, then over the
-//                  CTA in shared memory, then one global atomic per (tile,
-//                  Gaussian, value); k_bwd<true> + k_det_segsum: the
+//                  T, per-Gaussian gradients summed over the warp (through
+//                  shared memory, or by shuffles for two pairs at once), then
+//                  over the CTA in shared memory, then one global atomic per
+//                  (tile, Gaussian, value); k_bwd<true> + k_det_segsum: the
 //                  deterministic two-pass variant
 //   k_project_bwd  up to eight lanes per Gaussian over the views: screen-space
 //                  gradients -> parameter gradients, ADC statistics
@@ -453,12 +454,14 @@ __device__ __forceinline__ bool wait_gave_up(const uint32_t* st) { return __ldg(
 // (84 -> 52 us at 11.5 M pairs).
 //
 // Counts stay at kMostPairs once they reach it, beyond any cap (a sort takes fewer
-// than 2^30 pairs), so that a scene whose pairs pass 2^32 is not mistaken for a small one
-// (a sum of 32 entries is at most 2^31: an image has at most 2^26 tiles).  Status words as in
-// the sort (flag and 32-bit count), cleared beforehand.  The look-back is bounded: after spin_limit polls of an unpublished tile the
-// block counts a timeout (in st[6]) and carries on; positions stay below cap.  A
-// depth sort that gave up leaves places of sorted_g unwritten: an id of no
-// record (m or more) is an entry without pairs.
+// than 2^30 pairs), so that a scene whose pairs pass 2^32 is not mistaken for a
+// small one (a sum of 32 entries is at most 2^31: an image has at most 2^26 tiles).
+//
+// Status words as in the sort (flag and 32-bit count), cleared beforehand.  The
+// look-back is bounded: after spin_limit polls of an unpublished tile the block
+// counts a timeout (in st[6]) and carries on; positions stay below cap.  A depth
+// sort that gave up leaves places of sorted_g unwritten: an id of no record (m or
+// more) is an entry without pairs.
 // The claim counter's upper half counts the blocks that gave up, so that the last
 // one to leave knows.  host (page-locked, may be null) gets the total, the timeouts
 // so far and, where a block gave up later, those again for the host.
@@ -469,8 +472,8 @@ __global__ void __launch_bounds__(256) k_bin_emit(const uint32_t* __restrict__ s
                                                   uint32_t cap, uint32_t* __restrict__ keys,
                                                   uint32_t* __restrict__ vals, uint32_t* __restrict__ total,
                                                   unsigned long long* __restrict__ status,
-                                                  unsigned long long* __restrict__ counter, uint32_t* st, uint32_t spin_limit,
-                                                  uint32_t stall_tile, volatile uint32_t* host) {
+                                                  unsigned long long* __restrict__ counter, uint32_t* st,
+                                                  uint32_t spin_limit, uint32_t stall_tile, volatile uint32_t* host) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr unsigned long long kAgg = 1ull << 32, kInc = 2ull << 32;
   __shared__ uint32_t s_tile, s_excl, s_warp[8];
@@ -743,14 +746,15 @@ __device__ __forceinline__ void fwd_pairs(const Rec* __restrict__ sr, uint32_t m
 }
 
 // Forward raster, PPT vertically adjacent pixels per thread: 256 / PPT
-// threads per 16 x 16 tile, a warp covers a 16 x 2·PPT strip, records staged
-// SB = SPS · 256 / PPT at a time.  (PPT, SB) is the autotuned variant.
+// threads per 16 x 16 tile, a warp covers a strip of it (TileMap16), records
+// staged SB = SPS · 256 / PPT at a time.  (PPT, SB) is the autotuned variant.
 // kOrd: a 1D grid whose block b takes work item order[b] (longest tile
 // lists first), else the grid is (tiles x, tiles y, views).  Registers: 64 for
 // 1 pixel per thread, 56 for 2 (nine 128-thread blocks per SM; ten spill, eight
 // give 493 us where nine give 487).
 template <int PPT, int SPS, bool kOrd>
-__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 4 : PPT == 2 ? 9 : 1) k_fwd(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 4 : PPT == 2 ? 9 : 1) k_fwd(const Rec* __restrict__ recs,
+                                                   const uint32_t* __restrict__ vals,
                                                    const uint32_t* __restrict__ rstart,
                                                    const uint32_t* __restrict__ rend, uint32_t W, uint32_t H,
                                                    uint32_t tiles_x, uint32_t num_tiles, float3 bg,
@@ -1496,13 +1500,15 @@ __device__ __forceinline__ bool pixels_bwd(PixBwd (&p)[PPT], const Rec& rec, uin
 // Gaussian) record.  (Adding the warp totals to the records directly is 4%
 // faster, and where a large Gaussian's terms cancel the longer sums lose digits
 // to it, so the block's share is summed first.)  PPT is the
-// autotuned variant.  Issue-bound at 2 pixels per thread (77% of the issue slots):
+// autotuned variant.  Issue-bound at 2 pixels per thread (73% of the issue slots):
 // 72 registers, seven 128-thread blocks per SM (eight are 5% slower at 57k Gaussians
-// and the same at 200k); 1240 -> 921 us at 200k Gaussians, 8 views of 800 x 800.  One pixel per thread serves small grids, which are bound by the latency of
-// the chain from pair to pair: two pairs are evaluated and reduced together
+// and the same at 200k); 1240 -> 921 us at 200k Gaussians, 8 views of 800 x 800.
+// One pixel per thread serves small grids, which are bound by the latency of the
+// chain from pair to pair: two pairs are evaluated and reduced together
 // (65 -> 40 us at 16 tiles, with 80 registers).
 template <int PPT, int SPS, bool kOrd>
-__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_bwd2(const Rec* __restrict__ recs, const uint32_t* __restrict__ vals,
+__global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 3 : PPT == 2 ? 7 : 1) k_bwd2(const Rec* __restrict__ recs,
+                                                    const uint32_t* __restrict__ vals,
                                                     const uint32_t* __restrict__ rstart,
                                                     const uint32_t* __restrict__ rend, uint32_t W, uint32_t H,
                                                     uint32_t tiles_x, uint32_t num_tiles, float3 bg,
@@ -2232,7 +2238,9 @@ struct nps_gs {
   // views of the current step
   uint32_t nv = 0;
   DevBuf views;  // nv view records, then nv target ids (one upload)
-  const uint32_t* tids() const { return reinterpret_cast<const uint32_t*>(views.as<float>() + (size_t)gsm::kViewRec * nv); }
+  const uint32_t* tids() const {
+    return reinterpret_cast<const uint32_t*>(views.as<float>() + (size_t)gsm::kViewRec * nv);
+  }
   // forward state
   DevBuf recs, counts, bins, dkeys, dvals, total, mcount, keys, vals, ranges;
   DevBuf bin_status;             // k_bin_emit: tile counter, then one status word per tile
@@ -2425,10 +2433,11 @@ int nps_gs_destroy(nps_gs* o) {
     b->release();
   for (DevBuf* b : {&o->tile_last, &o->ws_order_f, &o->ws_order_b, &o->ws_q}) b->release();
   for (DevBuf* b : {&o->params, &o->grads, &o->am, &o->av, &o->adc_grad, &o->adc_denom, &o->tgt_own, &o->views,
-                    &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals, &o->bin_status, &o->total, &o->mcount, &o->keys, &o->vals, &o->ranges, &o->img,
-                    &o->ncontrib, &o->maps,
+                    &o->recs, &o->counts, &o->bins, &o->dkeys, &o->dvals, &o->bin_status, &o->total, &o->mcount,
+                    &o->keys, &o->vals, &o->ranges, &o->img, &o->ncontrib, &o->maps,
                     &o->partial, &o->loss, &o->dimg, &o->g2, &o->sw_depth.partial,
-                    &o->sw_depth.lookback, &o->sw_depth.keys_alt, &o->sw_depth.vals_alt, &o->sw_tile.partial, &o->sw_tile.lookback, &o->sw_tile.keys_alt, &o->sw_tile.vals_alt})
+                    &o->sw_depth.lookback, &o->sw_depth.keys_alt, &o->sw_depth.vals_alt, &o->sw_tile.partial,
+                    &o->sw_tile.lookback, &o->sw_tile.keys_alt, &o->sw_tile.vals_alt})
     b->release();
   delete o;
   return NPS_OK;
@@ -2736,7 +2745,8 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool clear
   uint32_t* err = o->stepst.as<uint32_t>() + 6;
   if (form == 1) {
     uint32_t* q = o->ws_q.as<uint32_t>();
-    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(), q);
+    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems,
+                                                               o->ws_order_f.as<uint32_t>(), q);
     NPS_CHECK_LAUNCH();
 #define NPS_FWD_WS(TS, PPT, SB)                                                                                \
   do {                                                                                                         \
@@ -2771,8 +2781,8 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool clear
   }
   const bool ord = form == 2;
   if (ord) {
-    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems, o->ws_order_f.as<uint32_t>(),
-                                                o->ws_q.as<uint32_t>());
+    gs::k_order_items<false><<<gs::kOrderBlocks, 1024, 0, s>>>(rstart, rend, nullptr, nitems,
+                                                               o->ws_order_f.as<uint32_t>(), o->ws_q.as<uint32_t>());
     NPS_CHECK_LAUNCH();
   }
   const dim3 grid = ord ? dim3(nitems, 1, 1) : dim3(tiles_x, tiles_y, nv);
@@ -2915,7 +2925,8 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
   NPS_TRY(o->img.ensure(sizeof(float4) * npix));
   NPS_TRY(o->ncontrib.ensure(sizeof(uint32_t) * npix));
   if (train) NPS_TRY(o->g2.ensure(sizeof(float) * gs::kG2 * (M + 1)));
-  // here and not in nps_gs_create: after set_views has page-locked its staging these words are 0.02 ms, before it 2.5 ms
+  // here and not in nps_gs_create: after set_views has page-locked its staging
+  // these words take 0.02 ms, before it 2.5 ms
   if (!capture && !o->h_fwd) {
     NPS_CUDA(cudaMallocHost((void**)&o->h_fwd, 16));
     NPS_CUDA(cudaEventCreateWithFlags(&o->fwd_counted, cudaEventDisableTiming));

@@ -420,7 +420,8 @@ struct nps_mesh {
   int matcap_w = 1, matcap_h = 1, env_w = 1, env_h = 1, albedo_w = 1, albedo_h = 1, nmap_w = 1, nmap_h = 1;
   uint32_t first_pbr = 0xffffffffu;  // triangles from here on use the PBR stage
   ~nps_mesh() {
-    for (DevBuf* b : {&verts, &idx, &vout, &chunks, &offsets, &total, &zbuf, &matcap, &env, &albedo, &nmap, &work.partial, &work.lookback, &work.keys_alt, &work.vals_alt})
+    for (DevBuf* b : {&verts, &idx, &vout, &chunks, &offsets, &total, &zbuf, &matcap, &env, &albedo, &nmap,
+                      &work.partial, &work.lookback, &work.keys_alt, &work.vals_alt})
       b->release();
   }
 };

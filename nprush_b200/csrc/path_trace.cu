@@ -584,9 +584,9 @@ __device__ __forceinline__ float3 trace_pixel(const Scene& sc, const Camera& cam
 }
 
 template <bool kOrdered>
-__global__ void __launch_bounds__(128, kOrdered ? 8 : 10) k_path_trace(Scene sc, Camera cam, float4* __restrict__ accum, uint32_t w,
-                                                    uint32_t h, uint32_t frame0, uint32_t frames,
-                                                    uint32_t* overflow) {
+__global__ void __launch_bounds__(128, kOrdered ? 8 : 10) k_path_trace(Scene sc, Camera cam,
+                                                    float4* __restrict__ accum, uint32_t w, uint32_t h,
+                                                    uint32_t frame0, uint32_t frames, uint32_t* overflow) {
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t x = blockIdx.x * 16u + (warp & 1u) * 8u + (lane & 7u);
   const uint32_t y = blockIdx.y * 8u + (warp >> 1) * 4u + (lane >> 3);

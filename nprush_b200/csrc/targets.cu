@@ -159,8 +159,9 @@ __global__ void k_depth_blur(const float4* __restrict__ color, const float4* __r
 // and halo with the depth beside the colour (one 16-byte load per tap), two
 // vertically adjacent pixels per thread (a tap's load serves both, at two
 // values of dy), the spatial weights from a table.  Two exponentials per tap
-// remain and bound it (packed arithmetic for the two pixels gained nothing).  kEdge: the halo leaves the image, so taps are tested.
-// 1024 x 768, radius 4: 167 -> 89 us.
+// remain and bound it (packed arithmetic for the two pixels gained nothing).
+// kEdge: the halo leaves the image, so taps are tested.  1024 x 768, radius 4: 167
+// -> 89 us.
 template <bool kEdge>
 __device__ __forceinline__ void depth_blur_tile(const float4* tile, const float* spatial, int radius, int sw, int lx,
                                                 int ly, int x, int y, int w, int h, float4* __restrict__ dst,
