@@ -285,7 +285,9 @@ int nps_gs_set_image_size(nps_gs* gs, uint32_t width, uint32_t height);
  * and for each the index of its target image (null = 0, 1, 2, ...). */
 int nps_gs_set_views(nps_gs* gs, const float* vp, const float* vp_inv, const uint32_t* target_ids, uint32_t num_views);
 /* Paired differentiable rendering: forward keeps only per-record and per-pixel
- * state (final transmittance + last contributor); backward replays. */
+ * state (final transmittance + last contributor); backward replays.  More
+ * tile pairs than the sort takes (2^30 - 1, a quarter of room included):
+ * NPS_ERR_INVALID, with nothing allocated for them. */
 int nps_gs_forward(nps_gs* gs, float* out_rgba_device);
 /* Fused loss of the last forward against the targets; loss3 (host, may be
  * null) = {loss, mean L1, mean SSIM} (L1 + D-SSIM) or {loss, mean L1, mean

@@ -876,8 +876,9 @@ __global__ void __launch_bounds__(256 / PPT, PPT == 1 ? 4 : PPT == 2 ? 9 : 1) k_
 // shared memory instead read seventeen words per output for the second pass
 // and recompute 31% of the first one (both kernels 348 -> 321 us at 8 views of 800 x 800, 1084 -> 895
 // at 8 views of 1920 x 1080).  Values that share a weight (x and y, xx and yy) are added
-// in packed pairs (forward 203 us without).  The forward is bound by issue and the FMA
-// pipe, the backward by shared-memory bandwidth and issue.
+// in packed pairs (forward 203 us without).  The forward issues in 62% of the slots, the
+// FMA pipe busy half of the time; the backward in 54%, its warps waiting for the maps'
+// rows, with shared memory the busiest unit (63%).
 constexpr int kHalo = kSsimWin / 2;
 constexpr int kSsimCols = 32, kSsimRow = kSsimCols + 2 * kHalo;  // outputs of a row, staged columns
 
