@@ -34,6 +34,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -2712,7 +2713,7 @@ static RasterVariant raster_variant(const nps_gs* o, bool bwd) {
 
 // Resident CTAs of a persistent kernel on the device (queried once per kernel).
 template <class K>
-static int persistent_grid(nps_gs* o, K kernel, int threads, int* cache) {
+static int persistent_grid(nps_gs* o, K kernel, int threads, std::atomic<int>* cache) {
   if (*cache == 0) {
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0) != cudaSuccess || per_sm < 1)
@@ -2751,7 +2752,7 @@ static int launch_fwd_raster(nps_gs* o, int form, int ppt, int stage, bool clear
     NPS_CHECK_LAUNCH();
 #define NPS_FWD_WS(TS, PPT, SB)                                                                                \
   do {                                                                                                         \
-    static int grid_cache = 0;                                                                                 \
+    static std::atomic<int> grid_cache{0};                                                                     \
     const int grid = persistent_grid(o, gs::k_fwd_ws<TS, PPT, SB>, TS * TS / PPT + 32, &grid_cache);           \
     gs::k_fwd_ws<TS, PPT, SB><<<grid, TS * TS / PPT + 32, 0, s>>>(                                             \
         o->recs.as<gs::Rec>(), o->sorted_vals, rstart, rend, o->ws_order_f.as<uint32_t>(), q, W, H, tiles_x,   \
@@ -2826,7 +2827,7 @@ static int launch_bwd_raster(nps_gs* o, int form, int ppt, int stage, const floa
     NPS_CHECK_LAUNCH();
 #define NPS_BWD_WS(TS, PPT, SB)                                                                                \
   do {                                                                                                         \
-    static int grid_cache = 0;                                                                                 \
+    static std::atomic<int> grid_cache{0};                                                                     \
     const int grid = persistent_grid(o, gs::k_bwd_ws<TS, PPT, SB>, TS * TS / PPT + 32, &grid_cache);           \
     gs::k_bwd_ws<TS, PPT, SB><<<grid, TS * TS / PPT + 32, 0, s>>>(                                             \
         o->recs.as<gs::Rec>(), o->sorted_vals, rstart, o->tile_last.as<uint32_t>(),                            \
@@ -3112,7 +3113,7 @@ int nps_gs_loss(nps_gs* o, float* loss3_host) {
                                                  (float)nv / (float)lv, o->loss.as<float>());
     NPS_CHECK_LAUNCH();
   } else {
-    static int resident_fwd = 0, resident_bwd = 0;
+    static std::atomic<int> resident_fwd{0}, resident_bwd{0};
     const uint32_t columns = div_up(W, gs::kSsimCols);
     const uint32_t rows_f = ssim_strip_rows(columns * nv, H, persistent_grid(o, gs::k_ssim_fwd, 96, &resident_fwd));
     const uint32_t rows_b = ssim_strip_rows(columns * nv, H, persistent_grid(o, gs::k_ssim_bwd, 96, &resident_bwd));

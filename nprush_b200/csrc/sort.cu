@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <utility>
 
 #include "common.cuh"
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(uint32_t* __restri
 template <int ITEMS>
 int launch_small(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int passes, bool iota,
                  cudaStream_t s) {
-  static bool set[64] = {};  // per device; a second thread setting it again does no harm
+  static std::atomic<bool> set[64] = {};  // per device; a second thread setting it again does no harm
   int dev = 0;
   NPS_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !set[dev]) {
