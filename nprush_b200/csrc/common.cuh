@@ -93,5 +93,10 @@ int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, ui
 // possibly empty) that has to be zero before each sort of these sizes.
 int radix_sort_prepare(uint32_t cap, int bits, SortWork& w, void** region, size_t* bytes);
 
+// Key and value buffers of a pair list for `pairs` pairs and a quarter of room.
+// More than the sort takes is refused before anything is allocated; the
+// capacity is 0 while the buffers are replaced.
+int grow_pair_buffers(uint32_t pairs, DevBuf& keys, DevBuf& vals, uint32_t* cap);
+
 
 }  // namespace nps

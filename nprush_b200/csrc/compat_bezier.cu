@@ -1367,12 +1367,7 @@ int nps_bezier_opt_backward(nps_bezier_opt* o, float* out_rgbd) {
   uint32_t K = 0;
   NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   NPS_CUDA(cudaStreamSynchronize(s));
-  if (K > o->pair_cap || o->pair_cap == 0) {
-    const uint32_t cap = K + K / 4 + 4096;
-    NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)cap));
-    NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)cap));
-    o->pair_cap = cap;
-  }
+  if (K > o->pair_cap || o->pair_cap == 0) NPS_TRY(grow_pair_buffers(K, o->keys, o->vals, &o->pair_cap));
   NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * (size_t)num_tiles * nv, s));
   uint32_t* rstart = o->ranges.as<uint32_t>();
   uint32_t* rend = rstart + (size_t)num_tiles * nv;
@@ -1503,12 +1498,7 @@ int nps_bezier_opt_render(nps_bezier_opt* o, const float* vp, uint32_t w, uint32
   uint32_t K = 0;
   NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   NPS_CUDA(cudaStreamSynchronize(s));
-  if (K > o->r_pair_cap || o->r_pair_cap == 0) {
-    const uint32_t cap = K + K / 4 + 4096;
-    NPS_TRY(o->r_keys.ensure(sizeof(uint32_t) * (size_t)cap));
-    NPS_TRY(o->r_vals.ensure(sizeof(uint32_t) * (size_t)cap));
-    o->r_pair_cap = cap;
-  }
+  if (K > o->r_pair_cap || o->r_pair_cap == 0) NPS_TRY(grow_pair_buffers(K, o->r_keys, o->r_vals, &o->r_pair_cap));
   uint32_t* rstart = o->r_ranges.as<uint32_t>();
   uint32_t* rend = rstart + num_tiles;
   NPS_CUDA(cudaMemsetAsync(rstart, 0, sizeof(uint32_t) * 2 * num_tiles, s));

@@ -1459,12 +1459,7 @@ int nps_splat_opt_backward(nps_splat_opt* o, float* out_rgbd) {
               hk[1]);
     return NPS_ERR_TIMEOUT;
   }
-  if (K > o->pair_cap) {
-    uint32_t cap = K + K / 4 + 4096;
-    NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)cap));
-    NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)cap));
-    o->pair_cap = cap;
-  }
+  if (K > o->pair_cap) NPS_TRY(grow_pair_buffers(K, o->keys, o->vals, &o->pair_cap));
   NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * (size_t)num_tiles * nv, s));
   uint32_t* rstart = o->ranges.as<uint32_t>();
   uint32_t* rend = rstart + (size_t)num_tiles * nv;
@@ -1635,12 +1630,7 @@ static int splat_render(nps_splat_opt* o, const float* vp, uint32_t w, uint32_t 
   uint32_t K = 0;
   NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   NPS_CUDA(cudaStreamSynchronize(s));
-  if (K > rw.pair_cap || rw.pair_cap == 0) {
-    const uint32_t cap = K + K / 4 + 4096;
-    NPS_TRY(rw.keys.ensure(sizeof(uint32_t) * (size_t)cap));
-    NPS_TRY(rw.vals.ensure(sizeof(uint32_t) * (size_t)cap));
-    rw.pair_cap = cap;
-  }
+  if (K > rw.pair_cap || rw.pair_cap == 0) NPS_TRY(grow_pair_buffers(K, rw.keys, rw.vals, &rw.pair_cap));
   uint32_t* rstart = rw.ranges.as<uint32_t>();
   uint32_t* rend = rstart + num_tiles;
   NPS_CUDA(cudaMemsetAsync(rstart, 0, sizeof(uint32_t) * 2 * num_tiles, s));

@@ -3040,17 +3040,12 @@ static int gs_forward_impl(nps_gs* o, float* out_rgba, bool capture, bool train 
       return NPS_ERR_TIMEOUT;
     }
     if (cap > 0 && K <= cap) break;
-    const uint64_t want = (uint64_t)K + K / 4 + 4096;
-    if (round > 0 || want >= (1ull << 30)) {
-      o->fwd_valid = o->loss_valid = false;
-      set_error("gs_forward: %u or more tile pairs do not fit the %u that the sort takes", K,
-                round > 0 ? cap : (1u << 30) - 1u);
+    o->fwd_valid = o->loss_valid = false;
+    if (round > 0) {
+      set_error("gs_forward: the emission counted %u pairs after fewer than %u", K, cap);
       return NPS_ERR_INVALID;
     }
-    o->pair_cap = 0;  // until both buffers are there
-    NPS_TRY(o->keys.ensure(sizeof(uint32_t) * (size_t)want));
-    NPS_TRY(o->vals.ensure(sizeof(uint32_t) * (size_t)want));
-    o->pair_cap = (uint32_t)want;
+    NPS_TRY(grow_pair_buffers(K, o->keys, o->vals, &o->pair_cap));
   }
   o->K = K;
   if (out_rgba) NPS_CUDA(cudaMemcpyAsync(out_rgba, o->img.p, sizeof(float4) * npix, cudaMemcpyDeviceToDevice, s));

@@ -579,6 +579,20 @@ int radix_sort_prepare(uint32_t cap, int bits, SortWork& w, void** region, size_
   return NPS_OK;
 }
 
+int grow_pair_buffers(uint32_t pairs, DevBuf& keys, DevBuf& vals, uint32_t* cap) {
+  const uint64_t want = (uint64_t)pairs + pairs / 4 + 4096;
+  if (want >= (1ull << 30)) {
+    set_error("%u or more tile pairs and a quarter of room are beyond the %u that the sort takes", pairs,
+              (1u << 30) - 1u);
+    return NPS_ERR_INVALID;
+  }
+  *cap = 0;
+  NPS_TRY(keys.ensure(sizeof(uint32_t) * (size_t)want));
+  NPS_TRY(vals.ensure(sizeof(uint32_t) * (size_t)want));
+  *cap = (uint32_t)want;
+  return NPS_OK;
+}
+
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, const uint32_t* count_dev, uint32_t cap, int bits, SortWork& w,
                    cudaStream_t s, uint32_t** keys_out, uint32_t** vals_out, bool iota, bool cleared) {
   return radix_sort_impl<uint32_t>(keys, vals, count_dev, cap, bits, w, s, keys_out, vals_out, iota, cleared);

@@ -243,3 +243,34 @@ def test_colour_that_is_not_finite(cls, channel, value):
     np.testing.assert_array_equal(np.isnan(got), np.isnan(ref["image"]))
     np.testing.assert_allclose(got, ref["image"], atol=1e-5, rtol=0, equal_nan=True)
     np.testing.assert_array_equal(m.read_state()["grads"], ref["grads_q"])
+
+
+def test_more_pairs_than_a_sort_takes(cls):
+    """Curves that each cover all 2500 tiles of 8 views: 3.6e9 pairs, where a 25%
+    margin on the count passes 2^32.  The dispatch reports that they are too many, and
+    the handle then composites a small scene as a fresh one does."""
+    n, w, h = 180_000, 800, 800
+    big = bezier_scene(n, 5, width=(6.0, 7.0))
+    vp, vpi = zip(*(camera(w, h, dist=1.4, eye=e) for e in ((1.4, 0.1, 0.2), (-1.4, 0.3, 0.1), (0.1, 0.2, 1.4), (0.2, 0.1, -1.4),
+                                                       (1.0, 0.2, 1.0), (-1.0, 0.1, 1.0), (1.0, 0.2, -1.0), (-1.0, 0.3, -1.0))))
+    from nprush_b200._lib import NpsError
+    tex = [torch.zeros((8, h, w, 4), device="cuda") if k in (0, 2, 4) else torch.ones((8, h, w), device="cuda") for k in range(5)]
+    imgs = []
+    for first in (big, None):
+        m = cls(n, init=first)
+        m.write_vp(np.stack(vp), np.stack(vpi))
+        m.write_mode(1.0)
+        m.set_backward_target(*tex, w, h)
+        if first is not None:
+            with pytest.raises(NpsError) as e:
+                m.backward()
+            assert e.value.code == -1  # NPS_ERR_INVALID
+        small = bezier_scene(n, 6)
+        small[300:, 19] = 0.0
+        m.write_params(small)
+        img = torch.zeros((8, h, w, 4), device="cuda")
+        m.backward(out_rgbd=img)
+        imgs.append(img.cpu().numpy())
+        m.close()
+    np.testing.assert_array_equal(imgs[0], imgs[1])
+    assert imgs[0].std() > 0
