@@ -180,6 +180,11 @@ int nps_splat_opt_stats(nps_splat_opt* opt, nps_stats* out);
  * out on a normal input: the raster's CTA for that tile stops, and the next
  * backward returns NPS_ERR_TIMEOUT.  No counterpart in the reference. */
 int nps_splat_opt_set_wait_guard(nps_splat_opt* opt, uint32_t spin_limit, uint32_t stall_batch);
+/* The same for the look-back of the optimiser's and the display forward's tile
+ * sorts (polls of a tile's status, 0 = the default, 2^20; a tile whose status
+ * is treated as never published, 0xffffffff = none).  A call whose sort gave up
+ * sees empty tile lists, and the next one of its kind returns NPS_ERR_TIMEOUT. */
+int nps_splat_opt_set_sort_guard(nps_splat_opt* opt, uint32_t spin_limit, uint32_t stall_tile);
 /* Sets the manager's stepCount (GpuSplatOptimizerManager.ts:380, dispatch()
  * calls so far; ADC runs when it reaches a multiple of 25): a restored
  * checkpoint continues the ADC schedule. */
@@ -241,6 +246,8 @@ int nps_bezier_opt_buffers(nps_bezier_opt* opt, float** beziers, int32_t** grads
 int nps_bezier_opt_stats(nps_bezier_opt* opt, nps_stats* out);
 /* Sets the manager's stepCount (GpuBezierOptimizerManager.ts:398). */
 int nps_bezier_opt_set_step_count(nps_bezier_opt* opt, uint32_t count);
+/* Bounds of the tile sorts' look-backs, as nps_splat_opt_set_sort_guard. */
+int nps_bezier_opt_set_sort_guard(nps_bezier_opt* opt, uint32_t spin_limit, uint32_t stall_tile);
 
 /* ====================================== 3D Gaussians (the trainer)
  * No counterpart in the reference, which fits linear-parameter generalised

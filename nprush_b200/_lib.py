@@ -123,6 +123,8 @@ SIGNATURES = {
     "nps_gs_get_raster": [P, P],
     "nps_gs_autotune_raster": [P, ctypes.c_char_p, P, P],
     "nps_splat_opt_set_wait_guard": [P, U32, U32],
+    "nps_splat_opt_set_sort_guard": [P, U32, U32],
+    "nps_bezier_opt_set_sort_guard": [P, U32, U32],
     "nps_gs_set_sort_guard": [P, U32, U32],
     "nps_gs_set_bin_guard": [P, U32, U32],
     "nps_gs_autotune": [P, ctypes.c_char_p, P, P],

@@ -192,6 +192,11 @@ class GpuBezierOptimizerManager:
         """stepCount (dispatch() calls so far; ADC every adc_period)."""
         call("nps_bezier_opt_set_step_count", self._h, int(count))
 
+    def set_sort_guard(self, spin_limit: int = 0, stall_tile: int = 0xFFFFFFFF):
+        """Look-back bound of the tile sorts (0: the default); stall_tile (tests) is
+        a tile whose status is treated as never published."""
+        call("nps_bezier_opt_set_sort_guard", self._h, int(spin_limit), int(stall_tile))
+
     def close(self):
         if getattr(self, "_h", None):
             call("nps_bezier_opt_destroy", self._h)

@@ -2,6 +2,8 @@
 // the tile bounds must equal the reference's float values bit for bit).
 #include "binning.cuh"
 
+#include "common.cuh"
+
 namespace nps {
 namespace bin {
 
@@ -39,13 +41,27 @@ __global__ void k_emit(const uint32_t* __restrict__ counts, const uint32_t* __re
 }
 
 __global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ total, uint32_t cap,
-                         uint32_t* __restrict__ rstart, uint32_t* __restrict__ rend) {
-  const uint32_t K = min(*total, cap);
+                         const uint32_t* __restrict__ gave_up, uint32_t* __restrict__ rstart,
+                         uint32_t* __restrict__ rend) {
+  const uint32_t K = *gave_up ? 0u : min(*total, cap);
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < K; p += gridDim.x * blockDim.x) {
     const uint32_t k = keys[p];
     if (p == 0 || keys[p - 1] != k) rstart[k] = p;
     if (p == K - 1 || keys[p + 1] != k) rend[k] = p + 1;
   }
+}
+
+int read_total(uint32_t* total, const char* what, uint32_t* pairs, cudaStream_t s) {
+  uint32_t hk[2] = {0, 0};
+  NPS_CUDA(cudaMemcpyAsync(hk, total, sizeof(hk), cudaMemcpyDeviceToHost, s));
+  NPS_CUDA(cudaStreamSynchronize(s));
+  *pairs = hk[0];
+  if (hk[1] != 0) {
+    NPS_CUDA(cudaMemsetAsync(total + 1, 0, sizeof(uint32_t), s));
+    set_error("%s: %u bounded waits of the previous one's sort gave up (its result is not valid)", what, hk[1]);
+    return NPS_ERR_TIMEOUT;
+  }
+  return NPS_OK;
 }
 
 }  // namespace bin

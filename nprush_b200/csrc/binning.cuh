@@ -62,9 +62,15 @@ __global__ void k_emit(const uint32_t* __restrict__ counts, const uint32_t* __re
                        const uint2* __restrict__ rects, uint32_t n, uint32_t nv, uint32_t tiles_x, uint32_t num_tiles,
                        uint32_t cap, uint32_t* __restrict__ keys, uint32_t* __restrict__ vals);
 
-// Tile list bounds in the sorted key array.
+// Tile list bounds in the sorted key array; none after a sort that gave up
+// waiting (*gave_up), whose output may hold any key and any primitive.
 __global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ total, uint32_t cap,
-                         uint32_t* __restrict__ rstart, uint32_t* __restrict__ rend);
+                         const uint32_t* __restrict__ gave_up, uint32_t* __restrict__ rstart,
+                         uint32_t* __restrict__ rend);
+
+// Number of pairs (*pairs) from total[0], with the count of sorts that gave up
+// since the last call in total[1]: reported and cleared.  Waits for the stream.
+int read_total(uint32_t* total, const char* what, uint32_t* pairs, cudaStream_t s);
 
 }  // namespace bin
 }  // namespace nps

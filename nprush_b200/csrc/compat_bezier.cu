@@ -1177,6 +1177,7 @@ int nps_bezier_opt_create(nps_ctx* ctx, uint32_t num_beziers, nps_bezier_opt** o
   cudaMemsetAsync(o->lacc.p, 0, sizeof(float) * n, s);
   cudaMemsetAsync(o->pixel_loss.p, 0, sizeof(int32_t) * bz::kPixelLossSize, s);
   cudaMemsetAsync(o->stat.p, 0, 64, s);
+  cudaMemsetAsync(o->total.p, 0, 16, s);
   NPS_CUDA(cudaGetLastError());
   *out = o;
   return NPS_OK;
@@ -1362,11 +1363,11 @@ int nps_bezier_opt_backward(nps_bezier_opt* o, float* out_rgbd) {
                                                    o->tabs.as<float>(), tiles_x, tiles_y, o->fwd.as<float>(),
                                                    o->bwd.as<float>(), o->counts.as<uint32_t>(), o->rects.as<uint2>());
   NPS_CHECK_LAUNCH();
-  uint32_t* total = o->total.as<uint32_t>();
+  uint32_t* total = o->total.as<uint32_t>();  // [0] pairs, [1] sort waits that gave up
+  o->sw.err = total + 1;
   NPS_TRY(exclusive_scan_u32(o->counts.as<uint32_t>(), o->offsets.as<uint32_t>(), (uint32_t)g, total, o->sw, s));
   uint32_t K = 0;
-  NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  NPS_CUDA(cudaStreamSynchronize(s));
+  NPS_TRY(bin::read_total(total, "bezier backward", &K, s));
   if (K > o->pair_cap || o->pair_cap == 0) NPS_TRY(grow_pair_buffers(K, o->keys, o->vals, &o->pair_cap));
   NPS_CUDA(cudaMemsetAsync(o->ranges.p, 0, sizeof(uint32_t) * 2 * (size_t)num_tiles * nv, s));
   uint32_t* rstart = o->ranges.as<uint32_t>();
@@ -1382,7 +1383,7 @@ int nps_bezier_opt_backward(nps_bezier_opt* o, float* out_rgbd) {
     uint32_t *ks = nullptr, *vv = nullptr;
     NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total, o->pair_cap, bits, o->sw, s, &ks,
                            &vv));
-    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->pair_cap, rstart, rend);
+    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->pair_cap, total + 1, rstart, rend);
     NPS_CHECK_LAUNCH();
     vs = vv;
   }
@@ -1482,7 +1483,10 @@ int nps_bezier_opt_render(nps_bezier_opt* o, const float* vp, uint32_t w, uint32
   NPS_TRY(o->r_counts.ensure(sizeof(uint32_t) * n));
   NPS_TRY(o->r_offsets.ensure(sizeof(uint32_t) * n));
   NPS_TRY(o->r_rects.ensure(sizeof(uint2) * n));
-  NPS_TRY(o->r_total.ensure(16));
+  if (!o->r_total.p) {
+    NPS_TRY(o->r_total.ensure(16));
+    NPS_CUDA(cudaMemsetAsync(o->r_total.p, 0, 16, s));
+  }
   NPS_TRY(o->r_cam.ensure(64));
   NPS_TRY(o->r_ranges.ensure(sizeof(uint32_t) * 2 * num_tiles));
   NPS_TRY(o->r_tabs.ensure(sizeof(float) * 2 * (tiles_x + tiles_y)));
@@ -1494,10 +1498,10 @@ int nps_bezier_opt_render(nps_bezier_opt* o, const float* vp, uint32_t w, uint32
                                                           o->r_rects.as<uint2>());
   NPS_CHECK_LAUNCH();
   uint32_t* total = o->r_total.as<uint32_t>();
+  o->r_sw.err = total + 1;
   NPS_TRY(exclusive_scan_u32(o->r_counts.as<uint32_t>(), o->r_offsets.as<uint32_t>(), n, total, o->r_sw, s));
   uint32_t K = 0;
-  NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  NPS_CUDA(cudaStreamSynchronize(s));
+  NPS_TRY(bin::read_total(total, "bezier render", &K, s));
   if (K > o->r_pair_cap || o->r_pair_cap == 0) NPS_TRY(grow_pair_buffers(K, o->r_keys, o->r_vals, &o->r_pair_cap));
   uint32_t* rstart = o->r_ranges.as<uint32_t>();
   uint32_t* rend = rstart + num_tiles;
@@ -1513,7 +1517,7 @@ int nps_bezier_opt_render(nps_bezier_opt* o, const float* vp, uint32_t w, uint32
     uint32_t *ks = nullptr, *vv = nullptr;
     NPS_TRY(radix_sort_u32(o->r_keys.as<uint32_t>(), o->r_vals.as<uint32_t>(), total, o->r_pair_cap, bits, o->r_sw, s,
                            &ks, &vv));
-    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->r_pair_cap, rstart, rend);
+    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->r_pair_cap, total + 1, rstart, rend);
     NPS_CHECK_LAUNCH();
     vs = vv;
   }
@@ -1534,6 +1538,15 @@ int nps_bezier_opt_buffers(nps_bezier_opt* o, float** bzp, int32_t** grads, floa
   if (gacc) *gacc = o->gacc.as<float>();
   if (lacc) *lacc = o->lacc.as<float>();
   if (pixel_loss) *pixel_loss = o->pixel_loss.as<int32_t>();
+  return NPS_OK;
+}
+
+int nps_bezier_opt_set_sort_guard(nps_bezier_opt* o, uint32_t spin_limit, uint32_t stall_tile) {
+  NPS_TRY(check_bz(o));
+  for (SortWork* w : {&o->sw, &o->r_sw}) {
+    w->spin_limit = spin_limit ? spin_limit : 1u << 20;
+    w->stall_tile = stall_tile;
+  }
   return NPS_OK;
 }
 

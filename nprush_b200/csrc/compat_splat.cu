@@ -400,10 +400,12 @@ __global__ void k_range_len(const uint32_t* __restrict__ rstart, const uint32_t*
     tile_len[i] = rend[i] - rstart[i];
 }
 
-// Tile list bounds in the sorted key array.
+// Tile list bounds in the sorted key array; none after a sort that gave up
+// waiting, whose output may hold any key and any splat.
 __global__ void k_ranges(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ total, uint32_t cap,
-                         uint32_t* __restrict__ rstart, uint32_t* __restrict__ rend) {
-  const uint32_t K = min(*total, cap);
+                         const uint32_t* __restrict__ gave_up, uint32_t* __restrict__ rstart,
+                         uint32_t* __restrict__ rend) {
+  const uint32_t K = *gave_up ? 0u : min(*total, cap);
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < K; p += gridDim.x * blockDim.x) {
     const uint32_t k = keys[p];
     if (p == 0 || keys[p - 1] != k) rstart[k] = p;
@@ -1494,7 +1496,7 @@ int nps_splat_opt_backward(nps_splat_opt* o, float* out_rgbd) {
     uint32_t *ks = nullptr, *vs = nullptr;
     NPS_TRY(radix_sort_u32(o->keys.as<uint32_t>(), o->vals.as<uint32_t>(), total, o->pair_cap, bits, o->sw, s, &ks,
                            &vs));
-    compat::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->pair_cap, rstart, rend);
+    compat::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, o->pair_cap, total + 1, rstart, rend);
     NPS_CHECK_LAUNCH();
     ra.vals = vs;
   }
@@ -1569,6 +1571,13 @@ int nps_splat_opt_set_wait_guard(nps_splat_opt* o, uint32_t spin_limit, uint32_t
   return NPS_OK;
 }
 
+int nps_splat_opt_set_sort_guard(nps_splat_opt* o, uint32_t spin_limit, uint32_t stall_tile) {
+  NPS_TRY(check_opt(o));
+  o->sw.spin_limit = spin_limit ? spin_limit : 1u << 20;
+  o->sw.stall_tile = stall_tile;
+  return NPS_OK;
+}
+
 int nps_splat_opt_stats(nps_splat_opt* o, nps_stats* out) {
   NPS_TRY(check_opt(o));
   if (!out) return NPS_ERR_INVALID;
@@ -1609,13 +1618,18 @@ static int splat_render(nps_splat_opt* o, const float* vp, uint32_t w, uint32_t 
   }
   if (!o->rw) o->rw = new RenderWork();
   RenderWork& rw = *o->rw;
+  rw.sw.spin_limit = o->sw.spin_limit;
+  rw.sw.stall_tile = o->sw.stall_tile;
   cudaStream_t s = o->ctx->stream;
   const uint32_t n = o->n, tiles_x = div_up(w, 16), tiles_y = div_up(h, 16), num_tiles = tiles_x * tiles_y;
   NPS_TRY(rw.rec.ensure(sizeof(float) * compat::kRend * n));
   NPS_TRY(rw.counts.ensure(sizeof(uint32_t) * n));
   NPS_TRY(rw.offsets.ensure(sizeof(uint32_t) * n));
   NPS_TRY(rw.rects.ensure(sizeof(uint2) * n));
-  NPS_TRY(rw.total.ensure(16));
+  if (!rw.total.p) {
+    NPS_TRY(rw.total.ensure(16));
+    NPS_CUDA(cudaMemsetAsync(rw.total.p, 0, 16, s));
+  }
   NPS_TRY(rw.cam.ensure(64));
   NPS_TRY(rw.ranges.ensure(sizeof(uint32_t) * 2 * num_tiles));
   NPS_TRY(rw.tabs.ensure(sizeof(float) * 2 * (tiles_x + tiles_y)));
@@ -1625,11 +1639,11 @@ static int splat_render(nps_splat_opt* o, const float* vp, uint32_t w, uint32_t 
                                                            rw.tabs.as<float>(), tiles_x, tiles_y, rw.rec.as<float>(),
                                                            rw.counts.as<uint32_t>(), rw.rects.as<uint2>());
   NPS_CHECK_LAUNCH();
-  uint32_t* total = rw.total.as<uint32_t>();
+  uint32_t* total = rw.total.as<uint32_t>();  // [0] pairs, [1] sort waits that gave up
+  rw.sw.err = total + 1;
   NPS_TRY(exclusive_scan_u32(rw.counts.as<uint32_t>(), rw.offsets.as<uint32_t>(), n, total, rw.sw, s));
   uint32_t K = 0;
-  NPS_CUDA(cudaMemcpyAsync(&K, total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  NPS_CUDA(cudaStreamSynchronize(s));
+  NPS_TRY(bin::read_total(total, "splat render", &K, s));
   if (K > rw.pair_cap || rw.pair_cap == 0) NPS_TRY(grow_pair_buffers(K, rw.keys, rw.vals, &rw.pair_cap));
   uint32_t* rstart = rw.ranges.as<uint32_t>();
   uint32_t* rend = rstart + num_tiles;
@@ -1645,7 +1659,7 @@ static int splat_render(nps_splat_opt* o, const float* vp, uint32_t w, uint32_t 
     uint32_t *ks = nullptr, *vv = nullptr;
     NPS_TRY(radix_sort_u32(rw.keys.as<uint32_t>(), rw.vals.as<uint32_t>(), total, rw.pair_cap, bits, rw.sw, s, &ks,
                            &vv));
-    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, rw.pair_cap, rstart, rend);
+    bin::k_ranges<<<4 * kNumSMs, 256, 0, s>>>(ks, total, rw.pair_cap, total + 1, rstart, rend);
     NPS_CHECK_LAUNCH();
     vs = vv;
   }

@@ -225,6 +225,11 @@ class GpuSplatOptimizerManager:
         issued, so its wait runs out."""
         call("nps_splat_opt_set_wait_guard", self._h, int(spin_limit), int(stall_batch))
 
+    def set_sort_guard(self, spin_limit: int = 0, stall_tile: int = 0xFFFFFFFF):
+        """Look-back bound of the tile sorts (0: the default); stall_tile (tests) is
+        a tile whose status is treated as never published."""
+        call("nps_splat_opt_set_sort_guard", self._h, int(spin_limit), int(stall_tile))
+
     def set_step_count(self, count: int):
         """stepCount (dispatch() calls so far; ADC every 25th)."""
         call("nps_splat_opt_set_step_count", self._h, int(count))

@@ -274,3 +274,40 @@ def test_more_pairs_than_a_sort_takes(cls):
         m.close()
     np.testing.assert_array_equal(imgs[0], imgs[1])
     assert imgs[0].std() > 0
+
+
+def test_sort_timeout_is_reported(cls):
+    """The tile sort's look-back made to run out (tile 2 of its tiles never
+    published, 1000 polls): the backward and the display forward see empty lists, the
+    next of each reports NPS_ERR_TIMEOUT, and with the default bound they are those of a
+    fresh optimiser again, bit for bit."""
+    from nprush_b200._lib import NpsError
+    n, w, h = 3000, 128, 96
+    b = bezier_scene(n, 35)
+    vp, vpi = camera(w, h, dist=1.4)
+    tex = bezier_textures(w, h, 36)
+    out = []
+    for stall in (True, False):
+        m = cls(n, init=b)
+        m.write_vp(vp, vpi)
+        m.write_mode(1.0)
+        m.set_backward_target(*tex, w, h)
+        img = torch.zeros((1, h, w, 4), device="cuda")
+        shown = torch.zeros((h, w, 4), device="cuda")
+        for call in (lambda: m.backward(out_rgbd=img), lambda: m.render(vp, w, h, shown)):
+            if stall:
+                m.set_sort_guard(1000, 2)
+                call()
+                with pytest.raises(NpsError) as e:
+                    call()
+                assert e.value.code == -5  # NPS_ERR_TIMEOUT
+                m.set_sort_guard()
+            m.write_state(grads=np.zeros((n, 18), np.int32))
+            call()
+        m.read_state()  # waits
+        out.append((img.cpu().numpy(), shown.cpu().numpy(), m.read_state()["grads"]))
+        assert m.stats()["pairs"] > 4096
+        m.close()
+    for x, y in zip(*out):
+        np.testing.assert_array_equal(x, y)
+    assert out[1][0].std() > 0 and out[1][1].std() > 0

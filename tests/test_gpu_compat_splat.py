@@ -341,3 +341,39 @@ def test_saturated_terms_wrap(mgr_cls, w, h, seed):
     wrap = lambda t: (t * n + 2 ** 31) % 2 ** 32 - 2 ** 31  # noqa: E731
     assert ref["grads_q"][0, 4:6].tolist() == [wrap(2147483520), wrap(-2 ** 31)]
     np.testing.assert_array_equal(g[0, 4:6], ref["grads_q"][0, 4:6])
+
+
+def test_sort_timeout_is_reported(mgr_cls):
+    """The tile sort's look-back made to run out (tile 2 of its tiles never
+    published, 1000 polls): the backward and the display forward see empty lists, the
+    next of each reports NPS_ERR_TIMEOUT, and with the default bound they are those of a
+    fresh optimiser again, bit for bit."""
+    from nprush_b200._lib import NpsError
+    n, w, h = 4000, 128, 96
+    s = splat_scene(n, 33)
+    vp, vpi = camera(w, h)
+    tgt, depth = targets(w, h, 34)
+    out = []
+    for stall in (True, False):
+        m = mgr_cls(n, init=s)
+        m.write_splat_vp_matrix(vp, vpi)
+        m.set_backward_target(tgt, depth, w, h)
+        img = torch.zeros((1, h, w, 4), device="cuda")
+        shown = torch.zeros((h, w, 4), device="cuda")
+        for call in (lambda: m.backward(out_rgbd=img), lambda: m.render(vp, w, h, shown)):
+            if stall:
+                m.set_sort_guard(1000, 2)
+                call()
+                with pytest.raises(NpsError) as e:
+                    call()
+                assert e.value.code == -5  # NPS_ERR_TIMEOUT
+                m.set_sort_guard()
+            m.write_state(grads=np.zeros((n, 16), np.int32))
+            call()
+            m.sync()
+        out.append((img.cpu().numpy(), shown.cpu().numpy(), m.read_state()["grads"]))
+        assert m.stats()["pairs"] > 4096
+        m.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[1][0].std() > 0 and out[1][1].std() > 0
